@@ -24,6 +24,7 @@
 #include <cfloat>
 
 #include "common.cuh"
+#include "tc_sm100.cuh"
 
 #include <algorithm>
 #include <string>
@@ -809,9 +810,11 @@ __global__ void __launch_bounds__(256) k_xcorr(double2* __restrict__ X0, long lo
 }
 
 // ----------------------------------------------------------------------------- stage 2
-// Band storage: column j holds A[j + o, j] for o = 0 .. LDB-1 (the band, o <= b, and room for
-// the bulges, o <= 2b - 1).
-constexpr int LDB = 2 * BW + 2;
+// Band storage: column j holds A[j + o, j] for o = 0 .. LDB-1 (the band, o <= b, and the bulges,
+// o <= 2b - 1).  Entries past row N are zero and stay zero, and AB_PAD zero columns follow column
+// N-1, so that the chase reads whole blocks at the end of the matrix without masks.
+constexpr int LDB = 2 * BW;
+constexpr int AB_PAD = 2 * BW;
 constexpr int BG_WARPS = 4;                 // sweep workers per CTA
 constexpr int BG_LD = BW + 1;               // padded row length of the per-warp work tiles
 constexpr int BG_WARP_TILE = 3 * BW * BG_LD + 2 * BW;   // Bs, Ds, B1s, v, w (double2) per warp
@@ -832,7 +835,7 @@ __global__ void __launch_bounds__(256) k_band_extract(const double2* __restrict_
   const long long j = blockIdx.x;
   for (int o = threadIdx.x; o < LDB; o += blockDim.x) {
     double2 v = make_double2(0, 0);
-    if (o <= BW && j + o < N) v = A[(j + o) + j * N];
+    if (o <= BW && j + o < N) v = A[(j + o) + j * N];   // zero in the padding columns j >= N
     if (o == 0) v.y = 0.0;
     AB[j * LDB + o] = v;
   }
@@ -1061,256 +1064,492 @@ __global__ void __launch_bounds__(32 * BG_WARPS, 1) k_bulge(BulgeArgs a) {
   }
 }
 
-// Stage 2 with one CTA of four warps per sweep.  After the fetch (all 128 threads) warp 0
-// forms the reflector while warp 2 completes the Hermitian diagonal block; then the four updates,
-// which need only v and tau, run concurrently: warp 0 the annihilated column, the velocity
-// vectors and the stored reflector, warp 1 the left application to the bulge block, warp 2 the
-// two-sided update of the diagonal block, warp 3 the right application to the block below.
-constexpr int B4_THREADS = 128;
-constexpr int B4_TILE = 3 * BW * BG_LD + 4 * BW + 8;   // Bs, Ds, B1s, v, w1, w2, scalars (double2)
-constexpr size_t B4_SMEM = (size_t)B4_TILE * 16;
+// Stage 2 with one CTA per sweep and specialised warps.  The launch is one dependency chain: sweep
+// s may start step t once sweep s-1 has published step t+2, so it takes about N times (three
+// steps + one hand-over between CTAs), and everything in a step that is not on the way from one
+// reflector to the next is moved off that way:
+//   * the reflector's vector is used unscaled: with u = x - beta e_0 the reflector is
+//     H = I - kappa u u^H, kappa = -u_0 / (beta |u_0|^2), and every product D u, B1 u, u^H B is the
+//     product with x minus beta times the first column (row), so the products of a step run beside
+//     the scalars (one reciprocal square root, one reciprocal) instead of after them;
+//   * the block below (B1) is the next step's bulge block (B): the four warps that update it keep it
+//     in registers, so it is written once, after its second update.  Four groups of four warps take
+//     turns: group n mod 4 does B1 of step n, then B of step n+1, then the diagonal block of step n+2,
+//     so that the chain from x to x passes from group to group and waits for none of the rest;
+//   * only the first column of B1 (the next x) is on the chain; it is updated first and announced,
+//     and the rest of B1, the B update with its stores, the diagonal block and the velocity vectors
+//     have their own warps and follow through mbarriers;
+//   * one warp waits for the predecessor and copies the next blocks into a ring in shared memory,
+//     one publishes finished steps, so no poll, no L2 round trip and no fence stalls the others.
+// A step is bound by the latency of its instruction chain (2700 cycles from x to x; the FP64 pipe is
+// busy 24 % of them), so index arithmetic is kept out of it: a warp holds 8 rows x 32 columns of a
+// 32 x 32 block, lane -> rows i = 8 wg + ig + 4r (r < 2), columns c = qb + 8m (m < 4) with ig = lane & 3,
+// qb = 4 (bit 2) + (lane >> 3), and an element's place in the band, 63 c + i from its block's corner, is
+// one lane offset plus the constant 504 m + 4 r; the sums over the columns (B1, D) stay within one
+// warp, and the shared-memory accesses are free of bank conflicts.
+// Measured (whole stage, five velocity vectors): N = 576 4.3 ms, 2304 18.9 ms, 8100 80 ms, 14400 161 ms;
+// with one CTA of four warps per sweep and CTA barriers between the parts of a step it was 10.9, 46.7,
+// 169 and 309 ms.  Tried: bulk copies instead of cp.async (longer latency, 19.5 ms at 2304), blocks
+// loaded from L2 into a second set of registers (spills, 24 ms), two groups that swap B1 and B (21 ms).
+constexpr int CH_NS = 4;    // ring slots: steps the groups may be apart
+constexpr int CH_NX = 8;    // steps of x and scalars kept (more than CH_NS + 2)
+constexpr int CH_WARPS = 19;   // 4 x 4 block warps, velocity, producer, publisher (104 registers a thread)
+constexpr int CH_THREADS = 32 * CH_WARPS;
+constexpr int CH_BLK = BW * LDB;                      // one block of 32 band columns
+constexpr int CH_SLOT = CH_BLK + LDB + NGMAX * BW;    // + column s (first step), velocity rows
+constexpr size_t CH_SMEM = (size_t)CH_NS * CH_SLOT * sizeof(double2);
 
-// Bs, Ds, B1s: the bulge block, the diagonal block and the block below; gv: warp 0's rows of the
-// velocity vectors.  With pre, the previous step of the sweep has already placed them (Bs is its
-// block below, updated in place; Ds, B1s and gv prefetched) except the corner of B1s, which the
-// predecessor sweep's step t + 3 writes and which is read here after the wait.
-__device__ void bulge_step4(const BulgeArgs& a, long long s, long long t, double2* Bs, double2* Ds, double2* B1s,
-                            double2* tail, double2 (&gv)[NGMAX], bool pre) {
-  double2* vs = tail;
-  double2* w1 = vs + BW;
-  double2* w2 = w1 + BW;
-  double2* sc = w2 + BW;   // [0] tau, [1] (beta, 0)
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const long long N = a.N;
-  double2* AB = a.AB;
-  const long long r0 = s + 1 + t * BW;
-  const int L = (int)min((long long)BW, N - r0);
-  const long long c0 = r0 - BW;
-  const long long r1 = r0 + L;
-  const int L1 = (r1 < N) ? (int)min((long long)BW, N - r1) : 0;
-  // ---- fetch (element e of each tile: row e % 32, column e / 32)
-  if (!pre) {
-    if (t > 0)
-      for (int e = tid; e < BW * BW; e += B4_THREADS) {
-        const int i = e & 31, q = e >> 5;
-        cpa16(Bs + i * BG_LD + q, AB + (c0 + q) * LDB + (BW + i - q), i < L);
-      }
-    for (int e = tid; e < BW * BW; e += B4_THREADS) {
-      const int i = e & 31, q = e >> 5;
-      if (q < L) {
-        const bool ok = i >= q && i < L;
-        cpa16(Ds + i * BG_LD + q, ok ? AB + (r0 + q) * LDB + (i - q) : AB, ok);
-        cpa16(B1s + i * BG_LD + q, AB + (r0 + q) * LDB + (L + i - q), i < L1);
-      }
-    }
-  } else if (tid == 0 && L == BW && L1 == BW) {
-    cpa16(B1s + (BW - 1) * BG_LD + (BW - 1), AB + (r0 + BW - 1) * LDB + L, true);
-  }
-  asm volatile("cp.async.commit_group;" ::: "memory");
-  if (wid == 0 && !pre) {
-#pragma unroll
-    for (int al2 = 0; al2 < NGMAX; ++al2)
-      gv[al2] = (al2 < a.ng && lane < L) ? __ldcg(a.g + (long long)al2 * N + r0 + lane) : make_double2(0, 0);
-  }
-  double2 x = make_double2(0, 0);
-  if (wid == 0 && t == 0 && lane < L) x = __ldcg(AB + s * LDB + 1 + lane);
-  asm volatile("cp.async.wait_all;" ::: "memory");
-  __syncthreads();
-  // ---- reflector (warp 0) | Hermitian fill of D (warp 2)
-  if (wid == 0) {
-    if (t > 0) x = Bs[lane * BG_LD];
-    double xn2 = (lane >= 1 && lane < L) ? x.x * x.x + x.y * x.y : 0.0;
-    xn2 = warp_sum(xn2);
-    const double2 al = make_double2(__shfl_sync(0xffffffffu, x.x, 0), __shfl_sync(0xffffffffu, x.y, 0));
-    double2 tau, scal;
-    double beta;
-    if (xn2 == 0.0 && al.y == 0.0) {
-      tau = make_double2(0, 0);
-      scal = make_double2(0, 0);
-      beta = al.x;
-    } else {
-      beta = -copysign(sqrt(al.x * al.x + al.y * al.y + xn2), al.x);
-      tau = make_double2((beta - al.x) / beta, -al.y / beta);
-      const double2 den = make_double2(al.x - beta, al.y);
-      const double dd = den.x * den.x + den.y * den.y;
-      scal = make_double2(den.x / dd, -den.y / dd);
-    }
-    vs[lane] = (lane == 0) ? make_double2(1.0, 0.0) : (lane < L ? cmul(x, scal) : make_double2(0, 0));
-    if (lane == 0) {
-      sc[0] = tau;
-      sc[1] = make_double2(beta, 0.0);
-    }
-  } else if (wid == 2 && lane < L) {
-    for (int q = 0; q <= lane; ++q) {
-      double2 d = Ds[lane * BG_LD + q];
-      if (q == lane) {
-        d.y = 0.0;
-        Ds[lane * BG_LD + q] = d;
-      } else {
-        Ds[q * BG_LD + lane] = cconj(d);
-      }
-    }
-  }
-  __syncthreads();
-  const double2 tau = sc[0];
-  const double2 v = vs[lane];
-  if (wid == 0) {
-    // annihilated column, velocity vectors, stored reflector
-    if (lane < L) {
-      const double2 nv = (lane == 0) ? sc[1] : make_double2(0, 0);
-      if (t == 0) AB[s * LDB + 1 + lane] = nv;
-      else AB[c0 * LDB + BW + lane] = nv;
-    }
-    double2 sg[NGMAX];
-#pragma unroll
-    for (int al2 = 0; al2 < NGMAX; ++al2) sg[al2] = cmul(v, gv[al2]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-      for (int al2 = 0; al2 < NGMAX; ++al2)
-        if (al2 < a.ng) {
-          sg[al2].x += __shfl_xor_sync(0xffffffffu, sg[al2].x, o);
-          sg[al2].y += __shfl_xor_sync(0xffffffffu, sg[al2].y, o);
-        }
-    if (lane < L) {
-      const double2 tcv = cmul(tau, cconj(v));
-#pragma unroll
-      for (int al2 = 0; al2 < NGMAX; ++al2)
-        if (al2 < a.ng) a.g[(long long)al2 * N + r0 + lane] = csub(gv[al2], cmul(tcv, sg[al2]));
-      if (a.store) a.A[(r0 + lane - s - 1) + (N - 1 - s) * N] = v;
-    }
-    if (a.store && lane == 0) a.tau2[tau2_offset(N, s) + t] = tau;
-  } else if (wid == 1) {
-    // left application to the bulge block: B <- H^H B (columns 1..31)
-    if (t > 0) {
-      if (lane >= 1) {
-        double2 a0 = make_double2(0, 0), a1 = a0, a2 = a0, a3 = a0;
-        for (int i = 0; i < L; i += 4) {
-          a0 = cadd(a0, cmulc(vs[i], Bs[i * BG_LD + lane]));
-          if (i + 1 < L) a1 = cadd(a1, cmulc(vs[i + 1], Bs[(i + 1) * BG_LD + lane]));
-          if (i + 2 < L) a2 = cadd(a2, cmulc(vs[i + 2], Bs[(i + 2) * BG_LD + lane]));
-          if (i + 3 < L) a3 = cadd(a3, cmulc(vs[i + 3], Bs[(i + 3) * BG_LD + lane]));
-        }
-        w1[lane] = cadd(cadd(a0, a1), cadd(a2, a3));
-      }
-      __syncwarp();
-      if (lane < L) {
-        const double2 cv = cmul(cconj(tau), v);
-#pragma unroll 4
-        for (int q = 1; q < BW; ++q) AB[(c0 + q) * LDB + (BW + lane - q)] = csub(Bs[lane * BG_LD + q], cmul(cv, w1[q]));
-      }
-    }
-  } else if (wid == 2) {
-    // two-sided update of the diagonal block: D <- H^H D H
-    double2 y = make_double2(0, 0);
-    if (lane < L) {
-      double2 y1 = y, y2 = y, y3 = y;
-      for (int q = 0; q < L; q += 4) {
-        y = cadd(y, cmul(Ds[lane * BG_LD + q], vs[q]));
-        if (q + 1 < L) y1 = cadd(y1, cmul(Ds[lane * BG_LD + q + 1], vs[q + 1]));
-        if (q + 2 < L) y2 = cadd(y2, cmul(Ds[lane * BG_LD + q + 2], vs[q + 2]));
-        if (q + 3 < L) y3 = cadd(y3, cmul(Ds[lane * BG_LD + q + 3], vs[q + 3]));
-      }
-      y = cadd(cadd(y, y1), cadd(y2, y3));
-    }
-    const double pv = warp_sum(cmulc(v, y).x);
-    const double t2 = tau.x * tau.x + tau.y * tau.y;
-    const double2 w = csub(cmul(tau, y), cscale(v, 0.5 * t2 * pv));
-    w2[lane] = w;
-    __syncwarp();
-    if (lane < L)
-#pragma unroll 4
-      for (int q = 0; q <= lane; ++q) {
-        double2 d = csub(Ds[lane * BG_LD + q], cadd(cmulc(w2[q], v), cmulc(vs[q], w)));
-        if (q == lane) d.y = 0.0;
-        AB[(r0 + q) * LDB + (lane - q)] = d;
-      }
-  } else if (L1 > 0 && lane < L1) {
-    // right application to the block below: B1 <- B1 H
-    double2 z = make_double2(0, 0), z1 = z, z2 = z, z3 = z;
-    for (int q = 0; q < L; q += 4) {
-      z = cadd(z, cmul(B1s[lane * BG_LD + q], vs[q]));
-      if (q + 1 < L) z1 = cadd(z1, cmul(B1s[lane * BG_LD + q + 1], vs[q + 1]));
-      if (q + 2 < L) z2 = cadd(z2, cmul(B1s[lane * BG_LD + q + 2], vs[q + 2]));
-      if (q + 3 < L) z3 = cadd(z3, cmul(B1s[lane * BG_LD + q + 3], vs[q + 3]));
-    }
-    z = cadd(cadd(z, z1), cadd(z2, z3));
-    const double2 tz = cmul(tau, z);
-    // also in place: the next step's bulge block
-#pragma unroll 4
-    for (int q = 0; q < L; ++q) {
-      const double2 nb = csub(B1s[lane * BG_LD + q], cmul(tz, cconj(vs[q])));
-      AB[(r0 + q) * LDB + (L + lane - q)] = nb;
-      B1s[lane * BG_LD + q] = nb;
-    }
+// named barriers of whole warps: bar is an aligned instruction, so the warp's lanes are brought
+// together first (they may have left a wait or a lane branch one by one)
+__device__ __forceinline__ void bar_sync(int id, int cnt) {
+  __syncwarp();
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(cnt) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(int id, int cnt) {
+  __syncwarp();
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(cnt) : "memory");
+}
+__device__ __forceinline__ double2 shfl2(double2 v, int src) {
+  return make_double2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
+}
+__device__ __forceinline__ double2 shfl2_xor(double2 v, int o) {
+  return make_double2(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o));
+}
+// c + a b, c - a b, c + conj(a) b, c - conj(a) b: four FMAs each
+__device__ __forceinline__ double2 cfma(double2 a, double2 b, double2 c) {
+  return make_double2(fma(-a.y, b.y, fma(a.x, b.x, c.x)), fma(a.y, b.x, fma(a.x, b.y, c.y)));
+}
+__device__ __forceinline__ double2 cfms(double2 a, double2 b, double2 c) {
+  return make_double2(fma(a.y, b.y, fma(-a.x, b.x, c.x)), fma(-a.y, b.x, fma(-a.x, b.y, c.y)));
+}
+__device__ __forceinline__ double2 cfmac(double2 a, double2 b, double2 c) {
+  return make_double2(fma(a.y, b.y, fma(a.x, b.x, c.x)), fma(-a.y, b.x, fma(a.x, b.y, c.y)));
+}
+__device__ __forceinline__ double2 cfmsc(double2 a, double2 b, double2 c) {
+  return make_double2(fma(-a.y, b.y, fma(-a.x, b.x, c.x)), fma(a.y, b.x, fma(-a.x, b.y, c.y)));
+}
+__device__ __forceinline__ double2 caxpy(double a, double2 b, double2 c) {
+  return make_double2(fma(a, b.x, c.x), fma(a, b.y, c.y));
+}
+// Reflector scalars of x (first entry al, xn2 = the squared norm of the others): beta =
+// -sign(Re al) |x|, kappa = -u_0 / (beta |u_0|^2), 1/beta, 1/|u_0|^2; no reflector (kappa = 0, al kept)
+// where x is already (real, 0, ..., 0).  The square root and the reciprocal start from the hardware's
+// first approximation (relative error about 2^-20) and take one third-order step each, which leaves
+// rounding errors only; both arguments are normal numbers (|u_0|^2 >= |x|^2).
+__device__ __forceinline__ void chase_scalars(double2 al, double xn2, double2& kap, double& beta, double& ib, double& rd) {
+  const double ay2 = al.y * al.y;
+  const double q = fma(al.x, al.x, ay2 + xn2);
+  kap = make_double2(0, 0);
+  beta = al.x;
+  ib = rd = 0.0;
+  if (q >= DBL_MIN && !(xn2 == 0.0 && al.y == 0.0)) {
+    double y, r;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(q));
+    const double t = q * y, e = fma(-t, y, 1.0);         // 1/sqrt(q) = y (1 + e/2 + 3/8 e^2 + O(e^3))
+    const double c = e * fma(e, 0.375, 0.5);
+    const double nr = fma(t, c, t);
+    ib = -copysign(fma(y, c, y), al.x);
+    beta = -copysign(nr, al.x);
+    const double ux = al.x - beta, d = fma(ux, ux, ay2);
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+    const double g = fma(-d, r, 1.0);                    // 1/d = r (1 + g + g^2 + O(g^3))
+    rd = fma(r, fma(g, g, g), r);
+    const double f = -ib * rd;
+    kap = make_double2(f * ux, f * al.y);
   }
 }
+// bounded wait for a phase of an mbarrier; the clock is read every 64 polls (a read takes longer than
+// most waits)
+__device__ __forceinline__ bool mbar_wait_bounded(uint32_t a, uint32_t parity) {
+  unsigned int spins = 0;
+  unsigned long long t0 = 0;
+  while (!tc::mbar_try(a, parity)) {
+    if ((++spins & 63u) == 0u) {
+      if (t0 == 0) t0 = globaltimer();
+      if (globaltimer() - t0 > kWaitNs) return false;
+    }
+  }
+  return true;
+}
+__device__ __forceinline__ bool mbar_test(uint32_t a, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+               : "=r"(ok)
+               : "r"(a), "r"(parity)
+               : "memory");
+  return ok != 0;
+}
 
-__global__ void __launch_bounds__(B4_THREADS) k_bulge4(BulgeArgs a) {
-  extern __shared__ __align__(16) double2 b4sm[];
-  __shared__ int s_bad;
-  const int tid = threadIdx.x;
-  const long long W = (long long)gridDim.x;
-  const long long N = a.N;
+__global__ void __launch_bounds__(CH_THREADS, 1) k_chase(BulgeArgs a) {
+  extern __shared__ __align__(128) double2 ring[];
+  // full: a step's blocks are in its ring slot; empty: every reader has taken them (each arrives after
+  // its wait for full, so the phases stay in step); xr: x of a step is in s_x (4 arrivals); sr: its
+  // scalars are in s_sc; done: every store of a step has been issued
+  __shared__ __align__(8) uint64_t s_full[CH_NS], s_empty[CH_NS], s_done[CH_NX], s_xr[CH_NX], s_sr[CH_NX];
+  __shared__ __align__(16) double2 s_x[CH_NX][BW];
+  __shared__ __align__(16) double s_np[CH_NX][4];    // partial |x_i|^2, i >= 1
+  __shared__ __align__(16) double2 s_sc[CH_NX][2];   // kappa, (beta, 1/beta)
+  __shared__ double s_rd[CH_NX];                     // 1/|u_0|^2
+  __shared__ double2 s_pw[4][4][BW], s_b0[4][BW];    // per group: partial x^H B, first row of B
+  __shared__ double2 s_wv[16][BW];                   // per warp: w of the B and D updates
+  __shared__ double2 s_y[4][BW], s_d0[4][BW];        // by step mod 4: D x, first column of D
+  // the warp's index as a value that is uniform by construction, and (below) waits that end by a vote:
+  // where the compiler can see that a warp is together, a shuffle is one instruction, else a guarded one
+  const int lane = threadIdx.x & 31, wid = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+  const int N = (int)a.N;
   const long long np = a.nprob;
-  // same sweep order and wait rule as k_bulge, one CTA per sweep
-  for (long long u = blockIdx.x; u < np * (N - 1); u += W) {
-    const long long q = u % np, s = u / np;
-    BulgeArgs b = a;
-    b.AB = a.AB + q * a.ab_stride;
-    unsigned int* prog = a.prog + q * a.prog_stride;
-    const long long ns = nsteps_of(N, s);
-    const long long nprev = (s > 0) ? nsteps_of(N, s - 1) : 0;
-    double2* Bb = b4sm;                // roles of the three tiles rotate between steps
-    double2* Db = b4sm + BW * BG_LD;
-    double2* B1b = Db + BW * BG_LD;
-    double2* tail = b4sm + 3 * BW * BG_LD;
-    double2 gv[NGMAX];
-    bool pre = false;
-    for (long long t = 0; t < ns; ++t) {
-      if (tid == 0) s_bad = (s > 0 && !wait_at_least(prog + s - 1, (unsigned int)min(t + 3, nprev), a.err)) ? 1 : 0;
-      __syncthreads();
-      if (s_bad) return;
-      bulge_step4(b, s, t, Bb, Db, B1b, tail, gv, pre);
-      // publish: the CTA barrier orders every thread's writes before the release store, issued
-      // by warp 3 so that its latency overlaps thread 0's wait for the next step
-      __syncthreads();
-      if (tid == 96) st_release(prog + s, (unsigned int)(t + 1));
-      pre = false;
-      if (t + 1 < ns) {
-        // Prefetch for step t + 1 (rows r0n = r0 + 32 on): its bulge block is this step's block
-        // below (updated in place); its diagonal block, its block below and the velocity rows
-        // are final already: the predecessor sweep's steps <= t + 2 that write them are done
-        // (this step waited for t + 3), this step wrote none of them, and of the predecessor's
-        // step t + 3 only the corner (31, 31) of the block below overlaps (read after the wait).
-        // The successor sweep runs at most step t - 1 from now on and touches rows above.
-        double2* tmp = Bb;
-        Bb = B1b;
-        B1b = tmp;
-        const long long r0n = s + 1 + (t + 1) * BW;
-        const int Ln = (int)min((long long)BW, N - r0n);
-        const long long r1n = r0n + Ln;
-        const int L1n = (r1n < N) ? (int)min((long long)BW, N - r1n) : 0;
-        if (tid < 96) {
-          for (int e = tid; e < BW * BW; e += 96) {
-            const int i = e & 31, q = e >> 5;
-            if (q < Ln) {
-              const bool ok = i >= q && i < Ln;
-              cpa16(Db + i * BG_LD + q, ok ? b.AB + (r0n + q) * LDB + (i - q) : b.AB, ok);
-              if (!(i == BW - 1 && q == BW - 1 && Ln == BW && L1n == BW))
-                cpa16(B1b + i * BG_LD + q, b.AB + (r0n + q) * LDB + (Ln + i - q), i < L1n);
-            }
-          }
-          asm volatile("cp.async.commit_group;" ::: "memory");
+  if (threadIdx.x == 0) {
+    for (int k = 0; k < CH_NS; ++k) {
+      tc::mbar_init(tc::smem_u32(&s_full[k]), 32);    // the producer's lanes
+      tc::mbar_init(tc::smem_u32(&s_empty[k]), 10);   // B1 4, D 4, velocity, publisher
+    }
+    for (int k = 0; k < CH_NX; ++k) {
+      tc::mbar_init(tc::smem_u32(&s_done[k]), 9);     // B 4, D 4, velocity
+      tc::mbar_init(tc::smem_u32(&s_xr[k]), 4);
+      tc::mbar_init(tc::smem_u32(&s_sr[k]), 1);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  static_assert((CH_NS & (CH_NS - 1)) == 0 && (CH_NX & (CH_NX - 1)) == 0, "ring sizes are powers of two");
+  // Every wait is bounded.  A wait on another sweep that runs out sets *err, after which this CTA
+  // goes on without waiting for its predecessors (indices stay in range, the results are void); the
+  // copies it issues always complete, so the waits inside the CTA end as well.
+  auto wait_bar = [&](uint64_t* b, int cnt, int n) {
+    if (!mbar_wait_bounded(tc::smem_u32(b + (n & (cnt - 1))), (unsigned)(n / cnt) & 1u)) atomicExch(a.err, 1);
+  };
+  // the same by all lanes of a warp, which leave together
+  auto wait_warp = [&](uint64_t* b, int cnt, int n) {
+    const uint32_t bar = tc::smem_u32(b + (n & (cnt - 1))), par = (unsigned)(n / cnt) & 1u;
+    unsigned int spins = 0;
+    unsigned long long t0 = 0;
+    while (!__all_sync(0xffffffffu, tc::mbar_try(bar, par))) {
+      if ((++spins & 63u) == 0u) {
+        const unsigned long long now = globaltimer();
+        if (t0 == 0) t0 = now;
+        if (__any_sync(0xffffffffu, now - t0 > kWaitNs)) {
+          if (lane == 0) atomicExch(a.err, 1);
+          break;
         }
-        if (tid < 32) {
-#pragma unroll
-          for (int al2 = 0; al2 < NGMAX; ++al2)
-            gv[al2] = (al2 < a.ng && tid < Ln) ? __ldcg(a.g + (long long)al2 * N + r0n + tid) : make_double2(0, 0);
-        }
-        pre = true;
       }
     }
+  };
+  auto arrive = [&](uint64_t* b, int cnt, int n) {
+    __syncwarp();
+    if (lane == 0) tc::mbar_arrive(tc::smem_u32(b + (n & (cnt - 1))));
+  };
+  const int grp = wid >> 2, wg = wid & 3;
+  int ig = lane & 3, qb = 4 * ((lane >> 2) & 1) + (lane >> 3);
+  int i0 = 8 * wg + ig;
+  asm("" : "+r"(qb), "+r"(i0));   // opaque: the compiler folded the tests i >= c below wrongly from the bit ranges
+  const int lb = (LDB - 1) * qb + i0;   // lane offset of a block's elements; element (r, m) at lb + EM m + 4 r
+  constexpr int EM = 8 * (LDB - 1);
+  int n = 0;   // steps of this CTA so far
+  // sweep u of the launch = sweep s = u / np of band u % np: a sweep waits only on sweep s-1 of its
+  // own band, which has a smaller u and is running or finished.  Each role loops by itself (one loop
+  // around the roles would keep the block warps' registers alive in all of them).
+  auto sweeps = [&](auto&& body) {
+    for (long long u = blockIdx.x; u < np * (N - 1); u += gridDim.x) {
+      const int q = (int)(u % np), s = (int)(u / np);
+      body(a.AB + q * a.ab_stride, a.prog + q * a.prog_stride, s, (int)nsteps_of(N, s));
+    }
+  };
+  if (wid == 17) {   // producer
+    bool alone = false;   // a wait on a predecessor has failed
+    sweeps([&](double2* AB, unsigned int* prog, int s, int ns) {
+      const int nprev = (s > 0) ? (int)nsteps_of(N, s - 1) : 0;
+      int seen = 0;
+      const double2* src = AB + (long long)(s + 1) * LDB + lane;
+      for (int t = 0; t < ns; ++t, ++n, src += CH_BLK) {
+        if (n >= CH_NS) wait_bar(s_empty, CH_NS, n - CH_NS);
+        const int need = min(t + 3, nprev);
+        if (lane == 0 && s > 0 && seen < need && !alone) {
+          alone = !wait_at_least(prog + s - 1, (unsigned)need, a.err);
+          seen = (int)ld_acquire(prog + s - 1);
+        }
+        __syncwarp();
+        const uint32_t dst = tc::smem_u32(ring + (n & (CH_NS - 1)) * CH_SLOT + lane);
+        auto cp = [](uint32_t d, const double2* g) {
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(g) : "memory");
+        };
+        // column c: its block below (entries 32 - c .. 63 - c) is in its second half and, from 32 - c
+        // on, its first; the diagonal block in its first
+#pragma unroll
+        for (int c = 0; c < BW; ++c) cp(dst + (c * LDB + BW) * 16, src + c * LDB + BW);
+#pragma unroll
+        for (int c = 0; c < BW; ++c) cp(dst + c * LDB * 16, src + c * LDB);
+        if (t == 0) {
+          cp(dst + CH_BLK * 16, AB + (long long)s * LDB + lane);
+          if (lane == 0) cp(dst + (CH_BLK + BW) * 16, AB + (long long)s * LDB + BW);
+        }
+        const double2* gp = a.g + min(s + 1 + t * BW + lane, N - 1);
+        for (int al = 0; al < a.ng; ++al, gp += N) cp(dst + (CH_BLK + LDB + al * BW) * 16, gp);
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(tc::smem_u32(&s_full[n & (CH_NS - 1)])) : "memory");
+      }
+    });
+  } else if (wid == 18) {   // publisher: a step whose successor is finished too is left to that one
+    sweeps([&](double2*, unsigned int* prog, int s, int ns) {
+      if (lane == 0)
+        for (int t = 0; t < ns; ++t, ++n) {
+          tc::mbar_arrive(tc::smem_u32(&s_empty[n & (CH_NS - 1)]));
+          wait_bar(s_done, CH_NX, n);
+          if (t + 1 < ns && mbar_test(tc::smem_u32(&s_done[(n + 1) & (CH_NX - 1)]), (unsigned)((n + 1) / CH_NX) & 1u)) continue;
+          st_release(prog + s, (unsigned int)(t + 1));
+        }
+    });
+  } else if (grp == 4) {
+    sweeps([&](double2*, unsigned int*, int s, int ns) {
+      // velocity vectors g <- g - kappa conj(u) (u^T g), five at a time, and the stored reflector
+      for (int t = 0; t < ns; ++t, ++n) {
+        const int r0 = s + 1 + t * BW, L = min(BW, N - r0), xb = n & (CH_NX - 1);
+        const double2* sl = ring + (n & (CH_NS - 1)) * CH_SLOT + CH_BLK + LDB + lane;
+        wait_warp(s_full, CH_NS, n);
+        wait_warp(s_sr, CH_NX, n);
+        const double2 kap = s_sc[xb][0], bi = s_sc[xb][1];
+        double2 uv = s_x[xb][lane];
+        if (lane == 0) uv.x -= bi.x;
+        const double2 ku = cmulc(uv, kap);
+        double2* gp = a.g + r0 + lane;
+        for (int j0 = 0; j0 < a.ng; j0 += 5, sl += 5 * BW) {
+          double2 gv[5], p[5];
+#pragma unroll
+          for (int j = 0; j < 5; ++j) {
+            gv[j] = lane < L ? sl[j * BW] : make_double2(0, 0);
+            p[j] = cmul(uv, gv[j]);
+          }
+          // the five sums over the 32 rows: halves exchanged over lane bits 4, 3 and 2 (8 slots, 3 of
+          // them empty), so that lane bits (4, 3, 2) = j end with sum j; then over bits 1 and 0
+          const double2 z0 = make_double2(0, 0);
+          const bool h4 = lane & 16, h3 = lane & 8, h2 = lane & 4;
+          const double2 e1 = shfl2_xor(p[1], 16), e2 = shfl2_xor(p[2], 16), e3 = shfl2_xor(p[3], 16);
+          const double2 a0 = cadd(h4 ? p[4] : p[0], shfl2_xor(h4 ? p[0] : p[4], 16));
+          const double2 a1 = h4 ? z0 : cadd(p[1], e1), a2 = h4 ? z0 : cadd(p[2], e2), a3 = h4 ? z0 : cadd(p[3], e3);
+          const double2 b0 = cadd(h3 ? a2 : a0, shfl2_xor(h3 ? a0 : a2, 8));
+          const double2 b1 = cadd(h3 ? a3 : a1, shfl2_xor(h3 ? a1 : a3, 8));
+          double2 c = cadd(h2 ? b1 : b0, shfl2_xor(h2 ? b0 : b1, 4));
+          c = cadd(c, shfl2_xor(c, 2));
+          c = cadd(c, shfl2_xor(c, 1));
+#pragma unroll
+          for (int j = 0; j < 5; ++j, gp += N) {
+            const double2 sg = shfl2(c, 4 * j);   // sum j sits in the lanes 4j .. 4j+3
+            if (lane < L) *gp = cfms(ku, sg, gv[j]);
+          }
+        }
+        arrive(s_empty, CH_NS, n);   // after the scalars: by then the first x has been read as well
+        if (a.store) {
+          // tau = -u_0 / beta, v = u / u_0
+          const double2 u0 = make_double2(s_x[xb][0].x - bi.x, s_x[xb][0].y);
+          double2 v = make_double2(lane == 0 ? 1.0 : 0.0, 0.0), tau = make_double2(0, 0);
+          if (kap.x != 0.0 || kap.y != 0.0) {
+            tau = cscale(u0, -bi.y);
+            if (lane > 0) v = cscale(cmulc(u0, uv), s_rd[xb]);
+          }
+          if (lane < L) a.A[(r0 + lane - s - 1) + (long long)(N - 1 - s) * N] = v;
+          if (lane == 0) a.tau2[tau2_offset(N, s) + t] = tau;
+        }
+        arrive(s_done, CH_NX, n);
+      }
+    });
+  } else {
+    double2 M[2][4] = {};
+    const int ub = (LDB - 1) * i0 + qb;   // lane offset of D's mirrored elements: ub + 8 m + 4 (LDB - 1) r
+    // z = M x over the warp's rows, the same in the 8 lanes of a row
+    auto dot_rows = [&](const double2* x, double2(&z)[2]) {
+      double2 xq[4];
+#pragma unroll
+      for (int m = 0; m < 4; ++m) xq[m] = x[qb + 8 * m];
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+        z[r] = cadd(cfma(M[r][1], xq[1], cmul(M[r][0], xq[0])), cfma(M[r][3], xq[3], cmul(M[r][2], xq[2])));
+#pragma unroll
+      for (int o = 4; o <= 16; o <<= 1)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) z[r] = cadd(z[r], shfl2_xor(z[r], o));
+    };
+    // x of step n1 into s_x (lanes 0..3 of the group's warps: rows i0, i0 + 4), with its partial norm
+    auto post_x = [&](int n1, double2 x0, double2 x1) {
+      const int xn = n1 & (CH_NX - 1);
+      double pn = fma(x1.x, x1.x, x1.y * x1.y);
+      if (i0 > 0) pn = fma(x0.x, x0.x, fma(x0.y, x0.y, pn));
+      pn += __shfl_xor_sync(0xffffffffu, pn, 1);
+      pn += __shfl_xor_sync(0xffffffffu, pn, 2);
+      if (lane < 4) {
+        s_x[xn][i0] = x0;
+        s_x[xn][i0 + 4] = x1;
+      }
+      if (lane == 0) s_np[xn][wg] = pn;
+      bar_arrive(1 + (n1 & 1), 256);
+      arrive(s_xr, CH_NX, n1);
+    };
+    sweeps([&](double2* AB, unsigned int*, int s, int ns) {
+      for (int t = 0; t < ns; ++t, ++n) {
+        const int r0 = s + 1 + t * BW, xb = n & (CH_NX - 1);
+        const double2* sl = ring + (n & (CH_NS - 1)) * CH_SLOT;
+        const int role = (n - grp) & 3;
+        if (role == 0) {
+          // ---- the block below, B1 <- B1 H
+          wait_warp(s_full, CH_NS, n);
+#pragma unroll
+          for (int r = 0; r < 2; ++r)
+#pragma unroll
+            for (int m = 0; m < 4; ++m) M[r][m] = sl[lb + BW + EM * m + 4 * r];
+          arrive(s_empty, CH_NS, n);
+          bar_sync(1 + (n & 1), 256);   // x
+          double2 z[2], kap;
+          double beta, ib, rd;
+          const double2* xs = s_x[xb];
+          const double* pn = s_np[xb];
+          chase_scalars(xs[0], (pn[0] + pn[1]) + (pn[2] + pn[3]), kap, beta, ib, rd);
+          dot_rows(xs, z);
+          // x is read again below rather than kept: registers
+          asm volatile("" ::: "memory");
+#pragma unroll
+          for (int r = 0; r < 2; ++r) z[r] = cmul(kap, caxpy(-beta, shfl2(M[r][0], ig), z[r]));
+          {
+            double2 x0 = xs[qb];
+            if (qb == 0) x0.x -= beta;
+#pragma unroll
+            for (int r = 0; r < 2; ++r) M[r][0] = cfmsc(x0, z[r], M[r][0]);
+          }
+          if (t + 1 < ns) post_x(n + 1, M[0][0], M[1][0]);
+          if (wg == 0) {
+            if (lane == 0) {
+              s_sc[xb][0] = kap;
+              s_sc[xb][1] = make_double2(beta, ib);
+              s_rd[xb] = rd;
+            }
+            arrive(s_sr, CH_NX, n);
+          }
+          if (t + 1 < ns) {
+#pragma unroll
+            for (int m = 1; m < 4; ++m) {
+              const double2 xm = xs[qb + 8 * m];
+#pragma unroll
+              for (int r = 0; r < 2; ++r) M[r][m] = cfmsc(xm, z[r], M[r][m]);
+            }
+            // partial x^H B of the next step: x of the own rows is column 0
+            const double2 x0 = shfl2(M[0][0], ig), x1 = shfl2(M[1][0], ig);
+            double2 p[4];
+#pragma unroll
+            for (int m = 0; m < 4; ++m) p[m] = cfmac(x1, M[1][m], cmulc(x0, M[0][m]));
+            // sums over the 4 lanes of a column group; lane (bit 0, bit 1) ends with m = 2 bit0 + bit1
+            const bool b0 = lane & 1, b1 = lane & 2;
+            double2 e0 = b0 ? p[2] : p[0], e1 = b0 ? p[3] : p[1];
+            e0 = cadd(e0, shfl2_xor(b0 ? p[0] : p[2], 1));
+            e1 = cadd(e1, shfl2_xor(b0 ? p[1] : p[3], 1));
+            s_pw[grp][wg][qb + 16 * (lane & 1) + 4 * (lane & 2)] = cadd(b1 ? e1 : e0, shfl2_xor(b1 ? e0 : e1, 2));
+            if (i0 == 0)
+#pragma unroll
+              for (int m = 0; m < 4; ++m) s_b0[grp][qb + 8 * m] = M[0][m];
+          }
+        } else if (role == 1) {
+          const bool in0 = i0 < N - r0, in1 = i0 + 4 < N - r0;
+          if (t > 0) {
+            // ---- B <- H^H B, stored
+            double2 xi[2];
+            xi[0] = shfl2(M[0][0], ig);
+            xi[1] = shfl2(M[1][0], ig);
+            bar_sync(3 + grp, 128);   // s_pw, s_b0
+            const double2(*pw)[BW] = s_pw[grp];
+            const double2 w = cadd(cadd(pw[0][lane], pw[1][lane]), cadd(pw[2][lane], pw[3][lane]));
+            const double2 br = s_b0[grp][lane];
+            double2* dst = AB + (long long)(r0 - BW) * LDB + lb + BW;
+            wait_warp(s_sr, CH_NX, n);
+            const double beta = s_sc[xb][1].x;
+            double2* wv = s_wv[wid];
+            wv[lane] = cmulc(s_sc[xb][0], caxpy(-beta, br, w));
+            __syncwarp();
+            if (i0 == 0) xi[0].x -= beta;
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+              const double2 cw = wv[qb + 8 * m];
+              double2 v0 = cfms(xi[0], cw, M[0][m]), v1 = cfms(xi[1], cw, M[1][m]);
+              if (m == 0 && qb == 0) {   // the annihilated column
+                v0 = make_double2(i0 == 0 ? beta : 0.0, 0.0);
+                v1 = make_double2(0.0, 0.0);
+              }
+              if (in0) dst[EM * m] = v0;
+              if (in1) dst[EM * m + 4] = v1;
+            }
+          } else {
+            // first step: x is column s below its diagonal, which becomes (beta, 0, ..., 0)
+            wait_warp(s_full, CH_NS, n);
+            double2 x0 = make_double2(0, 0), x1 = x0;
+            if (lane < 4) {
+              x0 = sl[CH_BLK + 1 + i0];
+              x1 = sl[CH_BLK + 5 + i0];
+            }
+            post_x(n, x0, x1);
+            wait_warp(s_sr, CH_NX, n);
+            double2* dst = AB + (long long)s * LDB + 1 + i0;
+            if (lane < 4 && in0) dst[0] = make_double2(i0 == 0 ? s_sc[xb][1].x : 0.0, 0.0);
+            if (lane < 4 && in1) dst[4] = make_double2(0.0, 0.0);
+          }
+          arrive(s_done, CH_NX, n);
+        } else if (role == 2) {
+          // ---- the diagonal block, D <- H^H D H
+          const int yb = n & 3;
+          wait_warp(s_full, CH_NS, n);
+          // the stored lower triangle, the rest mirrored
+#pragma unroll
+          for (int r = 0; r < 2; ++r)
+#pragma unroll
+            for (int m = 0; m < 4; ++m) {
+              const int d = i0 + 4 * r - (qb + 8 * m);
+              M[r][m] = sl[d >= 0 ? lb + EM * m + 4 * r : ub + 8 * m + 4 * (LDB - 1) * r];
+              M[r][m].y = d > 0 ? M[r][m].y : (d < 0 ? -M[r][m].y : 0.0);
+            }
+          arrive(s_empty, CH_NS, n);
+          wait_warp(s_xr, CH_NX, n);
+          double2 y[2];
+          dot_rows(s_x[xb], y);
+          if (lane < 4) {
+            s_y[yb][i0] = y[0];
+            s_y[yb][i0 + 4] = y[1];
+            s_d0[yb][i0] = M[0][0];
+            s_d0[yb][i0 + 4] = M[1][0];
+          }
+          bar_sync(3 + grp, 128);
+          double2 yl = s_y[yb][lane];
+          const double2 d0 = s_d0[yb][lane];
+          double2 ul = s_x[xb][lane];
+          wait_warp(s_sr, CH_NX, n);
+          const double2 kap = s_sc[xb][0];
+          const double beta = s_sc[xb][1].x;
+          // lane = row: w = kappa y - 1/2 |kappa|^2 (u^H y) u, y = D u; then D <- D - u w^H - w u^H
+          if (lane == 0) ul.x -= beta;
+          yl = caxpy(-beta, d0, yl);
+          const double hk = 0.5 * fma(kap.x, kap.x, kap.y * kap.y) * warp_sum(fma(ul.x, yl.x, ul.y * yl.y));
+          double2* wv = s_wv[wid];
+          wv[lane] = caxpy(-hk, ul, cmul(kap, yl));
+          __syncwarp();
+          double2 ui[2], wi[2];
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            ui[r] = s_x[xb][i0 + 4 * r];
+            wi[r] = wv[i0 + 4 * r];
+          }
+          if (i0 == 0) ui[0].x -= beta;
+          double2* dst = AB + (long long)r0 * LDB + lb;
+          const bool in0 = i0 < N - r0, in1 = i0 + 4 < N - r0;
+#pragma unroll
+          for (int m = 0; m < 4; ++m) {
+            if (m > wg) break;   // above the diagonal for every row of the warp
+            const double2 wq = wv[qb + 8 * m];
+            double2 xm = s_x[xb][qb + 8 * m];
+            if (m == 0 && qb == 0) xm.x -= beta;
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+              const int d = i0 + 4 * r - (qb + 8 * m);
+              double2 v = cfmsc(wq, ui[r], cfmsc(xm, wi[r], M[r][m]));
+              if (d == 0) v.y = 0.0;
+              if (d >= 0 && (r ? in1 : in0)) dst[EM * m + 4 * r] = v;
+            }
+          }
+          arrive(s_done, CH_NX, n);
+        }
+      }
+    });
   }
 }
 
@@ -1462,7 +1701,7 @@ static int two_stage_buffers(wtbg_ctx* ctx, int nband) {
   ENSURE(ctx->t2T, (size_t)std::max<long long>(npan, 1) * 1024 * 16);
   ENSURE(ctx->t2P, (size_t)nsm * (16 + 2 * 16 * BW + 16 * BW * BW + 16 * BW * NGMAX) + 4096 +
                         (size_t)std::max<long long>(npan, 1) * 4);
-  ENSURE(ctx->t2AB, (size_t)nband * N * LDB * 16);
+  ENSURE(ctx->t2AB, (size_t)nband * (N + AB_PAD) * LDB * 16);
   ENSURE(ctx->t2prog, (size_t)nband * N * 4 + 64);
   ENSURE(ctx->triErr, 16);
   return 0;
@@ -1609,7 +1848,7 @@ static int run_stage1(wtbg_ctx* ctx, int ng, int band) {
     mark(pl, 5);
     her2k_flops[pl] = (double)ml * (ml + 1.0) * 0.5 * 16.0 * Kg;
   }
-  k_band_extract<<<(unsigned)N, 128, 0, s>>>(A, N, ctx->t2AB.as<double2>() + (size_t)band * N * LDB);
+  k_band_extract<<<(unsigned)(N + AB_PAD), BW * 2, 0, s>>>(A, N, ctx->t2AB.as<double2>() + (size_t)band * (N + AB_PAD) * LDB);
   WTBG_COUNT(ctx, 1);
   CKL("k_band_extract");
   if (prof) {
@@ -1667,7 +1906,7 @@ static int run_stage2(wtbg_ctx* ctx, int nband, int ng, bool store, double* dd, 
   ba.err = ctx->triErr.as<int>();
   ba.store = store ? 1 : 0;
   ba.nprob = nband;
-  ba.ab_stride = N * LDB;
+  ba.ab_stride = (N + AB_PAD) * LDB;
   ba.prog_stride = N;
   const long long nsweep = (long long)nband * (N - 1);
   if (ctx->bulge_warp_mode) {   // one warp per sweep
@@ -1679,16 +1918,14 @@ static int run_stage2(wtbg_ctx* ctx, int nband, int ng, bool store, double* dd, 
                                                                     (nsweep + BG_WARPS - 1) / BG_WARPS));
     void* args[] = {&ba};
     CK(cudaLaunchCooperativeKernel((const void*)k_bulge, dim3(gb), dim3(32 * BG_WARPS), args, bsm, s));
-  } else {   // one CTA of four warps per sweep
-    CK(cudaFuncSetAttribute(k_bulge4, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)B4_SMEM));
-    int per = 1;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_bulge4, B4_THREADS, B4_SMEM));
-    const int gb = (int)std::max<long long>(1, std::min<long long>((long long)nsm * std::max(per, 1), nsweep));
+  } else {   // one CTA per sweep
+    CK(cudaFuncSetAttribute(k_chase, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CH_SMEM));
+    const int gb = (int)std::max<long long>(1, std::min<long long>(nsm, nsweep));
     void* args[] = {&ba};
-    CK(cudaLaunchCooperativeKernel((const void*)k_bulge4, dim3(gb), dim3(B4_THREADS), args, B4_SMEM, s));
+    CK(cudaLaunchCooperativeKernel((const void*)k_chase, dim3(gb), dim3(CH_THREADS), args, CH_SMEM, s));
   }
   for (int q = 0; q < nband; ++q)
-    k_band_to_tridiag<<<(int)((N + 255) / 256), 256, 0, s>>>(AB + (size_t)q * N * LDB, N, dd + (size_t)q * N,
+    k_band_to_tridiag<<<(int)((N + 255) / 256), 256, 0, s>>>(AB + (size_t)q * (N + AB_PAD) * LDB, N, dd + (size_t)q * N,
                                                               ee + (size_t)q * N);
   WTBG_COUNT(ctx, 1 + nband);
   CKL("two-stage bulge chasing");
