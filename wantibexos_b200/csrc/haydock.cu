@@ -66,12 +66,13 @@ __global__ void __launch_bounds__(256) k_chain_dot(const double2* Vv, const doub
   }
 }
 
-__global__ void k_chain_reduce(const double* part, int nparts, int ncomp, double* out) {
-  const int c = threadIdx.x;
-  if (c >= ncomp) return;
+// sum of the row blocks' partials, one warp per chain, lanes over the blocks (fixed order)
+__global__ void k_chain_reduce(const double* __restrict__ part, int nparts, int ncomp, double* __restrict__ out) {
+  const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;
   double s = 0;
-  for (int k = 0; k < nparts; ++k) s += part[(long long)k * MAXC + c];
-  out[c] = s;
+  for (int k = lane; k < nparts; k += 32) s += part[(long long)k * MAXC + c];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) out[c] = s;
 }
 
 // w <- w - a v - b vp  (a = alpha_j, b = beta_{j-1})
@@ -157,47 +158,42 @@ __global__ void k_cfrac(const double* alpha, const double* beta, const double* n
 }
 
 // eps from the chain Green functions: diagonal components directly, off-diagonal ones by
-// polarisation; then imagrenorm against E_1 and real(spinf * x)
-__global__ void k_haydock_eps(const double* om, const double* gre, const double* gim, int nw, int nout,
-                              const int* ocode, double caux, double e1, int renorm, double spinf, double* re, double* im,
-                              float* eps) {
-  const int o = threadIdx.x;
-  if (o >= nout) return;
+// polarisation; then imagrenorm against E_1 and real(spinf * x).  One block per output component; the
+// edge is the first photon energy above E_1 - 0.15, as in k_renorm_out.
+constexpr int kEpsThreads = 512;
+__global__ void __launch_bounds__(kEpsThreads) k_haydock_eps(const double* __restrict__ om, const double* __restrict__ gre,
+                                                             const double* __restrict__ gim, int nw,
+                                                             const int* __restrict__ ocode, double caux, double e1, int renorm,
+                                                             double spinf, float* __restrict__ eps) {
+  const int o = blockIdx.x, tid = threadIdx.x;
   const int kind = ocode[2 * o], idx = ocode[2 * o + 1];
-  double* ro = re + (long long)o * nw;
-  double* io = im + (long long)o * nw;
-  for (int j = 0; j < nw; ++j) {
-    double r, i;
-    if (kind == 0) {   // diagonal: chain idx
-      r = gre[(long long)idx * nw + j];
-      i = gim[(long long)idx * nw + j];
-    } else {           // off-diagonal: chains idx (plus) and idx+1 (minus)
-      r = 0.25 * (gre[(long long)idx * nw + j] - gre[(long long)(idx + 1) * nw + j]);
-      i = 0.25 * (gim[(long long)idx * nw + j] - gim[(long long)(idx + 1) * nw + j]);
-    }
-    const double delta = (kind == 0) ? 1.0 : 0.0;
-    ro[j] = delta + r * caux;
-    io[j] = i * caux;
+  const double* r0 = gre + (long long)idx * nw;
+  const double* i0 = gim + (long long)idx * nw;
+  // kind 0: chain idx; else the chains idx (plus) and idx + 1 (minus)
+  auto imag = [&](int j) { return (kind == 0 ? i0[j] : 0.25 * (i0[j] - i0[nw + j])) * caux; };
+  const double aux = e1 - (double)0.15f;
+  const bool on = renorm && !(aux <= 0.000);
+  __shared__ int s_first;
+  if (tid == 0) s_first = nw;
+  __syncthreads();
+  if (on) {
+    int first = nw;
+    for (int i = tid; i < nw && first == nw; i += kEpsThreads)
+      if (!(om[i] <= aux)) first = i;
+    if (first < nw) atomicMin(&s_first, first);
   }
-  if (renorm) {
-    const double aux = e1 - (double)0.15f;
-    if (!(aux <= 0.000)) {
-      int ibegin = 1;
-      for (int i = 1; i <= nw; ++i) {
-        if (om[i - 1] <= aux) ibegin = i;
-        else break;
-      }
-      const double aux3 = (ibegin < nw) ? io[ibegin] : 0.0;
-      for (int i = 1; i <= ibegin; ++i) io[i - 1] = 0.0;
-      for (int i = ibegin + 1; i <= nw; ++i) {
-        const double v = io[i - 1] - aux3;
-        io[i - 1] = (v < 0.0) ? 0.0 : v;
-      }
+  __syncthreads();
+  const int ibegin = max(s_first, 1);
+  const double aux3 = (on && ibegin < nw) ? imag(ibegin) : 0.0;
+  for (int j = tid; j < nw; j += kEpsThreads) {
+    const double r = kind == 0 ? r0[j] : 0.25 * (r0[j] - r0[nw + j]);
+    double v = imag(j);
+    if (on) {
+      v = v - aux3;
+      v = (j < ibegin || v < 0.0) ? 0.0 : v;
     }
-  }
-  for (int j = 0; j < nw; ++j) {
-    eps[(long long)j + (long long)nw * (0 + 2 * o)] = (float)(spinf * ro[j]);
-    eps[(long long)j + (long long)nw * (1 + 2 * o)] = (float)(spinf * io[j]);
+    eps[(long long)j + (long long)nw * (0 + 2 * o)] = (float)(spinf * ((kind == 0 ? 1.0 : 0.0) + r * caux));
+    eps[(long long)j + (long long)nw * (1 + 2 * o)] = (float)(spinf * v);
   }
 }
 
@@ -231,18 +227,18 @@ int run_haydock(wtbg_ctx* ctx, int K, int ncomp, const int* codes, std::vector<d
   CK(cudaMemsetAsync(db0, 0, MAXC * 8, s));
   k_chain_init<<<nparts, th, 0, s>>>(ctx->h.as<double2>(), N, ncomp, dcode, V); WTBG_COUNT(ctx, 1);
   k_chain_dot<<<nparts, th, 0, s>>>(V, V, N, ncomp, 0, part); WTBG_COUNT(ctx, 1);
-  k_chain_reduce<<<1, 32, 0, s>>>(part, nparts, ncomp, dn2); WTBG_COUNT(ctx, 1);
+  k_chain_reduce<<<1, 32 * ncomp, 0, s>>>(part, nparts, ncomp, dn2); WTBG_COUNT(ctx, 1);
   k_chain_next<<<nparts, th, 0, s>>>(V, V, VP, N, ncomp, dn2); WTBG_COUNT(ctx, 1);   // v = u/|u|, vp = u (reset below)
   CK(cudaMemsetAsync(VP, 0, (size_t)N * m * 16, s));
   CKL("haydock init");
   for (int j = 0; j < K; ++j) {
     if (int r = run_hemm_narrow(ctx, V, (int)N, m, Wv, (int)N)) return r;
     k_chain_dot<<<nparts, th, 0, s>>>(V, Wv, N, ncomp, 1, part); WTBG_COUNT(ctx, 1);
-    k_chain_reduce<<<1, 32, 0, s>>>(part, nparts, ncomp, dal + (size_t)j * MAXC); WTBG_COUNT(ctx, 1);
+    k_chain_reduce<<<1, 32 * ncomp, 0, s>>>(part, nparts, ncomp, dal + (size_t)j * MAXC); WTBG_COUNT(ctx, 1);
     const double* bprev = (j == 0) ? db0 : dbe + (size_t)(j - 1) * MAXC;
     k_chain_axpy<<<nparts, th, 0, s>>>(Wv, V, VP, N, ncomp, dal + (size_t)j * MAXC, bprev); WTBG_COUNT(ctx, 1);
     k_chain_dot<<<nparts, th, 0, s>>>(Wv, Wv, N, ncomp, 0, part); WTBG_COUNT(ctx, 1);
-    k_chain_reduce<<<1, 32, 0, s>>>(part, nparts, ncomp, dbe + (size_t)j * MAXC); WTBG_COUNT(ctx, 1);
+    k_chain_reduce<<<1, 32 * ncomp, 0, s>>>(part, nparts, ncomp, dbe + (size_t)j * MAXC); WTBG_COUNT(ctx, 1);
     k_chain_next<<<nparts, th, 0, s>>>(Wv, V, VP, N, ncomp, dbe + (size_t)j * MAXC); WTBG_COUNT(ctx, 1);
     k_copy_scalar<<<1, 32, 0, s>>>(dbe + (size_t)j * MAXC, dbe + (size_t)j * MAXC, ncomp, 1); WTBG_COUNT(ctx, 1);
   }
@@ -271,12 +267,10 @@ int run_haydock_spectrum(wtbg_ctx* ctx, int K, int nchain, const double* alpha, 
                          double numbse, double eta, double e1, int renorm, double spinf, double* d_om, float* d_eps) {
   const int nw = (int)numbse;
   cudaStream_t s = ctx->stream;
-  ENSURE(ctx->sp_out, (size_t)(2 * nchain + 2 * nout) * nw * 8 + (size_t)(2 * K + 1) * nchain * 8 + 64 * 4 + 64);
+  ENSURE(ctx->sp_out, (size_t)2 * nchain * nw * 8 + (size_t)(2 * K + 1) * nchain * 8 + 64 * 4 + 64);
   double* gre = ctx->sp_out.as<double>();
   double* gim = gre + (size_t)nchain * nw;
-  double* re = gim + (size_t)nchain * nw;
-  double* im = re + (size_t)nout * nw;
-  double* da = im + (size_t)nout * nw;
+  double* da = gim + (size_t)nchain * nw;
   double* db = da + (size_t)K * nchain;
   double* dn = db + (size_t)K * nchain;
   int* doc = reinterpret_cast<int*>(dn + nchain);
@@ -289,7 +283,7 @@ int run_haydock_spectrum(wtbg_ctx* ctx, int K, int nchain, const double* alpha, 
                                                     gim); WTBG_COUNT(ctx, 1);
   const double baux = (double)(float)(ngrid[0] * ngrid[1] * ngrid[2]) * vcell3d;
   const double caux = (double)180.90f / (baux * 1.0);
-  k_haydock_eps<<<1, 32, 0, s>>>(d_om, gre, gim, nw, nout, doc, caux, e1, renorm, spinf, re, im, d_eps); WTBG_COUNT(ctx, 1);
+  k_haydock_eps<<<nout, kEpsThreads, 0, s>>>(d_om, gre, gim, nw, doc, caux, e1, renorm, spinf, d_eps); WTBG_COUNT(ctx, 1);
   CKL("haydock spectrum");
   return 0;
 }

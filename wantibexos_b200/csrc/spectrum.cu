@@ -18,12 +18,27 @@
 
 namespace {
 
-__global__ void k_avgsme(const double* e, int n, double sme, double* eta_out) {
-  // sequential, in the reference's order (one thread)
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// eta of avgsme: one block, each thread sums the level distances of its stride and the block adds the
+// threads' sums in a tree.  One thread in the reference's order was a chain of 2 n dependent
+// additions behind uncached loads: with k_renorm_out 1.0 ms of a spectrum at n = 576, 1.8 ms at
+// 14400 (2001 energies); the two take 0.01 ms now.  The sum differs from the ordered one by rounding.
+constexpr int kAvgThreads = 1024;
+__global__ void __launch_bounds__(kAvgThreads) k_avgsme(const double* __restrict__ e, int n, double sme, double* eta_out) {
+  __shared__ double red[kAvgThreads / 32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   double s = 0.0;
-  for (int i = 1; i < n; ++i) s = s + e[i] - e[i - 1];
-  *eta_out = 10.0 * (s / (double)n) + sme;
+#pragma unroll 4
+  for (int i = 1 + (int)threadIdx.x; i < n; i += kAvgThreads) s += e[i] - e[i - 1];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) red[wid] = s;
+  __syncthreads();
+  if (wid == 0) {
+    s = red[lane];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) *eta_out = 10.0 * (s / (double)n) + sme;
+  }
 }
 
 constexpr int kMaxComp = 8;
@@ -78,31 +93,37 @@ __global__ void __launch_bounds__(256) k_spectrum(const double* __restrict__ E, 
   }
 }
 
-// imagrenorm per component + real(spinf*x) output, eps(nw,2,6)
-__global__ void k_renorm_out(const double* E, const double* om, const double* re, double* im, int nw, int ncomp,
-                             int renorm, double spinf, float* eps) {
-  const int c = threadIdx.x;
-  if (c >= ncomp) return;
-  double* ic = im + (long long)c * nw;
-  if (renorm) {
-    const double aux = E[0] - (double)0.15f;
-    if (!(aux <= 0.000)) {
-      int ibegin = 1;
-      for (int i = 1; i <= nw; ++i) {
-        if (om[i - 1] <= aux) ibegin = i;
-        else break;
-      }
-      const double aux3 = (ibegin < nw) ? ic[ibegin] : 0.0;   // dielf(ibegin+1,3)
-      for (int i = 1; i <= ibegin; ++i) ic[i - 1] = 0.0;
-      for (int i = ibegin + 1; i <= nw; ++i) {
-        const double v = ic[i - 1] - aux3;
-        ic[i - 1] = (v < 0.0) ? 0.0 : v;
-      }
-    }
+// imagrenorm per component + real(spinf*x) output, eps(nw,2,6): one block per component.  ibegin is the
+// number of leading photon energies up to the edge E_1 - 0.15 (at least one), found as the first index
+// above it; the shift is read before any value is written.
+constexpr int kRenormThreads = 512;
+__global__ void __launch_bounds__(kRenormThreads) k_renorm_out(const double* __restrict__ E, const double* __restrict__ om,
+                                                               const double* __restrict__ re, const double* __restrict__ im,
+                                                               int nw, int renorm, double spinf, float* __restrict__ eps) {
+  const int c = blockIdx.x, tid = threadIdx.x;
+  const double* ic = im + (long long)c * nw;
+  const double aux = E[0] - (double)0.15f;
+  const bool on = renorm && !(aux <= 0.000);
+  __shared__ int s_first;
+  if (tid == 0) s_first = nw;
+  __syncthreads();
+  if (on) {
+    int first = nw;
+    for (int i = tid; i < nw && first == nw; i += kRenormThreads)
+      if (!(om[i] <= aux)) first = i;
+    if (first < nw) atomicMin(&s_first, first);
   }
-  for (int i = 0; i < nw; ++i) {
+  __syncthreads();
+  const int ibegin = max(s_first, 1);
+  const double aux3 = (on && ibegin < nw) ? ic[ibegin] : 0.0;   // dielf(ibegin+1,3)
+  for (int i = tid; i < nw; i += kRenormThreads) {
+    double v = ic[i];
+    if (on) {
+      v = v - aux3;
+      v = (i < ibegin || v < 0.0) ? 0.0 : v;
+    }
     eps[(long long)i + (long long)nw * (0 + 2 * c)] = (float)(spinf * re[(long long)c * nw + i]);
-    eps[(long long)i + (long long)nw * (1 + 2 * c)] = (float)(spinf * ic[i]);
+    eps[(long long)i + (long long)nw * (1 + 2 * c)] = (float)(spinf * v);
   }
 }
 
@@ -120,7 +141,7 @@ int launch_spectrum(wtbg_ctx* ctx, int n, int ncomp, const double* d_e, const do
   for (int c = 0; c < ncomp; ++c) rt.rt[c] = rtype[c];
   const double baux = (double)(float)(ngrid[0] * ngrid[1] * ngrid[2]) * vcell3d;
   const double caux = (double)180.90f / (baux * 1.0);
-  k_avgsme<<<1, 32, 0, ctx->stream>>>(d_e, n, sme, eta); WTBG_COUNT(ctx, 1);
+  k_avgsme<<<1, kAvgThreads, 0, ctx->stream>>>(d_e, n, sme, eta); WTBG_COUNT(ctx, 1);
   CKL("k_avgsme");
   const int threads = 256;
   const int blocks = (nw * 32 + threads - 1) / threads;
@@ -137,7 +158,7 @@ int launch_spectrum(wtbg_ctx* ctx, int n, int ncomp, const double* d_e, const do
   }
   WTBG_COUNT(ctx, 1);
   CKL("k_spectrum");
-  k_renorm_out<<<1, 32, 0, ctx->stream>>>(d_e, d_om, re, im, nw, ncomp, renorm, spinf, d_eps); WTBG_COUNT(ctx, 1);
+  k_renorm_out<<<ncomp, kRenormThreads, 0, ctx->stream>>>(d_e, d_om, re, im, nw, renorm, spinf, d_eps); WTBG_COUNT(ctx, 1);
   CKL("k_renorm_out");
   return 0;
 }
@@ -278,7 +299,7 @@ extern "C" int wtbg_spectrum_noalloc(int n, int ncomp, const double* d_ebse, con
   for (int c = 0; c < ncomp; ++c) rt.rt[c] = rtype[c];
   const double baux = (double)(float)(ngrid[0] * ngrid[1] * ngrid[2]) * vcell3d;
   const double caux = (double)180.90f / (baux * 1.0);
-  k_avgsme<<<1, 32, 0, s>>>(d_ebse, n, sme, eta);
+  k_avgsme<<<1, kAvgThreads, 0, s>>>(d_ebse, n, sme, eta);
   const int threads = 256;
   const int blocks = (nw * 32 + threads - 1) / threads;
   switch (ncomp) {
@@ -292,7 +313,7 @@ extern "C" int wtbg_spectrum_noalloc(int n, int ncomp, const double* d_ebse, con
 #undef WTBG_SPEC_CASE
     default: break;
   }
-  k_renorm_out<<<1, 32, 0, s>>>(d_ebse, d_omega, re, im, nw, ncomp, renorm, spinf, d_eps);
+  k_renorm_out<<<ncomp, kRenormThreads, 0, s>>>(d_ebse, d_omega, re, im, nw, renorm, spinf, d_eps);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return noalloc_fail(errbuf, errlen, WTBG_ERR_CUDA, cudaGetErrorString(e));
   return WTBG_OK;
