@@ -72,3 +72,29 @@ def test_several_bands_in_one_launch(n1, n2, nq, gpu_ctx):
             assert np.abs(W[i] - sla.eigvalsh(U + np.triu(U, 1).conj().T)).max() < 1e-11
     finally:
         ctx.set_reduction(0)
+
+
+@pytest.mark.parametrize("n1,n2", [(544, 1), (545, 1), (33, 32), (46, 46), (57, 55), (56, 56), (59, 57)])
+def test_panels_against_one_stage(n1, n2, gpu_ctx):
+    """Panel QR on one cluster: dimensions where the CTA count and the rows per thread change, and
+    (3192, 3363) where the first panels are too long for a cluster. N eps |H| is below 1.5e-11 eV."""
+    ctx, N = gpu_ctx, n1 * n2
+    k, _ = mesh(n1, n2)
+    c = wtbgpu.coulomb_params("V2DRK", [n1, n2, 1], 1e-3, [1, 1, 1], 1.0, 1.0, 0.0, 40.0)
+    ctx.set_model(MODEL)
+    ctx.bands(k, 1, 1, want_vectors=False)
+    h = ctx.velocity(0.05)
+    out = []
+    try:
+        for mode in (1, 2):
+            ctx.set_reduction(mode)
+            ctx.bse_build(c)
+            out.append(ctx.bse_solve(True, True))
+    finally:
+        ctx.set_reduction(0)
+    (W1, a1), (W2, a2) = out
+    assert np.abs(W1 - W2).max() < 3e-11
+    for col, v in ((0, 0), (1, 1), (2, 2), (6, 3), (7, 4)):
+        norm = (np.abs(h[:, v]) ** 2).sum()
+        assert abs(a2[:, col].sum() - norm) <= 1e-12 * N * norm + 1e-14
+        assert abs(a1[:, col].sum() - norm) <= 1e-12 * N * norm + 1e-14

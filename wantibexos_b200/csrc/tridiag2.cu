@@ -125,7 +125,6 @@ struct PanelArgs {
   double2* Tout;       // [32][32] column-major T factor
   double2* g;          // [ng][N]
   int ng;
-  double* partN;       // [grid]
   double2* partW;      // [2][grid][32] partial norms (column p) and unscaled dots, by parity of p
   double2* partG;      // [grid][32*32]
   double2* partVg;     // [grid][32*NGMAX]
@@ -383,6 +382,273 @@ __global__ void __launch_bounds__(PQ_THREADS, 1) k_panel_qr(PanelArgs a) {
     for (int q = 0; q < nref; ++q) s = cadd(s, cmul(cconj(vval(q, i)), s_z[q + al * BW]));
     double2* gp = a.g + (long long)al * N + rbeg + i;
     *gp = csub(*gp, s);
+  }
+}
+
+
+__device__ __forceinline__ double2 shfl2(double2 v, int src) {
+  return make_double2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
+}
+__device__ __forceinline__ double2 shfl2_xor(double2 v, int o) {
+  return make_double2(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o));
+}
+// c + a b, c - a b, c + conj(a) b, c - conj(a) b: four FMAs each
+__device__ __forceinline__ double2 cfma(double2 a, double2 b, double2 c) {
+  return make_double2(fma(-a.y, b.y, fma(a.x, b.x, c.x)), fma(a.y, b.x, fma(a.x, b.y, c.y)));
+}
+__device__ __forceinline__ double2 cfms(double2 a, double2 b, double2 c) {
+  return make_double2(fma(a.y, b.y, fma(-a.x, b.x, c.x)), fma(-a.y, b.x, fma(-a.x, b.y, c.y)));
+}
+__device__ __forceinline__ double2 cfmac(double2 a, double2 b, double2 c) {
+  return make_double2(fma(a.y, b.y, fma(a.x, b.x, c.x)), fma(-a.y, b.x, fma(a.x, b.y, c.y)));
+}
+__device__ __forceinline__ double2 cfmsc(double2 a, double2 b, double2 c) {
+  return make_double2(fma(-a.y, b.y, fma(-a.x, b.x, c.x)), fma(a.y, b.x, fma(-a.x, b.y, c.y)));
+}
+__device__ __forceinline__ double2 caxpy(double a, double2 b, double2 c) {
+  return make_double2(fma(a, b.x, c.x), fma(a, b.y, c.y));
+}
+// Reflector scalars of x (first entry al, xn2 = the squared norm of the others): beta =
+// -sign(Re al) |x|, kappa = -u_0 / (beta |u_0|^2), 1/beta, 1/|u_0|^2; no reflector (kappa = 0, al kept)
+// where x is already (real, 0, ..., 0).  The square root and the reciprocal start from the hardware's
+// first approximation (relative error about 2^-20) and take one third-order step each, which leaves
+// rounding errors only; both arguments are normal numbers (|u_0|^2 >= |x|^2).
+__device__ __forceinline__ void reflector_scalars(double2 al, double xn2, double2& kap, double& beta, double& ib, double& rd) {
+  const double ay2 = al.y * al.y;
+  const double q = fma(al.x, al.x, ay2 + xn2);
+  kap = make_double2(0, 0);
+  beta = al.x;
+  ib = rd = 0.0;
+  if (q >= DBL_MIN && !(xn2 == 0.0 && al.y == 0.0)) {
+    double y, r;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(q));
+    const double t = q * y, e = fma(-t, y, 1.0);         // 1/sqrt(q) = y (1 + e/2 + 3/8 e^2 + O(e^3))
+    const double c = e * fma(e, 0.375, 0.5);
+    const double nr = fma(t, c, t);
+    ib = -copysign(fma(y, c, y), al.x);
+    beta = -copysign(nr, al.x);
+    const double ux = al.x - beta, d = fma(ux, ux, ay2);
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+    const double g = fma(-d, r, 1.0);                    // 1/d = r (1 + g + g^2 + O(g^3))
+    rd = fma(r, fma(g, g, g), r);
+    const double f = -ib * rd;
+    kap = make_double2(f * ux, f * al.y);
+  }
+}
+
+// Panel QR on one cluster of C <= 16 CTAs, for panels of up to 16 x 8 x PC_NR rows.  CTA c owns rows
+// [k0 + cR, k0 + (c+1)R), R = 8 NR, and keeps them in registers: eight threads per column hold its rows
+// i = 8u + sl, and the conjugated velocity vectors are further columns.  Column step p: every column's
+// dot product S_q = sum_{r > k0+p} conj(x_r) P_rq with the pivot column x (in shared memory, zero up to
+// row p), the CTAs' sums exchanged through distributed shared memory, one cluster barrier; then with the
+// unscaled vector u = x - beta e_p the reflector is H = I - kappa u u^H and w_q = u^H P_q = S_q +
+// conj(u_p) P_pq (row p is posted by CTA 0) serves three ends: columns q > p are updated by P_q -=
+// conj(kappa) w_q u, finished columns q < p give the Gram entry v_q^H v_p = conj(w_q) / u_p that the T factor
+// needs, and the velocity columns give V^T g the same way.  T = T_1 + T_2 blocks by doubling.
+// Bound by the latency of the column chain.  The grid-wide form (k_panel_qr, still used for longer
+// panels) pays a barrier and two round trips through L2 per column, keeps the slice in shared memory
+// (whose bandwidth bounds update and dot products) and forms Gram matrix and V^T g in passes of their
+// own.  Per panel, grid-wide against cluster: N = 576 170 / 68 us, 2304 189 / 91 us.
+constexpr int PC_THREADS = 384;   // 48 columns x 8 threads: 32 of the panel, up to 10 velocity vectors
+constexpr int PC_COLS = BW + NGMAX;
+constexpr int PC_MAXC = 16;
+constexpr int PC_MAX_NR = 24;
+constexpr size_t pc_smem(int nr) {
+  return sizeof(double2) * (size_t)(2 * PC_MAXC * PC_COLS + 2 * BW * BW + BW * BW / 4 + 2 * BW * NGMAX + BW * (8 * nr + 1));
+}
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// one 16-byte store into the same shared-memory place of CTA `cta` of the cluster
+__device__ __forceinline__ void st_cluster(double2* p, uint32_t cta, double2 v) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(tc::smem_u32(p)), "r"(cta));
+  asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(a), "d"(v.x), "d"(v.y) : "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <int NR>
+__global__ void __launch_bounds__(PC_THREADS, 1) k_panel_qr_cl(PanelArgs a, int C) {
+  constexpr int R = 8 * NR, VS = R + 1;
+  extern __shared__ __align__(16) double2 psm[];
+  double2(*s_part)[PC_MAXC][PC_COLS] = reinterpret_cast<double2(*)[PC_MAXC][PC_COLS]>(psm);   // dot products, by parity of p
+  double2* s_G = psm + 2 * PC_MAXC * PC_COLS;
+  double2* s_T = s_G + BW * BW;
+  double2* s_w = s_T + BW * BW;
+  double2* s_y = s_w + BW * BW / 4;
+  double2* s_z = s_y + BW * NGMAX;
+  double2* Vs = s_z + BW * NGMAX;                      // [32][VS]: V of the own rows, at the end
+  __shared__ double2 s_x[2][R];                        // pivot column by parity of p
+  __shared__ double2 s_al[2][PC_COLS];                 // row p
+  __shared__ double2 s_tau[BW];
+  __shared__ double2 s_sc[2][3];                       // kappa; (beta, 0); 1/u_p
+  const int tid = threadIdx.x, lane = tid & 31, sl = tid & 7, q = tid >> 3;
+  const int c = (int)cluster_rank();
+  const long long N = a.N;
+  const long long rbeg = (long long)a.k0 + (long long)c * R;
+  const int nr = (int)max(0LL, min((long long)R, N - rbeg));
+  const int nref = a.nref, ng = a.ng;
+  const bool panel = q < BW, vel = q >= BW && q < BW + ng;
+  double2 P[NR];
+#pragma unroll
+  for (int u = 0; u < NR; ++u) {
+    const int i = 8 * u + sl;
+    P[u] = make_double2(0, 0);
+    if (i < nr) {
+      if (panel) P[u] = a.A[(rbeg + i) + (long long)(a.j0 + q) * N];
+      else if (vel) P[u] = cconj(__ldcg(a.g + (long long)(q - BW) * N + rbeg + i));
+    }
+  }
+  // the pivot column p into s_x (zero up to row p, which only CTA 0 holds), by its eight threads
+  auto post = [&](int p) {
+#pragma unroll
+    for (int u = 0; u < NR; ++u) s_x[p & 1][8 * u + sl] = (c == 0 && 8 * u + sl <= p) ? make_double2(0, 0) : P[u];
+  };
+  auto sum8 = [](double2 v) {
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v = cadd(v, shfl2_xor(v, o));
+    return v;
+  };
+  for (int e = tid; e < BW * BW; e += PC_THREADS) s_G[e] = s_T[e] = make_double2(0, 0);
+  for (int e = tid; e < BW * NGMAX; e += PC_THREADS) s_y[e] = make_double2(0, 0);
+  if (tid < BW) s_tau[tid] = make_double2(0, 0);
+  if (q == 0) post(0);
+  cluster_sync();   // every CTA of the cluster runs (its shared memory is written below)
+  for (int p = 0; p < nref; ++p) {
+    const int buf = p & 1;
+    double2* xs = s_x[buf];
+    {
+      double2 s0 = make_double2(0, 0), s1 = s0;
+#pragma unroll
+      for (int u = 0; u < NR; u += 2) {
+        s0 = cfmac(xs[8 * u + sl], P[u], s0);
+        if (u + 1 < NR) s1 = cfmac(xs[8 * u + 8 + sl], P[u + 1], s1);
+      }
+      const double2 S = sum8(cadd(s0, s1));
+      if (q < PC_COLS) {
+        if (sl < C) st_cluster(&s_part[buf][c][q], sl, S);
+        if (sl + 8 < C) st_cluster(&s_part[buf][c][q], sl + 8, S);
+      }
+      if (c == 0) {   // row p of every column, held by the thread sl = p mod 8 at u = p / 8 (rows < 32: u < 4)
+        const double2 v = (p >> 3) == 0 ? P[0] : ((p >> 3) == 1 ? P[1] : ((p >> 3) == 2 ? P[2] : P[3]));
+        const double2 r = shfl2(v, (lane & 24) | (p & 7));
+        if (q < PC_COLS) {
+          if (sl < C) st_cluster(&s_al[buf][q], sl, r);
+          if (sl + 8 < C) st_cluster(&s_al[buf][q], sl + 8, r);
+        }
+      }
+    }
+    cluster_sync();
+    double2 S = make_double2(0, 0);
+    if (q < PC_COLS) {
+      if (sl < C) S = s_part[buf][sl][q];
+      if (sl + 8 < C) S = cadd(S, s_part[buf][sl + 8][q]);
+    }
+    S = sum8(S);
+    if ((tid >> 5) == (p >> 2)) {   // the warp that holds column p forms the scalars
+      const double xn2 = __shfl_sync(0xffffffffu, S.x, 8 * (p & 3));
+      const double2 al = s_al[buf][p];
+      double2 kap;
+      double beta, ib, rd;
+      reflector_scalars(al, xn2, kap, beta, ib, rd);
+      if (lane == 0) {
+        const double2 u0 = make_double2(al.x - beta, al.y);
+        s_sc[buf][0] = kap;
+        s_sc[buf][1] = make_double2(beta, 0.0);
+        s_sc[buf][2] = cscale(cconj(u0), rd);
+        s_tau[p] = cscale(u0, -ib);
+        if (c == 0) xs[p] = u0;
+      }
+    }
+    __syncthreads();
+    const double2 kap = s_sc[buf][0], scal = s_sc[buf][2];
+    const double beta = s_sc[buf][1].x;
+    // w_q = S_q + conj(u_p) P_pq
+    const double2 al = s_al[buf][p];
+    const double2 w = q < PC_COLS ? cfmac(make_double2(al.x - beta, al.y), s_al[buf][q], S) : S;
+    if (panel && q > p) {
+      const double2 cw = cmulc(kap, w);
+#pragma unroll
+      for (int u = 0; u < NR; ++u) P[u] = cfms(xs[8 * u + sl], cw, P[u]);
+      if (q == p + 1 && q < nref) post(q);
+    } else if (q == p) {
+#pragma unroll
+      for (int u = 0; u < NR; ++u) {
+        const int i = 8 * u + sl;
+        if (c > 0 || i > p) P[u] = cmul(P[u], scal);
+        else if (i == p) P[u] = make_double2(beta, 0.0);
+      }
+    } else if (sl == 0) {
+      const double2 e = cmul(scal, cconj(w));
+      if (panel) s_G[q + p * BW] = e;                 // v_q^H v_p, q < p
+      else if (vel) s_y[p + (q - BW) * BW] = e;       // (V^T g)_p
+    }
+    __syncthreads();
+  }
+  // write back: A keeps R (rows <= k0+q) and v below; Vp and Vs get V with its unit and zeros
+  if (panel) {
+#pragma unroll
+    for (int u = 0; u < NR; ++u) {
+      const int i = 8 * u + sl;
+      double2 v = P[u];
+      if (q >= nref || (c == 0 && i < q)) v = make_double2(0, 0);
+      else if (c == 0 && i == q) v = make_double2(1.0, 0.0);
+      Vs[q * VS + i] = v;
+      if (i < nr) {
+        a.A[(rbeg + i) + (long long)(a.j0 + q) * N] = P[u];
+        a.Vp[(rbeg + i) + (long long)q * N] = v;
+      }
+    }
+  }
+  // T factor: T_ii = tau_i, and for neighbouring diagonal blocks of size h, T_12 = -T_11 (G_12 T_22)
+  if (tid < BW) s_T[tid + tid * BW] = s_tau[tid];
+  __syncthreads();
+  for (int h = 1; h < BW; h *= 2) {
+    const int cnt = BW / (2 * h) * h * h;   // entries of all pairs' T_12
+    int b = 0, i = 0, j = 0;
+    if (tid < cnt) {
+      b = tid / (h * h) * 2 * h;
+      i = tid % h;
+      j = (tid / h) % h;
+      double2 t = make_double2(0, 0);
+      for (int l = 0; l <= j; ++l) t = cfma(s_G[(b + i) + (b + h + l) * BW], s_T[(b + h + l) + (b + h + j) * BW], t);
+      s_w[tid] = t;
+    }
+    __syncthreads();
+    if (tid < cnt) {
+      double2 t = make_double2(0, 0);
+      const double2* wj = s_w + tid - i;   // column j of the pair's product
+      for (int l = i; l < h; ++l) t = cfms(s_T[(b + i) + (b + l) * BW], wj[l], t);
+      s_T[(b + i) + (b + h + j) * BW] = t;
+    }
+    __syncthreads();
+  }
+  if (c == 0)
+    for (int e = tid; e < BW * BW; e += PC_THREADS) a.Tout[e] = s_T[e];
+  // g <- g - conj(V) T^T (V^T g)
+  if (ng == 0) return;
+  for (int e = tid; e < BW * ng; e += PC_THREADS) {
+    const int j = e % BW, al = e / BW;
+    double2 t = make_double2(0, 0);
+    for (int i = 0; i <= j; ++i) t = cfma(s_T[i + j * BW], s_y[i + al * BW], t);
+    s_z[e] = t;
+  }
+  __syncthreads();
+  for (int e = tid; e < nr * ng; e += PC_THREADS) {
+    const int i = e % nr, al = e / nr;
+    double2 t0 = make_double2(0, 0), t1 = t0;
+#pragma unroll 4
+    for (int k = 0; k < BW; k += 2) {
+      t0 = cfmac(Vs[k * VS + i], s_z[k + al * BW], t0);
+      t1 = cfmac(Vs[(k + 1) * VS + i], s_z[k + 1 + al * BW], t1);
+    }
+    double2* gp = a.g + (long long)al * N + rbeg + i;
+    *gp = csub(*gp, cadd(t0, t1));
   }
 }
 
@@ -1109,55 +1375,6 @@ __device__ __forceinline__ void bar_arrive(int id, int cnt) {
   __syncwarp();
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(cnt) : "memory");
 }
-__device__ __forceinline__ double2 shfl2(double2 v, int src) {
-  return make_double2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
-}
-__device__ __forceinline__ double2 shfl2_xor(double2 v, int o) {
-  return make_double2(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o));
-}
-// c + a b, c - a b, c + conj(a) b, c - conj(a) b: four FMAs each
-__device__ __forceinline__ double2 cfma(double2 a, double2 b, double2 c) {
-  return make_double2(fma(-a.y, b.y, fma(a.x, b.x, c.x)), fma(a.y, b.x, fma(a.x, b.y, c.y)));
-}
-__device__ __forceinline__ double2 cfms(double2 a, double2 b, double2 c) {
-  return make_double2(fma(a.y, b.y, fma(-a.x, b.x, c.x)), fma(-a.y, b.x, fma(-a.x, b.y, c.y)));
-}
-__device__ __forceinline__ double2 cfmac(double2 a, double2 b, double2 c) {
-  return make_double2(fma(a.y, b.y, fma(a.x, b.x, c.x)), fma(-a.y, b.x, fma(a.x, b.y, c.y)));
-}
-__device__ __forceinline__ double2 cfmsc(double2 a, double2 b, double2 c) {
-  return make_double2(fma(-a.y, b.y, fma(-a.x, b.x, c.x)), fma(a.y, b.x, fma(-a.x, b.y, c.y)));
-}
-__device__ __forceinline__ double2 caxpy(double a, double2 b, double2 c) {
-  return make_double2(fma(a, b.x, c.x), fma(a, b.y, c.y));
-}
-// Reflector scalars of x (first entry al, xn2 = the squared norm of the others): beta =
-// -sign(Re al) |x|, kappa = -u_0 / (beta |u_0|^2), 1/beta, 1/|u_0|^2; no reflector (kappa = 0, al kept)
-// where x is already (real, 0, ..., 0).  The square root and the reciprocal start from the hardware's
-// first approximation (relative error about 2^-20) and take one third-order step each, which leaves
-// rounding errors only; both arguments are normal numbers (|u_0|^2 >= |x|^2).
-__device__ __forceinline__ void chase_scalars(double2 al, double xn2, double2& kap, double& beta, double& ib, double& rd) {
-  const double ay2 = al.y * al.y;
-  const double q = fma(al.x, al.x, ay2 + xn2);
-  kap = make_double2(0, 0);
-  beta = al.x;
-  ib = rd = 0.0;
-  if (q >= DBL_MIN && !(xn2 == 0.0 && al.y == 0.0)) {
-    double y, r;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(q));
-    const double t = q * y, e = fma(-t, y, 1.0);         // 1/sqrt(q) = y (1 + e/2 + 3/8 e^2 + O(e^3))
-    const double c = e * fma(e, 0.375, 0.5);
-    const double nr = fma(t, c, t);
-    ib = -copysign(fma(y, c, y), al.x);
-    beta = -copysign(nr, al.x);
-    const double ux = al.x - beta, d = fma(ux, ux, ay2);
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-    const double g = fma(-d, r, 1.0);                    // 1/d = r (1 + g + g^2 + O(g^3))
-    rd = fma(r, fma(g, g, g), r);
-    const double f = -ib * rd;
-    kap = make_double2(f * ux, f * al.y);
-  }
-}
 // bounded wait for a phase of an mbarrier; the clock is read every 64 polls (a read takes longer than
 // most waits)
 __device__ __forceinline__ bool mbar_wait_bounded(uint32_t a, uint32_t parity) {
@@ -1399,7 +1616,7 @@ __global__ void __launch_bounds__(CH_THREADS, 1) k_chase(BulgeArgs a) {
           double beta, ib, rd;
           const double2* xs = s_x[xb];
           const double* pn = s_np[xb];
-          chase_scalars(xs[0], (pn[0] + pn[1]) + (pn[2] + pn[3]), kap, beta, ib, rd);
+          reflector_scalars(xs[0], (pn[0] + pn[1]) + (pn[2] + pn[3]), kap, beta, ib, rd);
           dot_rows(xs, z);
           // x is read again below rather than kept: registers
           asm volatile("" ::: "memory");
@@ -1704,6 +1921,78 @@ static int two_stage_buffers(wtbg_ctx* ctx, int nband) {
   return 0;
 }
 
+// Panel QR on one cluster.  C CTAs of R = 8 NR rows with R >= 32 (CTA 0 holds the first 32 rows), as many
+// CTAs as that allows: the column step gets shorter with fewer rows per thread.
+using PanelClFn = void (*)(PanelArgs, int);
+static PanelClFn panel_cl_fn(int nr) {
+  switch (nr) {
+    case 4: return k_panel_qr_cl<4>;
+    case 6: return k_panel_qr_cl<6>;
+    case 8: return k_panel_qr_cl<8>;
+    case 10: return k_panel_qr_cl<10>;
+    case 12: return k_panel_qr_cl<12>;
+    case 14: return k_panel_qr_cl<14>;
+    case 16: return k_panel_qr_cl<16>;
+    case 18: return k_panel_qr_cl<18>;
+    case 20: return k_panel_qr_cl<20>;
+    case 22: return k_panel_qr_cl<22>;
+    default: return k_panel_qr_cl<24>;
+  }
+}
+static int launch_panel_cluster(wtbg_ctx* ctx, const PanelArgs& pa) {
+  const long long m = pa.N - pa.k0;
+  int C = 1;
+  while (C < ctx->panel_cl_max && (long long)C * 32 < m) C *= 2;
+  int nr = (int)((m + 8 * C - 1) / (8 * C));
+  nr = std::max(4, (nr + 1) & ~1);
+  PanelClFn fn = panel_cl_fn(nr);
+  const size_t smem = pc_smem(nr);
+  CK(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (C > 8) CK(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(C);
+  cfg.blockDim = dim3(PC_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = C;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  CK(cudaLaunchKernelEx(&cfg, fn, pa, C));
+  return 0;
+}
+// Largest cluster the device takes for the panel kernel (16 where a GPC has room for it, else 8) and the
+// panel rows that gives.
+static int panel_cluster_limits(wtbg_ctx* ctx) {
+  if (ctx->panel_cl_max > 0) return 0;
+  PanelClFn fn = panel_cl_fn(PC_MAX_NR);
+  const size_t smem = pc_smem(PC_MAX_NR);
+  CK(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CK(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(PC_MAXC);
+  cfg.blockDim = dim3(PC_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = PC_MAXC;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  int ncl = 0;
+  if (cudaOccupancyMaxActiveClusters(&ncl, (const void*)fn, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    ncl = 0;
+  }
+  ctx->panel_cl_max = ncl > 0 ? PC_MAXC : 8;
+  ctx->panel_cl_rows = (long long)ctx->panel_cl_max * 8 * PC_MAX_NR;
+  return 0;
+}
+
 // Stage 1 (dense -> band) of the context's matrix; the band goes to slot `band` of ctx->t2AB.
 // ng velocity vectors in ctx->g follow the reflectors.
 static int run_stage1(wtbg_ctx* ctx, int ng, int band) {
@@ -1725,13 +2014,13 @@ static int run_stage1(wtbg_ctx* ctx, int ng, int band) {
   double2* Cbuf = Cpart + (size_t)nI * 2 * (LOOKAHEAD - 1) * 1024;     // C1 (K x 32) then C2
   double2* Tbuf = ctx->t2T.as<double2>();
   char* pb = ctx->t2P.as<char>();
-  double* partN = reinterpret_cast<double*>(pb);
   double2* partW = reinterpret_cast<double2*>(pb + (size_t)nsm * 16);   // 16-byte aligned for any SM count
   double2* partG = partW + (size_t)2 * nsm * BW;
   double2* partVg = partG + (size_t)nsm * BW * BW;
   double2* alpha = partVg + (size_t)nsm * BW * NGMAX;
   unsigned int* cnt = reinterpret_cast<unsigned int*>(alpha + 2 * BW);   // one barrier counter per panel launch
   int* err = ctx->triErr.as<int>();
+  if (int r = panel_cluster_limits(ctx)) return r;
   CK(cudaMemsetAsync(cnt, 0, (size_t)std::max<long long>(npan, 1) * 4, s));
   CK(cudaFuncSetAttribute(k_hemm2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HM_SMEM));
   CK(cudaFuncSetAttribute(k_xreduce, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XR_SMEM));
@@ -1755,35 +2044,36 @@ static int run_stage1(wtbg_ctx* ctx, int ng, int band) {
     const int j0 = (int)(pnl * BW), k0 = j0 + BW;
     const long long m = N - k0;
     const int nref = (int)std::min<long long>(BW, m);
-    // panel QR: G CTAs of R rows (at most 64 CTAs while the rows fit: the panel is latency-bound,
-    // and fewer CTAs make the grid barrier and the cross-CTA reductions cheaper)
-    const int R = (int)std::min<long long>(PQ_MAX_R, std::max<long long>(64, (m + 63) / 64));
-    const int G = (int)((m + R - 1) / R);
-    PanelArgs pa;
+    PanelArgs pa{};
     pa.A = A;
     pa.N = N;
     pa.j0 = j0;
     pa.k0 = k0;
     pa.jb = BW;
     pa.nref = nref;
-    pa.R = R;
-    pa.RS = R | 1;
     pa.Vp = V;
     pa.Tout = Tbuf + (size_t)pnl * 1024;
     pa.g = g;
     pa.ng = ng;
-    pa.partN = partN;
-    pa.partW = partW;
-    pa.partG = partG;
-    pa.partVg = partVg;
-    pa.alpha = alpha;
-    pa.cnt = cnt + pnl;
-    pa.err = err;
-    const size_t psm = (size_t)BW * (R | 1) * 16;
-    CK(cudaFuncSetAttribute(k_panel_qr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm));
-    if (G > PQ_MAXG) return set_err(ctx, WTBG_ERR_UNSUPPORTED, "panel QR: more CTAs than the column reduction holds");
     mark(pnl, 0);
-    {
+    if (m <= ctx->panel_cl_rows) {
+      if (int r = launch_panel_cluster(ctx, pa)) return r;
+    } else {
+      // grid-wide: G CTAs of R rows (at most 64 CTAs while the rows fit: the panel is latency-bound,
+      // and fewer CTAs make the grid barrier and the cross-CTA reductions cheaper)
+      const int R = (int)std::min<long long>(PQ_MAX_R, std::max<long long>(64, (m + 63) / 64));
+      const int G = (int)((m + R - 1) / R);
+      pa.R = R;
+      pa.RS = R | 1;
+      pa.partW = partW;
+      pa.partG = partG;
+      pa.partVg = partVg;
+      pa.alpha = alpha;
+      pa.cnt = cnt + pnl;
+      pa.err = err;
+      const size_t psm = (size_t)BW * (R | 1) * 16;
+      CK(cudaFuncSetAttribute(k_panel_qr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm));
+      if (G > PQ_MAXG) return set_err(ctx, WTBG_ERR_UNSUPPORTED, "panel QR: more CTAs than the column reduction holds");
       void* args[] = {&pa};
       CK(cudaLaunchCooperativeKernel((const void*)k_panel_qr, dim3(G), dim3(PQ_THREADS), args, psm, s));
     }
