@@ -259,11 +259,6 @@ int wtbg_bands(wtbg_ctx* ctx, int nk, const double* kpt, int nv, int nc, double*
   CK(cudaMemcpyAsync(e.data(), ctx->eig.p, e.size() * 8, cudaMemcpyDeviceToHost, ctx->stream));
   std::vector<int> no(nk);
   CK(cudaMemcpyAsync(no.data(), ctx->nocp.p, (size_t)nk * 4, cudaMemcpyDeviceToHost, ctx->stream));
-  std::vector<double2> u;
-  if (vector) {
-    u.resize((size_t)nk * nb * w);
-    CK(cudaMemcpyAsync(u.data(), ctx->U.p, u.size() * 16, cudaMemcpyDeviceToHost, ctx->stream));
-  }
   CK(cudaStreamSynchronize(ctx->stream));
   double gap = 50.0;
   for (int k = 0; k < nk; ++k) {
@@ -277,14 +272,7 @@ int wtbg_bands(wtbg_ctx* ctx, int nk, const double* kpt, int nv, int nc, double*
   if (nocpk)
     for (int k = 0; k < nk; ++k) nocpk[k] = no[k];
   if (vector)
-    for (int k = 0; k < nk; ++k)
-      for (int j = 0; j < nb; ++j)
-        for (int m = 0; m < w; ++m) {
-          const double2 v = u[((size_t)k * nb + j) * w + m];
-          const size_t dst = (size_t)k + (size_t)nk * ((size_t)j + (size_t)nb * m);   // vector(k, j, m)
-          vector[2 * dst] = v.x;
-          vector[2 * dst + 1] = v.y;
-        }
+    if (int r = copy_vectors_out(ctx, ctx->U.as<double2>(), nk, nb, w, vector)) return r;   // vector(k, j, m)
   return WTBG_OK;
 }
 
@@ -542,28 +530,20 @@ int wtbg_eigsys(wtbg_ctx* ctx, int nk, const double* kpt, double* eig, double* v
   CK(cudaMemsetAsync(ds, 0, b_int, ctx->stream));
   if (int r = launch_eigsys_all(ctx, nk, dk, de, ctx->ws.as<double2>(), dn, ds)) return r;
   if (int r = t.stop()) return r;
-  std::vector<int> st(nk);
-  CK(cudaMemcpy(st.data(), ds, b_int, cudaMemcpyDeviceToHost));
+  // eigenvalues, nocp and status lie behind one another: one copy
+  const size_t o_eig = (b_kpt + 255) / 256 * 256, o_int = (b_eig + 255) / 256 * 256;
+  std::vector<double> buf((o_int + 2 * b_int + 7) / 8);
+  CK(cudaMemcpy(buf.data(), base + o_eig, o_int + 2 * b_int, cudaMemcpyDeviceToHost));
+  const double* e = buf.data();
+  const int* no = reinterpret_cast<const int*>(reinterpret_cast<const char*>(buf.data()) + o_int);
   for (int k = 0; k < nk; ++k)
-    if (st[k] == 1) return set_err(ctx, WTBG_ERR_NOCONV, "eigsys: Jacobi did not converge at k-point " + std::to_string(k + 1));
-  std::vector<double> e((size_t)nk * w);
-  CK(cudaMemcpy(e.data(), de, b_eig, cudaMemcpyDeviceToHost));
-  for (int k = 0; k < nk; ++k)
-    for (int b = 0; b < w; ++b) eig[k + (size_t)nk * b] = e[(size_t)k * w + b];
-  if (nocp) CK(cudaMemcpy(nocp, dn, b_int, cudaMemcpyDeviceToHost));
-  if (vec) {
-    std::vector<double2> u((size_t)nk * w * w);
-    CK(cudaMemcpy(u.data(), ctx->ws.p, u.size() * 16, cudaMemcpyDeviceToHost));
-    // vec(k, n, m): k fastest, then band n, then component m (the reference's autovetores per k)
-    for (int k = 0; k < nk; ++k)
-      for (int n = 0; n < w; ++n)
-        for (int m = 0; m < w; ++m) {
-          const double2 v = u[((size_t)k * w + n) * w + m];
-          const size_t o = k + (size_t)nk * (n + (size_t)w * m);
-          vec[2 * o] = v.x;
-          vec[2 * o + 1] = v.y;
-        }
-  }
+    if (no[nk + k] == 1) return set_err(ctx, WTBG_ERR_NOCONV, "eigsys: Jacobi did not converge at k-point " + std::to_string(k + 1));
+  for (int b = 0; b < w; ++b)
+    for (int k = 0; k < nk; ++k) eig[k + (size_t)nk * b] = e[(size_t)k * w + b];
+  if (nocp) memcpy(nocp, no, b_int);
+  // vec(k, n, m): k fastest, then band n, then component m (the reference's autovetores per k)
+  if (vec)
+    if (int r = copy_vectors_out(ctx, ctx->ws.as<double2>(), nk, w, w, vec)) return r;
   return WTBG_OK;
 }
 

@@ -748,6 +748,43 @@ static int bands_threads(wtbg_ctx* ctx, int w, long long nk) {
   return std::min(full, w <= 8 ? 32 : (w <= 16 ? 64 : (w <= 32 ? 128 : kBandsThreads)));
 }
 
+// vec(k, j, m) = U[k][j][m]: transposed through 32 x 32 tiles so that reads and writes are contiguous;
+// the component range [m0, m0 + mc) goes to out[k + nk (j + nb (m - m0))]
+__global__ void __launch_bounds__(256) k_vectors_out(const double2* __restrict__ U, int nk, int nb, int w, int m0, int mc,
+                                                     double2* __restrict__ out) {
+  __shared__ double2 tile[32][33];
+  const int kb = blockIdx.x * 32, cb = blockIdx.y * 32;   // column = j * mc + (m - m0): m runs fastest in U
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int ncol = nb * mc;
+  for (int y = ty; y < 32; y += 8) {
+    const int k = kb + y, c = cb + tx;
+    if (k < nk && c < ncol) tile[y][tx] = U[((size_t)k * nb + c / mc) * w + m0 + c % mc];
+  }
+  __syncthreads();
+  for (int y = ty; y < 32; y += 8) {
+    const int k = kb + tx, c = cb + y;
+    if (k < nk && c < ncol) out[(size_t)k + (size_t)nk * ((size_t)(c / mc) + (size_t)nb * (c % mc))] = tile[tx][y];
+  }
+}
+
+// The layout change on the device and one copy per piece of at most 128 MB (pieces are ranges of the
+// slowest output index m).  On the host it was a strided walk over the whole array: with the copy it
+// took 23 ms of 32 for 1296 k-points of 40 bands.
+int copy_vectors_out(wtbg_ctx* ctx, const double2* d_U, int nk, int nb, int w, double* vec) {
+  const size_t per = (size_t)nk * nb * 16;
+  const int mc = (int)std::max<size_t>(1, std::min<size_t>((size_t)w, (size_t)(128u << 20) / per));
+  ENSURE(ctx->tmp2, per * mc);
+  for (int m0 = 0; m0 < w; m0 += mc) {
+    const int c = std::min(mc, w - m0);
+    const dim3 grid((nk + 31) / 32, (unsigned)(((long long)nb * c + 31) / 32));
+    k_vectors_out<<<grid, 256, 0, ctx->stream>>>(d_U, nk, nb, w, m0, c, ctx->tmp2.as<double2>()); WTBG_COUNT(ctx, 1);
+    CKL("k_vectors_out");
+    CK(cudaMemcpyAsync(vec + 2 * (size_t)nk * nb * m0, ctx->tmp2.p, per * c, cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+  }
+  return 0;
+}
+
 // H(k) of every k of the mesh by the 3-term split-BF16 tensor-core GEMM (FP32 result
 // [2 w^2][nk] in ctx->pHk)
 static int run_precision_hk(wtbg_ctx* ctx, const double* kpt, int nk) {
