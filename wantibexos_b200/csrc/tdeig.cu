@@ -9,13 +9,14 @@
 //   * eigenvalues: one coarse round of Sturm counts at 32769 points of the Gershgorin interval
 //     gives every eigenvalue index its starting cell; then Sturm-count multisection, L lanes
 //     per eigenvalue index (L = 1: bisection), to full precision;
-//   * eigenvectors: inverse iteration with a partial-pivoting tridiagonal LU, three steps
-//     from a deterministic pseudo-random start vector; eigenvalues closer than
-//     1e-7 * ||T|| form a cluster that one thread processes in sequence with modified
-//     Gram-Schmidt against the earlier members (so degenerate excitons get orthogonal
-//     vectors); the vectors live in a chunked workspace laid out [k][slot] so that the
-//     threads' accesses coalesce;
-//   * the dot products with g are fused into the last pass over each vector.
+//   * eigenvectors: the recurrence of T - lambda from the top and from the bottom, joined at the
+//     row where the product of the two is largest (k_twist), the dot products with g taken in the
+//     last pass over the vector; one row's residual shows whether the vector is good;
+//   * eigenvalues closer than 1e-7 * ||T|| form a cluster: its vectors are orthonormalised in
+//     order (k_cluster), so degenerate excitons get orthogonal vectors;
+//   * what neither makes well (a residual that is too large, a cluster of nearly parallel
+//     vectors) and the vectors of BSE_WF are made by inverse iteration with a partial-pivoting
+//     tridiagonal LU, three steps from a deterministic pseudo-random start vector (k_inviter).
 // Selected exciton eigenvectors (BSE_WF) are back-transformed A_n = Q z_n panel by panel
 // with the compact-WY form I - V T V^H of each panel's reflectors.
 #include <algorithm>
@@ -29,23 +30,106 @@ namespace {
 
 constexpr int NG = 10;   // largest number of reduced h vectors (5, or 10 with temperature)
 
-__device__ __forceinline__ int sturm_count(const double* __restrict__ d, const double* __restrict__ e2, long long n,
-                                           double x, double pivmin) {
-  int cnt = 0;
-  double q = d[0] - x;
-  if (fabs(q) < pivmin) q = -pivmin;
-  cnt += (q < 0.0);
-  for (long long i = 1; i < n; ++i) {
-    q = (d[i] - x) - e2[i - 1] / q;
-    if (fabs(q) < pivmin) q = -pivmin;
-    cnt += (q < 0.0);
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N_>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N_) : "memory"); }
+
+// Records of T scaled by sc = 2^-j so that ||sc T|| <= 1, padded to a multiple of TD_TILE rows by rows that
+// change no count: cnt[k] = (d_k, -e_{k-1}^2) for the counts, vec[2k], vec[2k+1] = (d_k, e_k), (-1/e_k, -1/e_{k-1}) for
+// the vectors.  |e| is held above TD_EMIN, far below the rounding of T itself, so that the recurrences never
+// run into zero: eight steps shrink them by less than 2^-1000.
+constexpr int TD_TILE = 128;
+constexpr double TD_EMIN = 0x1p-80;
+__global__ void k_td_records(const double* __restrict__ d, const double* __restrict__ e, int n, int npad, double sc,
+                             double2* __restrict__ cnt, double2* __restrict__ vec) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= npad) return;
+  auto off = [&](int i) {
+    const double x = e[i] * sc;
+    return fabs(x) < TD_EMIN ? copysign(TD_EMIN, x) : x;
+  };
+  const double ep = (k >= 1 && k < n) ? off(k - 1) : 0.0, ek = (k < n - 1) ? off(k) : 1.0;
+  const double dk = (k < n) ? d[k] * sc : 4.0;
+  cnt[k] = make_double2(dk, -ep * ep);
+  vec[2 * k] = make_double2(dk, ek);
+  vec[2 * k + 1] = make_double2(-1.0 / ek, (k >= 1 && k < n) ? -1.0 / ep : 0.0);
+}
+
+// a, b scaled by the power of two that brings the larger to [1, 2); returns the exponent taken out
+__device__ __forceinline__ int rescale(double& a, double& b) {
+  const int h = max(__double2hiint(a) & 0x7ff00000, __double2hiint(b) & 0x7ff00000);
+  const double f = __hiloint2double(0x7fe00000 - h, 0);
+  a *= f;
+  b *= f;
+  return (h >> 20) - 1023;
+}
+
+// Number of eigenvalues of the scaled T below x, one point per thread: the sign changes of the leading
+// minors p_{k+1} = (d_k - x) p_k - e_{k-1}^2 p_{k-1} (the counts of the pivots p_{k+1} / p_k, and as backward
+// stable: each step is exact for d_k - x and e_{k-1}^2 changed by a few roundings).  Without a division the chain
+// is one FMA a step (N = 576 0.41 -> 0.07 ms, 3600 3.6 -> 0.71 ms); scaled every eight steps.  The records stream through a four-stage ring shared by the
+// block of TD_TILE threads, all of which must call this.
+constexpr int TD_ST = 4;
+__device__ __forceinline__ int block_sturm(const double2* __restrict__ rec, int ntile, double x,
+                                           double2 (*ring)[TD_TILE]) {
+  const int tid = threadIdx.x;
+  for (int t = 0; t < TD_ST - 1; ++t) {
+    if (t < ntile) cp_async16(&ring[t][tid], rec + (size_t)t * TD_TILE + tid);
+    cp_async_commit();
   }
+  double p = 1.0, pp = 0.0;
+  int cnt = 0;
+  for (int t = 0; t < ntile; ++t) {
+    cp_async_wait<TD_ST - 2>();
+    __syncthreads();
+    const int tn = t + TD_ST - 1;
+    if (tn < ntile) cp_async16(&ring[tn % TD_ST][tid], rec + (size_t)tn * TD_TILE + tid);
+    cp_async_commit();
+    const double2* c = ring[t % TD_ST];
+    double2 a[8], b[8];   // eight records at work, the next eight on their way
+    auto load = [&](double2* v, int g) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v[q] = c[g + q];
+    };
+    auto steps = [&](const double2* v) {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const double pn = fma(v[q].x - x, p, v[q].y * pp);
+        cnt += (unsigned)(__double2hiint(pn) ^ __double2hiint(p)) >> 31;
+        pp = p;
+        p = pn;
+      }
+      rescale(p, pp);
+    };
+    load(a, 0);
+#pragma unroll 1
+    for (int g = 0; g < TD_TILE; g += 16) {
+      load(b, g + 8);
+      steps(a);
+      load(a, (g + 16) & (TD_TILE - 1));
+      steps(b);
+    }
+  }
+  __syncthreads();
   return cnt;
 }
 
-__global__ void k_e2(const double* e, long long n, double* e2) {
-  long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i < n - 1) e2[i] = e[i] * e[i];
+// Coarse round: Sturm counts at the P + 1 points x_j = lo + (hi - lo) j / P of the Gershgorin
+// interval (count 0 at lo and n at hi by construction), one thread per point.
+constexpr int BIS_P = 32768;
+__global__ void __launch_bounds__(TD_TILE) k_bisect_grid(const double2* __restrict__ rec, int ntile, int n, double lo,
+                                                         double hi, double sc, double* __restrict__ xg,
+                                                         int* __restrict__ cg) {
+  __shared__ __align__(16) double2 ring[TD_ST][TD_TILE];
+  const int j = min(blockIdx.x * TD_TILE + (int)threadIdx.x, BIS_P);
+  const double x = (j == BIS_P) ? hi : lo + (hi - lo) * ((double)j / (double)BIS_P);
+  const int c = block_sturm(rec, ntile, x * sc, ring);
+  xg[j] = x;
+  cg[j] = (j == 0) ? 0 : (j == BIS_P ? n : c);
 }
 
 // Multisection: L consecutive lanes (L a power of two, L <= 32) share eigenvalue m and, per
@@ -55,21 +139,10 @@ __global__ void k_e2(const double* e, long long n, double* e2) {
 // at the midpoint, for L = 1: plain bisection), so the chain of dependent Sturm passes per
 // eigenvalue is log2(L + 1) times shorter, for L times more total passes; the host picks L.
 // Stopping rule as in bisection: width <= 2 eps max(|a|, |b|) + pivmin, or no double between.
-// Coarse round: Sturm counts at the P + 1 points x_j = lo + (hi - lo) j / P of the Gershgorin
-// interval (count 0 at lo and n at hi by construction), one thread per point.
-constexpr int BIS_P = 32768;
-__global__ void k_bisect_grid(const double* __restrict__ d, const double* __restrict__ e2, long long n, double lo,
-                              double hi, double pivmin, double* __restrict__ xg, int* __restrict__ cg) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j > BIS_P) return;
-  const double x = (j == BIS_P) ? hi : lo + (hi - lo) * ((double)j / (double)BIS_P);
-  xg[j] = x;
-  cg[j] = (j == 0) ? 0 : (j == BIS_P ? (int)n : sturm_count(d, e2, n, x, pivmin));
-}
-
-__global__ void __launch_bounds__(128) k_bisect(const double* __restrict__ d, const double* __restrict__ e2, long long n,
-                                                const double* __restrict__ xg, const int* __restrict__ cg,
-                                                double pivmin, int L, double* lam) {
+__global__ void __launch_bounds__(TD_TILE) k_bisect(const double2* __restrict__ rec, int ntile, long long n,
+                                                    const double* __restrict__ xg, const int* __restrict__ cg,
+                                                    double pivmin, double sc, int L, double* lam) {
+  __shared__ __align__(16) double2 ring[TD_ST][TD_TILE];
   const long long gt = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const long long m = gt / L;
   const int lane = threadIdx.x & 31, sl = lane & (L - 1), base = lane - sl;
@@ -90,9 +163,9 @@ __global__ void __launch_bounds__(128) k_bisect(const double* __restrict__ d, co
   for (int it = 0; it < 256; ++it) {
     const double mid = 0.5 * (a + b);
     const bool done = !active || !(mid > a && mid < b) || (b - a <= 2.0 * DBL_EPSILON * fmax(fabs(a), fabs(b)) + pivmin);
-    if (__all_sync(0xffffffffu, done)) break;
+    if (__syncthreads_and(done)) break;
     const double x = (L == 1) ? mid : a + (b - a) * ((double)(sl + 1) / (double)(L + 1));
-    const bool le = !done && sturm_count(d, e2, n, x, pivmin) <= m;
+    const bool le = block_sturm(rec, ntile, x * sc, ring) <= m && !done;
     const unsigned gb = (__ballot_sync(0xffffffffu, le) >> base) & (L == 32 ? 0xffffffffu : ((1u << L) - 1u));
     const int jhi = gb ? 31 - __clz(gb) : -1;   // highest point with count <= m
     const double xa = __shfl_sync(0xffffffffu, x, base + max(jhi, 0));
@@ -105,19 +178,16 @@ __global__ void __launch_bounds__(128) k_bisect(const double* __restrict__ d, co
   if (active && sl == 0) lam[m] = 0.5 * (a + b);
 }
 
-// Lanes per eigenvalue for k_bisect.  A round costs one Sturm pass (n dependent steps of about
-// 170 cycles) when the SM sub-partitions are idle, and n L / 32 warp passes of about 50 issue
-// cycles per step spread over 4 nsm sub-partitions when they are full; after the coarse round
-// (15 bits) rounds ~ 38 / log2(L+1).  (Constants fitted to B200 timings at N = 2304 and 9216
-// over L = 4 .. 32.)
+// Lanes per eigenvalue for k_bisect: after the coarse round (15 bits) rounds ~ 38 / log2(L+1), each of n
+// steps of about 21 cycles with one block on an SM and of 15 per block with more
+// (N = 576 with L = 32, 3600 with L = 4, 14400 with L = 1 and the coarse round).
 int bisect_lanes(long long n, int nsm) {
   int best = 1;
   double bt = 1e300;
   for (int L = 1; L <= 32; L *= 2) {
     const double rounds = std::ceil(38.0 / std::log2((double)L + 1.0));
-    const double lat = 170.0 * (double)n;
-    const double thr = 50.0 * (double)n * (double)n * (double)L / 32.0 / (4.0 * std::max(nsm, 1));
-    const double t = rounds * std::max(lat, thr);
+    const double blocks = std::ceil(std::ceil((double)n * L / TD_TILE) / std::max(nsm, 1));
+    const double t = rounds * std::max(21.0, 15.0 * blocks);
     if (t < bt) {
       bt = t;
       best = L;
@@ -139,7 +209,7 @@ struct InvArgs {
   const double* e;
   long long n;
   const double* lam;
-  const int* csize;     // cluster size at a leader index, 0 for non-leaders
+  const int* csize;     // cluster size at a leader index that is to be done, 0 for the others
   long long m0;         // first eigenvalue index of the chunk
   long long m1;         // one past the last eigenvalue index of the chunk
   int M;                // slots in the chunk
@@ -152,6 +222,335 @@ struct InvArgs {
   double* zsel;         // selected vectors (column-major n x nsel) or null
   long long zs0, zs1;
 };
+
+// act(a, b) = Re[(z^T g_a) conj(z^T g'_b)], g' = g (dielbsev/dielbsep) or the f-weighted
+// vectors with temperature (dielbseptemp)
+__device__ __forceinline__ void write_act(const double2* sg, int ng, int dtfull, int cpol, double* act, long long n,
+                                          long long mm) {
+  auto re = [&](int p, int q) {
+    const double2 u = sg[p], v = (ng == 10) ? sg[5 + q] : sg[q];
+    return u.x * v.x + u.y * v.y;
+  };
+  act[0 * n + mm] = re(0, 0);
+  act[1 * n + mm] = re(1, 1);
+  act[2 * n + mm] = re(2, 2);
+  act[3 * n + mm] = dtfull ? re(0, 1) : 0.0;
+  act[4 * n + mm] = dtfull ? re(0, 2) : 0.0;
+  act[5 * n + mm] = dtfull ? re(1, 2) : 0.0;
+  act[6 * n + mm] = cpol ? re(3, 3) : 0.0;
+  act[7 * n + mm] = cpol ? re(4, 4) : 0.0;
+}
+
+struct TwistArgs {
+  const double2* rec;   // vector records of k_td_records
+  int n, npad;
+  double sc;
+  const double* lam;
+  const int* csize;     // cluster size at a leader index, 0 for non-leaders
+  int* todo;            // csize of the leaders that k_inviter has to do
+  int m0, m1, M;        // eigenvalue indices of the chunk; slots (a multiple of 32)
+  double* t;            // [npad][M]: the recurrence from the top; for members of clusters then the vector
+  int* te;              // [npad / 8][M]: its exponents
+  const double2* g;     // [NG][n]
+  double* act;
+  int dtfull, cpol;
+  double rtol;          // largest residual of the joined row, ||sc T|| <= 1
+};
+
+// Eigenvector m of T without a factorisation, one lane each.  From the top z_{k+1} = -((d_k - lam) z_k + e_{k-1}
+// z_{k-1}) / e_k, and from the bottom the same upwards, satisfy every row of T - lam to rounding; joined at the
+// row r where |top_r bottom_r| is largest (there the diagonal of (T - lam)^-1 is largest, and so the residual of
+// the one row left smallest) they are the eigenvector, and that row's residual over the norm tells how good.
+// Three passes: top (stored, 8 bytes a step), bottom (finds r), bottom again with the sums over the joined vector.
+// Every eight steps the pair is scaled by a power of two.  A chain of an FMA and a multiplication a step, no
+// division, and one pass written and one and a half read, against three factorisations with their divisions and
+// 33 passes in inverse iteration.  Bound by that chain where the vectors are few: N = 576 0.82 -> 0.07 ms, 3600
+// 6.4 -> 0.42 ms, 14400 (one launch; a cluster of two in it made 51 ms) 1.8 ms.
+constexpr int TW = 32;   // rows of a tile of the ring
+constexpr int TW_ST = 3;
+template <int NGT>
+struct __align__(16) TwTile {
+  double2 rec[2 * TW];
+  double t[TW][32];
+  int te[TW / 8][32];
+  double2 g[NGT][TW];
+};
+__device__ __forceinline__ double tw_step(double a, double z, double e, double zp, double nie) {
+  return __dmul_rn(__fma_rn(a, z, __dmul_rn(e, zp)), nie);
+}
+__device__ __forceinline__ double pow2_clamped(int x) {
+  return __hiloint2double((min(max(x, -1023), 1000) + 1023) << 20, 0);   // 0 below 2^-1022
+}
+
+template <int NGT>
+__global__ void __launch_bounds__(32) k_twist(TwistArgs a) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  TwTile<NGT>* ring = reinterpret_cast<TwTile<NGT>*>(smem);
+  const int lane = threadIdx.x, j0 = blockIdx.x * 32, jj = j0 + lane, M = a.M, n = a.n;
+  const int m = min(a.m0 + jj, a.m1 - 1);
+  const bool live = a.m0 + jj < a.m1;
+  const double lam = a.lam[m] * a.sc;
+  const int nt = (n + TW - 1) / TW;
+  double* __restrict__ T = a.t + jj;
+  int* __restrict__ TE = a.te + jj;
+  // what: 1 = records, 2 = + top recurrence, 4 = + g
+  auto issue = [&](int tile, int st, int what) {
+    if (tile >= 0 && tile < nt) {
+      TwTile<NGT>& s = ring[st];
+      const int k0 = tile * TW;
+      cp_async16(&s.rec[lane], a.rec + 2 * (size_t)k0 + lane);
+      cp_async16(&s.rec[lane + 32], a.rec + 2 * (size_t)k0 + lane + 32);
+      if (what & 2) {
+        const int r0 = lane >> 4, c0 = (lane & 15) * 2;
+        for (int q = 0; q < TW; q += 2) cp_async16(&s.t[q + r0][c0], a.t + (size_t)(k0 + q + r0) * M + j0 + c0);
+        cp_async16(&s.te[lane >> 3][(lane & 7) * 4], a.te + (size_t)(k0 / 8 + (lane >> 3)) * M + j0 + (lane & 7) * 4);
+      }
+      if (what & 4)
+        for (int al = 0; al < NGT; ++al) cp_async16(&s.g[al][lane], a.g + (size_t)al * n + min(k0 + lane, n - 1));
+    }
+    cp_async_commit();
+  };
+  // ---- from the top
+  {
+    double z = 1.0, zp = 0.0, ep = 0.0;
+    int E = 0;
+    for (int t = 0; t < TW_ST - 1; ++t) issue(t, t, 1);
+    for (int t = 0; t < nt; ++t) {
+      cp_async_wait<TW_ST - 2>();
+      __syncwarp();
+      issue(t + TW_ST - 1, (t + TW_ST - 1) % TW_ST, 1);
+      const TwTile<NGT>& s = ring[t % TW_ST];
+      for (int b = 0; b < TW; b += 8) {
+        E += rescale(z, zp);
+        TE[(size_t)((t * TW + b) >> 3) * M] = E;
+        double2 de[8];
+        double nie[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          de[q] = s.rec[2 * (b + q)];
+          nie[q] = s.rec[2 * (b + q) + 1].x;
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          T[(size_t)(t * TW + b + q) * M] = z;
+          const double zn = tw_step(__dsub_rn(de[q].x, lam), z, ep, zp, nie[q]);
+          zp = z;
+          z = zn;
+          ep = de[q].y;
+        }
+      }
+    }
+  }
+  __threadfence_block();
+  cp_async_wait<0>();
+  __syncwarp();
+  // ---- from the bottom: r, and the two values there
+  const double z0 = (n % 8) ? 0.0 : 1.0;   // blocks of eight rows: the last may begin behind row n - 1
+  int r = n - 1, bE = 0, bTE = 0, bBE = 0;
+  double bM = 0.0, bT = 1.0, bB = 1.0;
+  bool have = false;
+  {
+    double z = z0, zp = 0.0;
+    int E = 0;
+    for (int t = 0; t < TW_ST - 1; ++t) issue(nt - 1 - t, t, 3);
+    for (int t = 0; t < nt; ++t) {
+      cp_async_wait<TW_ST - 2>();
+      __syncwarp();
+      issue(nt - 1 - (t + TW_ST - 1), (t + TW_ST - 1) % TW_ST, 3);
+      const TwTile<NGT>& s = ring[t % TW_ST];
+      const int k0 = (nt - 1 - t) * TW;
+      for (int b = TW - 8; b >= 0; b -= 8) {
+        if (k0 + b >= n) continue;
+        E += rescale(z, zp);
+        double vb = 0.0, tb = 1.0, bb = 1.0, tv[8], nie[8];
+        double2 de[8];
+        int kb = 0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          de[q] = s.rec[2 * (b + q)];
+          nie[q] = s.rec[2 * (b + q) + 1].y;
+          tv[q] = s.t[b + q][lane];
+        }
+#pragma unroll
+        for (int q = 7; q >= 0; --q) {
+          const double v = fabs(tv[q] * z);
+          if (v > vb) {
+            vb = v;
+            kb = q;
+            tb = tv[q];
+            bb = z;
+          }
+          const double zn = tw_step(__dsub_rn(de[q].x, lam), z, de[q].y, zp, nie[q]);
+          zp = z;
+          z = zn;
+          if (k0 + b + q == n) z = 1.0;   // rows behind the last: zeros up to it
+        }
+        const int tE = s.te[b >> 3][lane], h = __double2hiint(vb), ve = tE + E + (h >> 20) - 1023;
+        const double vm = __hiloint2double((h & 0x000fffff) | 0x3ff00000, __double2loint(vb));
+        if (vb > 0.0 && (!have || ve > bE || (ve == bE && vm > bM))) {
+          have = true;
+          bE = ve;
+          bM = vm;
+          r = k0 + b + kb;
+          bT = tb;
+          bTE = tE;
+          bB = bb;
+          bBE = E;
+        }
+      }
+    }
+  }
+  cp_async_wait<0>();
+  __syncwarp();
+  // ---- from the bottom again, joined with the top at r and scaled to z_r = 1
+  const bool member = a.csize[m] != 1, members = __any_sync(0xffffffffu, member);
+  const double st = 1.0 / bT, sb = 1.0 / bB;
+  const int rmax = __reduce_max_sync(0xffffffffu, r);
+  double2 sg[NGT];
+#pragma unroll
+  for (int al = 0; al < NGT; ++al) sg[al] = make_double2(0, 0);
+  double nrm = 0.0, zup = 0.0, zdn = 0.0;   // z_{r-1}, z_{r+1}
+  {
+    double z = z0, zp = 0.0;
+    int E = 0;
+    auto what = [&](int tile) { return 5 | (tile * TW <= rmax ? 2 : 0); };
+    for (int t = 0; t < TW_ST - 1; ++t) issue(nt - 1 - t, t, what(nt - 1 - t));
+    for (int t = 0; t < nt; ++t) {
+      cp_async_wait<TW_ST - 2>();
+      __syncwarp();
+      const int tn = nt - 1 - (t + TW_ST - 1);
+      issue(tn, (t + TW_ST - 1) % TW_ST, what(tn));
+      const TwTile<NGT>& s = ring[t % TW_ST];
+      const int k0 = (nt - 1 - t) * TW;
+      for (int b = TW - 8; b >= 0; b -= 8) {
+        if (k0 + b >= n) continue;
+        E += rescale(z, zp);
+        const double fb = sb * pow2_clamped(E - bBE);
+        const double ft = st * pow2_clamped(s.te[b >> 3][lane] - bTE);
+        double x[8], nie[8];
+        double2 de[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          de[q] = s.rec[2 * (b + q)];
+          nie[q] = s.rec[2 * (b + q) + 1].y;
+          x[q] = s.t[b + q][lane] * ft;   // taken up to row r only: a tile without the top is above it
+        }
+#pragma unroll
+        for (int q = 7; q >= 0; --q) {
+          const int k = k0 + b + q;
+          if (k > r) x[q] = z * fb;
+          if (k == r + 1) zdn = x[q];
+          if (k == r - 1) zup = x[q];
+          const double zn = tw_step(__dsub_rn(de[q].x, lam), z, de[q].y, zp, nie[q]);
+          zp = z;
+          z = zn;
+          if (k == n) z = 1.0;
+        }
+#pragma unroll
+        for (int q = 7; q >= 0; --q) {
+          nrm = fma(x[q], x[q], nrm);
+#pragma unroll
+          for (int al = 0; al < NGT; ++al) {
+            const double2 gk = s.g[al][b + q];
+            sg[al].x = fma(x[q], gk.x, sg[al].x);
+            sg[al].y = fma(x[q], gk.y, sg[al].y);
+          }
+        }
+        if (members && member && live) {
+#pragma unroll
+          for (int q = 0; q < 8; ++q) T[(size_t)(k0 + b + q) * M] = x[q];
+        }
+      }
+    }
+  }
+  if (!live) return;
+  const double2 de = a.rec[2 * (size_t)r];
+  const double res = fma(r > 0 ? a.rec[2 * (size_t)r - 2].y : 0.0, zup, fma(de.x - lam, 1.0, (r < n - 1 ? de.y : 0.0) * zdn));
+  if (!have || !(fabs(res) <= a.rtol * sqrt(nrm)) || !(nrm < 1e300)) {
+    int l = m;   // inverse iteration makes this vector, or the cluster that it is in
+    while (l > 0 && a.csize[l] == 0) --l;
+    a.todo[l] = a.csize[l];
+    return;
+  }
+  const double c = 1.0 / sqrt(nrm);
+#pragma unroll
+  for (int al = 0; al < NGT; ++al) sg[al] = cscale(sg[al], c);
+  write_act(sg, NGT, a.dtfull, a.cpol, a.act, n, m);
+}
+
+// The vectors of a cluster, one block each: modified Gram-Schmidt in order against the earlier members, then
+// the sums again.  Where less than a third of a vector is left the members were nearly parallel (eigenvalues
+// equal to rounding), and inverse iteration makes the cluster.
+constexpr int CL_T = 256;
+__device__ __forceinline__ double block_sum(double x, double* red) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = x;
+  __syncthreads();
+  double s = 0.0;
+#pragma unroll
+  for (int q = 0; q < CL_T / 32; ++q) s += red[q];
+  return s;
+}
+template <int NGT>
+__global__ void __launch_bounds__(CL_T) k_cluster(TwistArgs a) {
+  __shared__ double red[CL_T / 32];
+  const int m = a.m0 + blockIdx.x, cs = a.csize[m], n = a.n, tid = threadIdx.x;
+  if (cs < 2 || a.todo[m] != 0) return;
+  double* __restrict__ X = a.t + blockIdx.x;
+  const size_t M = (size_t)a.M;
+  for (int s = 0; s < cs; ++s) {
+    double before = 0.0, left = 0.0;
+    for (int k = tid; k < n; k += CL_T) before = fma(X[k * M + s], X[k * M + s], before);
+    before = block_sum(before, red);
+    for (int t = 0; t < s; ++t) {
+      double dot = 0.0;
+      for (int k = tid; k < n; k += CL_T) dot = fma(X[k * M + s], X[k * M + t], dot);
+      dot = block_sum(dot, red);
+      for (int k = tid; k < n; k += CL_T) X[k * M + s] = fma(-dot, X[k * M + t], X[k * M + s]);
+    }
+    for (int k = tid; k < n; k += CL_T) left = fma(X[k * M + s], X[k * M + s], left);
+    left = block_sum(left, red);
+    if (!(left >= 0.1 * before)) {
+      if (tid == 0) a.todo[m] = cs;
+      return;
+    }
+    const double c = 1.0 / sqrt(left);
+    double2 sg[NGT];
+#pragma unroll
+    for (int al = 0; al < NGT; ++al) sg[al] = make_double2(0, 0);
+    for (int k = tid; k < n; k += CL_T) {
+      const double x = X[k * M + s] * c;
+      X[k * M + s] = x;
+#pragma unroll
+      for (int al = 0; al < NGT; ++al) {
+        const double2 gk = a.g[(size_t)al * n + k];
+        sg[al].x = fma(x, gk.x, sg[al].x);
+        sg[al].y = fma(x, gk.y, sg[al].y);
+      }
+    }
+#pragma unroll
+    for (int al = 0; al < NGT; ++al) {
+      sg[al].x = block_sum(sg[al].x, red);
+      sg[al].y = block_sum(sg[al].y, red);
+    }
+    if (tid == 0) write_act(sg, NGT, a.dtfull, a.cpol, a.act, n, m + s);
+  }
+}
+
+template <int NGT>
+static int launch_twist(wtbg_ctx* ctx, const TwistArgs& a, bool clusters) {
+  const int cnt = a.m1 - a.m0, smem = TW_ST * (int)sizeof(TwTile<NGT>);
+  CK(cudaFuncSetAttribute(k_twist<NGT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  k_twist<NGT><<<(cnt + 31) / 32, 32, smem, ctx->stream>>>(a); WTBG_COUNT(ctx, 1);
+  CKL("k_twist");
+  if (clusters) {
+    k_cluster<NGT><<<cnt, CL_T, 0, ctx->stream>>>(a); WTBG_COUNT(ctx, 1);
+    CKL("k_cluster");
+  }
+  return 0;
+}
 
 constexpr int SB = 8;   // inverse-iteration steps whose loads are issued together
 
@@ -298,19 +697,7 @@ __global__ void __launch_bounds__(64) k_inviter(InvArgs a) {
         if (keep) a.zsel[(mm - a.zs0) * n + k] = x;
       }
     }
-    // act(a, b) = Re[(z^T g_a) conj(z^T g'_b)], g' = g (dielbsev/dielbsep) or the f-weighted
-    // vectors with temperature (dielbseptemp)
-    const int o = (ng == 10) ? 5 : 0;
-    auto re = [&](int p, int q) { return sg[p].x * sg[o + q].x + sg[p].y * sg[o + q].y; };
-    double* act = a.act;
-    act[0 * n + mm] = re(0, 0);
-    act[1 * n + mm] = re(1, 1);
-    act[2 * n + mm] = re(2, 2);
-    act[3 * n + mm] = a.dtfull ? re(0, 1) : 0.0;
-    act[4 * n + mm] = a.dtfull ? re(0, 2) : 0.0;
-    act[5 * n + mm] = a.dtfull ? re(1, 2) : 0.0;
-    act[6 * n + mm] = a.cpol ? re(3, 3) : 0.0;
-    act[7 * n + mm] = a.cpol ? re(4, 4) : 0.0;
+    write_act(sg, ng, a.dtfull, a.cpol, a.act, n, mm);
   }
 }
 
@@ -482,21 +869,25 @@ static int tridiagonal_solve_body(wtbg_ctx* ctx, int dtfull, int cpol, bool vect
   lo -= pad;
   hi += pad;
   ENSURE(ctx->lam, (size_t)n * 8);
-  ENSURE(ctx->tmp2, (size_t)n * 8 + 64);
-  double* e2 = ctx->tmp2.as<double>();
-  if (n > 1) {
-    k_e2<<<(int)((n + 255) / 256), 256, 0, s>>>(ctx->e.as<double>(), n, e2); WTBG_COUNT(ctx, 1);
-    CKL("k_e2");
-  }
+  // the recurrences run on T scaled by a power of two to ||T|| <= 1
+  int ex = 0;
+  if (tnorm > 0.0 && std::isfinite(tnorm)) (void)std::frexp(tnorm, &ex);
+  const double sc = std::ldexp(1.0, -std::min(std::max(ex, -1000), 1000));
+  const int npad = (int)((n + TD_TILE - 1) / TD_TILE * TD_TILE), ntile = npad / TD_TILE;
+  ENSURE(ctx->tmp2, (size_t)npad * 48);
+  double2* rcnt = ctx->tmp2.as<double2>();
+  double2* rvec = rcnt + npad;
+  k_td_records<<<(npad + 255) / 256, 256, 0, s>>>(ctx->d.as<double>(), ctx->e.as<double>(), (int)n, npad, sc, rcnt, rvec);
+  CKL("k_td_records");
   if (ctx->nsm <= 0) cudaDeviceGetAttribute(&ctx->nsm, cudaDevAttrMultiProcessorCount, ctx->device);
   const int lanes = bisect_lanes(n, ctx->nsm);
   ENSURE(ctx->bgrid, (size_t)(BIS_P + 1) * (8 + 4) + 64);
   double* xg = ctx->bgrid.as<double>();
   int* cg = reinterpret_cast<int*>(xg + BIS_P + 1);
-  k_bisect_grid<<<(BIS_P + 1 + 255) / 256, 256, 0, s>>>(ctx->d.as<double>(), e2, n, lo, hi, pivmin, xg, cg);
+  k_bisect_grid<<<(BIS_P + TD_TILE) / TD_TILE, TD_TILE, 0, s>>>(rcnt, ntile, (int)n, lo, hi, sc, xg, cg);
   CKL("k_bisect_grid");
-  k_bisect<<<(int)((n * lanes + 127) / 128), 128, 0, s>>>(ctx->d.as<double>(), e2, n, xg, cg, pivmin, lanes,
-                                                       ctx->lam.as<double>()); WTBG_COUNT(ctx, 2);
+  k_bisect<<<(int)((n * lanes + TD_TILE - 1) / TD_TILE), TD_TILE, 0, s>>>(rcnt, ntile, n, xg, cg, pivmin, sc, lanes,
+                                                                        ctx->lam.as<double>()); WTBG_COUNT(ctx, 3);
   CKL("k_bisect");
   ctx->lam_host.resize(n);
   CK(cudaMemcpyAsync(ctx->lam_host.data(), ctx->lam.as<double>(), n * 8, cudaMemcpyDeviceToHost, s));
@@ -524,9 +915,12 @@ static int tridiagonal_solve_body(wtbg_ctx* ctx, int dtfull, int cpol, bool vect
   M = std::max<long long>(M, maxc);
   M = std::min<long long>(M, n);
   M = std::max<long long>(M, 1);
-  ENSURE(ctx->ws, (size_t)4 * 8 * n * M);
+  const long long tM = (M + 31) / 32 * 32;   // slots of k_twist (its [npad][tM] is smaller but at the smallest n)
+  ENSURE(ctx->ws, std::max<size_t>((size_t)4 * 8 * n * M, (size_t)npad * tM * 8 + (size_t)npad / 8 * tM * 4));
   ENSURE(ctx->act, (size_t)8 * 8 * n);
-  ENSURE(ctx->csz, (size_t)n * 4 + 64);
+  ENSURE(ctx->csz, (size_t)n * 8 + 64);
+  int* todo = ctx->csz.as<int>() + n;
+  CK(cudaMemsetAsync(todo, 0, (size_t)n * 4, s));
   CK(cudaMemcpyAsync(ctx->csz.as<int>(), csize.data(), n * 4, cudaMemcpyHostToDevice, s));
   ctx->csize_host = csize;
   ctx->tnorm = tnorm;
@@ -535,7 +929,7 @@ static int tridiagonal_solve_body(wtbg_ctx* ctx, int dtfull, int cpol, bool vect
   a.e = ctx->e.as<double>();
   a.n = n;
   a.lam = ctx->lam.as<double>();
-  a.csize = ctx->csz.as<int>();
+  a.csize = todo;
   a.ws = ctx->ws.as<double>();
   a.pert = DBL_EPSILON * std::max(tnorm, DBL_MIN);
   a.g = ctx->g.as<double2>();
@@ -546,6 +940,23 @@ static int tridiagonal_solve_body(wtbg_ctx* ctx, int dtfull, int cpol, bool vect
   a.zsel = nullptr;
   a.zs0 = -1;
   a.zs1 = -1;
+  TwistArgs tw;
+  tw.rec = rvec;
+  tw.n = (int)n;
+  tw.npad = npad;
+  tw.sc = sc;
+  tw.lam = a.lam;
+  tw.csize = ctx->csz.as<int>();
+  tw.todo = todo;
+  tw.M = (int)tM;
+  tw.t = ctx->ws.as<double>();
+  tw.te = reinterpret_cast<int*>(tw.t + (size_t)npad * tM);
+  tw.g = a.g;
+  tw.act = a.act;
+  tw.dtfull = dtfull;
+  tw.cpol = cpol;
+  // the residual of the joined row is |lambda's error| / |z_r|, and |z_r| >= ||z|| / sqrt(n)
+  tw.rtol = 8.0 * DBL_EPSILON * std::sqrt((double)n);
   for (long long m0 = 0; m0 < n;) {
     // end the chunk at a cluster start
     long long m1 = std::min(n, m0 + M);
@@ -557,6 +968,9 @@ static int tridiagonal_solve_body(wtbg_ctx* ctx, int dtfull, int cpol, bool vect
     a.m1 = m1;
     a.M = (int)M;
     const int cnt = (int)(m1 - m0);
+    tw.m0 = (int)m0;
+    tw.m1 = (int)m1;
+    if (int r = a.ng == 10 ? launch_twist<10>(ctx, tw, maxc > 1) : launch_twist<5>(ctx, tw, maxc > 1)) return r;
     k_inviter<<<(cnt + 63) / 64, 64, 0, s>>>(a); WTBG_COUNT(ctx, 1);
     CKL("k_inviter");
     m0 = m1;
