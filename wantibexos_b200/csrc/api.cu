@@ -151,7 +151,7 @@ int wtbg_destroy(wtbg_ctx* ctx) {
                     &ctx->yv, &ctx->lam, &ctx->bgrid, &ctx->ws, &ctx->act, &ctx->zsel, &ctx->csz, &ctx->sp_in, &ctx->sp_out,
                     &ctx->sp_om, &ctx->tmp, &ctx->tmp2, &ctx->istat, &ctx->pOpA, &ctx->pOpB,
                     &ctx->pHk, &ctx->pOc, &ctx->pOv, &ctx->pErr, &ctx->triErr, &ctx->gwork,
-                    &ctx->t2V, &ctx->t2X, &ctx->t2D, &ctx->t2G, &ctx->t2T, &ctx->t2P, &ctx->t2AB, &ctx->t2prog, &ctx->t2de};
+                    &ctx->t2V, &ctx->t2X, &ctx->t2G, &ctx->t2T, &ctx->t2P, &ctx->t2AB, &ctx->t2prog, &ctx->t2de};
   for (DevBuf* b : bufs) free_buf(*b);
   for (cudaEvent_t e : ctx->evpool) cudaEventDestroy(e);
   if (ctx->tri_exec) cudaGraphExecDestroy(ctx->tri_exec);

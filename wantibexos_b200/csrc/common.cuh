@@ -102,7 +102,7 @@ struct wtbg_ctx {
   int bulge_warp_mode = 0;   // stage 2: 0 = one CTA per sweep (k_chase), 1 = one warp per sweep (k_bulge)
   int panel_cl_max = 0;          // largest cluster of the panel QR (0: not asked yet)
   long long panel_cl_rows = 0;   // panels of up to so many rows run on one cluster
-  DevBuf t2V, t2X, t2D, t2G, t2T, t2P, t2AB, t2prog, t2de;
+  DevBuf t2V, t2X, t2G, t2T, t2P, t2AB, t2prog, t2de;
   cudaGraphExec_t tri_exec = nullptr;
   std::vector<const void*> tri_sig;
   long long tri_launches = 0;

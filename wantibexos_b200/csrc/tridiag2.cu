@@ -653,35 +653,6 @@ __global__ void __launch_bounds__(PC_THREADS, 1) k_panel_qr_cl(PanelArgs a, int 
 }
 
 
-// Diagonal 64 x 64 tiles of A22 made full Hermitian (lower stored, upper = conj of lower,
-// diagonal real), column-major per tile: Dsym[I][c*64 + r].  Rows/columns past N are zero.
-constexpr int SD_LD = 65;
-constexpr size_t SD_SMEM = (size_t)64 * SD_LD * sizeof(double2);
-__global__ void __launch_bounds__(256) k_symdiag(const double2* __restrict__ A, long long N, long long k0,
-                                                 double2* __restrict__ Dsym) {
-  // the tile's lower half read once with coalesced loads into sL [c][r], then written out full
-  extern __shared__ __align__(16) double2 sL[];
-  const long long I0 = k0 + (long long)blockIdx.x * 64;
-  double2* D = Dsym + (size_t)blockIdx.x * 64 * 64;
-  for (int e = threadIdx.x; e < 64 * 64; e += 256) {
-    const int r = e & 63, c = e >> 6;
-    const long long gr = I0 + r, gc = I0 + c;
-    sL[c * SD_LD + r] = (r >= c && gr < N && gc < N) ? A[gr + gc * N] : make_double2(0, 0);
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < 64 * 64; e += 256) {
-    const int r = e & 63, c = e >> 6;
-    const long long gr = I0 + r, gc = I0 + c;
-    double2 v = make_double2(0, 0);
-    if (gr < N && gc < N) {
-      if (r > c) v = sL[c * SD_LD + r];
-      else if (r < c) v = cconj(sL[r * SD_LD + c]);
-      else v = make_double2(sL[c * SD_LD + r].x, 0.0);
-    }
-    D[e] = v;
-  }
-}
-
 // D += A B with A 16x16 (a_i: row gq + 8*(i%2), k = tq + 4*(i/2)) and B 16x8 (b_j: k = tq + 4*j,
 // column gq): FP64 tensor-core MMA.
 __device__ __forceinline__ void dmma16(double (&c)[4], const double (&a)[8], const double (&b)[4]) {
@@ -704,7 +675,8 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // CTA (I, s): the 64 rows I of X, column blocks J of A22 in split s, K staged in chunks of 32
 // through a two-stage cp.async ring.  The A operand of chunk (J, kc) is A[I, J] (J < I, staged
 // k-major), conj(A[J, I])^T (J > I, staged row-major, conjugated when the fragment is built) or
-// the symmetrised diagonal tile (J = I).  Complex products as real MMAs with the real and
+// the diagonal tile (J = I, each element from the stored triangle, the mirrored ones conjugated and the
+// diagonal made real when the fragment is built).  Complex products as real MMAs with the real and
 // imaginary parts concatenated along k: X_re = [Ar | Ai] [Vr; -Vi], X_im = [Ar | Ai] [Vi; Vr].
 // Warp (wr, wc): rows 16 wr .. +16, columns 16 wc .. +16 (two 8-wide n blocks).
 constexpr int HM_LDA = 66;   // sA[k][row], 64 rows + 2 (conflict-free fragment loads)
@@ -716,8 +688,8 @@ constexpr int HM_STAGE = HM_ABUF + 32 * HM_LDV;
 constexpr size_t HM_SMEM = 2 * (size_t)HM_STAGE * sizeof(double2);
 
 __global__ void __launch_bounds__(256, 2) k_hemm2(const double2* __restrict__ A, long long N, long long k0,
-                                                  const double2* __restrict__ Dsym, const double2* __restrict__ V,
-                                                  int nI, int chunkJ, double2* __restrict__ Xpart) {
+                                                  const double2* __restrict__ V, int nI, int chunkJ,
+                                                  double2* __restrict__ Xpart) {
   extern __shared__ __align__(16) double2 hs[];
   const int I = blockIdx.x, sp = blockIdx.y;
   const int J0 = sp * chunkJ, J1 = min(J0 + chunkJ, nI);
@@ -753,10 +725,11 @@ __global__ void __launch_bounds__(256, 2) k_hemm2(const double2* __restrict__ A,
         cp_async16(sA + r * HM_LDT + k, ok ? A + gr + gc * N : A, ok);
       }
     } else {
-      const double2* D = Dsym + (size_t)I * 64 * 64;
       for (int e = tid; e < 64 * 32; e += 256) {
         const int r = e & 63, k = e >> 6;
-        cp_async16(sA + k * HM_LDA + r, D + (size_t)(kc + k) * 64 + r, true);
+        const long long lo = max(rI + r, cJ + k), hi = min(rI + r, cJ + k);
+        const bool ok = lo < N;
+        cp_async16(sA + k * HM_LDA + r, ok ? A + lo + hi * N : A, ok);
       }
     }
     for (int e = tid; e < 32 * 32; e += 256) {
@@ -776,8 +749,8 @@ __global__ void __launch_bounds__(256, 2) k_hemm2(const double2* __restrict__ A,
     __syncthreads();
     const double2* sA = hs + (size_t)(c & 1) * HM_STAGE;
     const double2* sV = sA + HM_ABUF;
-    const bool tr = (J0 + (c >> 1)) > I;
-    const int r0 = wr * 16 + gq, r1 = r0 + 8;
+    const bool tr = (J0 + (c >> 1)) > I, dg = (J0 + (c >> 1)) == I;
+    const int r0 = wr * 16 + gq, r1 = r0 + 8, kc = (c & 1) * 32;
 #pragma unroll
     for (int kk = 0; kk < 32; kk += 8) {
       const int ka = kk + tq, kb = ka + 4;
@@ -792,6 +765,13 @@ __global__ void __launch_bounds__(256, 2) k_hemm2(const double2* __restrict__ A,
         x10 = sA[ka * HM_LDA + r1];
         x01 = sA[kb * HM_LDA + r0];
         x11 = sA[kb * HM_LDA + r1];
+        if (dg) {
+          auto herm = [](double2& x, int d) { x.y = d > 0 ? x.y : (d < 0 ? -x.y : 0.0); };   // d = row - column
+          herm(x00, r0 - kc - ka);
+          herm(x10, r1 - kc - ka);
+          herm(x01, r0 - kc - kb);
+          herm(x11, r1 - kc - kb);
+        }
       }
       const double a[8] = {x00.x, x10.x, x01.x, x11.x, x00.y, x10.y, x01.y, x11.y};
 #pragma unroll
@@ -817,128 +797,234 @@ __global__ void __launch_bounds__(256, 2) k_hemm2(const double2* __restrict__ A,
     }
 }
 
-constexpr int XR_LD = 65;   // row stride of sX, sV: odd, so the Gram loads of 32 columns hit distinct banks
-constexpr size_t XR_SMEM = (size_t)(32 * XR_LD + 32 * 32 + 32 * XR_LD) * sizeof(double2);
-// X = sum of the split partials; Y = X T into Wp; partial G_b = V_b^H Y_b over the 64 rows of
-// this block (Gpart[b][i + 32 j]).  Every sum keeps its order; the independent sums of a thread
-// are interleaved and the split partials' loads issued together (the kernel is latency-bound).
-__global__ void __launch_bounds__(256) k_xreduce(const double2* __restrict__ Xpart, int S, long long N, long long k0,
-                                                 const double2* __restrict__ T, const double2* __restrict__ V,
-                                                 double2* __restrict__ Wp, double2* __restrict__ Gpart) {
-  extern __shared__ __align__(16) double2 xsm[];   // sX [32][XR_LD], sT [32][32], sV [32][XR_LD]
-  double2* sX = xsm;
-  double2* sT = sX + 32 * XR_LD;
-  double2* sV = sT + 32 * 32;
-  const long long m = N - k0;
-  const long long rb = (long long)blockIdx.x * 64;
-  const int tid = threadIdx.x;
-  for (int e = tid; e < 32 * 32; e += 256) sT[e] = T[e];
-  for (int e = tid; e < 32 * 64; e += 256) {
-    const int r = e & 63, c = e >> 6;
-    const long long rr = rb + r;
-    double2 x = make_double2(0, 0), v = make_double2(0, 0);
-    if (rr < m) {
-      double2 xp[8];
-#pragma unroll
-      for (int s = 0; s < 8; ++s) xp[s] = (s < S) ? Xpart[((size_t)s * 32 + c) * (size_t)m + rr] : make_double2(0, 0);
-#pragma unroll
-      for (int s = 0; s < 8; ++s)
-        if (s < S) x = cadd(x, xp[s]);
-      v = V[k0 + rr + (long long)c * N];
+// W of a panel from X = A22 V (split partials): one cooperative launch for what needs the whole column range
+// three times over.  With C1 = Wacc^H V, C2 = Vacc^H V for the pending updates of the look-ahead group (K = 32 KB
+// columns), B = V^H X - C2^H C1 - C1^H C2 and Z = T^H B:
+//   W = (X - Vacc C1 - Wacc C2 - 1/2 V Z) T.
+// CTA b owns the 16-row tiles b, b + G, ...  (1) sums the split partials and takes its share of V^H X, C1 and C2;
+// (2) after a grid barrier the shares are summed, 32 entries a CTA, in a fixed order; (3, K > 0) after another the
+// 1024 entries of B, a warp each; (4) after the last W.  All products on the FP64 MMA; 16 rows so that up to
+// nsm * 16 rows run side by side.  The work itself is 1 to 7 us of FP64 an SM; as seven launches with their tails,
+// on 64-row blocks and with one CTA summing all shares, it took 76 us a panel at N = 2304,
+// as one 31 (whole stage 1: N = 576 3.04 -> 2.40 ms, 2304 16.6 -> 13.4, 3600 34.9 -> 29.8, 8100 179 -> 167).
+constexpr int WF_TR = 16;
+constexpr int WF_LT = 20;    // row tiles [col][row], 16 rows + 4
+constexpr int WF_LS = 36;    // 32 x 32 matrices [col][row]
+constexpr size_t wf_smem(int KB) {
+  return (size_t)((64 * KB + 64) * WF_LT + 32 * (64 * KB + 36) + 32 * WF_LS + 32 * WF_TR) * sizeof(double2);
+}
+struct WfArgs {
+  double2* X;            // [S][32][m] split partials; slot 0 takes their sum
+  int S;
+  long long N, k0;
+  const double2 *V, *T, *Vacc, *Wacc;
+  double2* W;
+  double2* part;         // [G][1 + 2 KB][32 x 32]
+  double2* red;          // [1 + 2 KB][32 x 32], then B
+  unsigned int* cnt;     // this launch's grid-barrier counter (zero at launch)
+  int* err;
+};
+// c += a b for a 16 x 8 (complex) fragment a = (x00 x01; x10 x11) and b = (v0; v1): see dmma16
+__device__ __forceinline__ void cmma(double (&cr)[4], double (&ci)[4], double2 x00, double2 x10, double2 x01, double2 x11,
+                                     double2 v0, double2 v1) {
+  const double a[8] = {x00.x, x10.x, x01.x, x11.x, x00.y, x10.y, x01.y, x11.y};
+  const double bre[4] = {v0.x, v1.x, -v0.y, -v1.y};
+  const double bim[4] = {v0.y, v1.y, v0.x, v1.x};
+  dmma16(cr, a, bre);
+  dmma16(ci, a, bim);
+}
+
+template <int KB>
+__global__ void __launch_bounds__(256, 1) k_wfuse(WfArgs a) {
+  constexpr int K = 32 * KB, NB = 1 + 2 * KB, LDC = 2 * K + 36;
+  extern __shared__ __align__(16) double2 wsm[];
+  double2* sL = wsm;                        // [Vacc | Wacc | V][WF_LT]
+  double2* sV = sL + (size_t)2 * K * WF_LT;
+  double2* sX = sV + 32 * WF_LT;
+  double2* sC = sX + 32 * WF_LT;            // [col][C1; C2; Z / 2]
+  double2* sT = sC + 32 * LDC;
+  double2* sP = sT + 32 * WF_LS;            // [col][row] half sums
+  const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5, gq = lane >> 2, tq = lane & 3;
+  const int G = gridDim.x, bid = blockIdx.x;
+  const long long m = a.N - a.k0;
+  const int ntile = (int)((m + WF_TR - 1) / WF_TR);
+  auto load_tile = [&](long long r0) {
+    for (int e = tid; e < (2 * K + 32) * WF_TR; e += 256) {
+      const int r = e % WF_TR, q = e / WF_TR;
+      const double2* src = q < K ? a.Vacc + (long long)q * a.N : (q < 2 * K ? a.Wacc + (long long)(q - K) * a.N
+                                                                            : a.V + (long long)(q - 2 * K) * a.N);
+      sL[q * WF_LT + r] = r0 + r < m ? src[a.k0 + r0 + r] : make_double2(0, 0);
     }
-    sX[c * XR_LD + r] = x;
-    sV[c * XR_LD + r] = v;
-  }
-  __syncthreads();
-  // y[u] = sum_{i <= j_u} X[r][i] T[i][j_u], j_u = tid/64 + 4u, the eight chains interleaved
-  double2 y[8];
-  const int r = tid & 63, jb0 = tid >> 6;
-#pragma unroll
-  for (int u = 0; u < 8; ++u) y[u] = make_double2(0, 0);
-  for (int i = 0; i <= jb0 + 28; ++i) {
-    const double2 xi = sX[i * XR_LD + r];
-#pragma unroll
-    for (int u = 0; u < 8; ++u)
-      if (i <= jb0 + 4 * u) y[u] = cadd(y[u], cmul(xi, sT[i + (jb0 + 4 * u) * 32]));
-  }
-  __syncthreads();
-#pragma unroll
-  for (int u = 0; u < 8; ++u) {
-    const int j = jb0 + 4 * u;
-    sX[j * XR_LD + r] = y[u];
-    if (rb + r < m) Wp[k0 + rb + r + (long long)j * N] = y[u];
-  }
-  __syncthreads();
-  // G[i][j] = sum_r conj(V[r][i]) Y[r][j]: thread t takes (i, j) = (t mod 32, t/32 + 8k), k < 4
+  };
+  // (1)
   {
-    const int i = tid & 31, j0 = tid >> 5;
-    double2 g4[4] = {make_double2(0, 0), make_double2(0, 0), make_double2(0, 0), make_double2(0, 0)};
-    for (int rr = 0; rr < 64; ++rr) {
-      const double2 vi = sV[i * XR_LD + rr];
+    const int ih = (wp & 1) * 16, col = (wp >> 1) * 8 + gq;
+    double cr[NB][4], ci[NB][4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) g4[k] = cadd(g4[k], cmulc(vi, sX[(j0 + 8 * k) * XR_LD + rr]));
+    for (int b = 0; b < NB; ++b)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) cr[b][k] = ci[b][k] = 0.0;
+    for (int t = bid; t < ntile; t += G) {
+      const long long r0 = (long long)t * WF_TR;
+      __syncthreads();
+      for (int e = tid; e < 32 * WF_TR; e += 256) {
+        const int r = e % WF_TR, c = e / WF_TR;
+        double2 x = make_double2(0, 0);
+        if (r0 + r < m) {
+          double2 xp[8];
+#pragma unroll
+          for (int s = 0; s < 8; ++s)
+            xp[s] = (s < a.S) ? a.X[((size_t)s * 32 + c) * (size_t)m + r0 + r] : make_double2(0, 0);
+#pragma unroll
+          for (int s = 0; s < 8; ++s)
+            if (s < a.S) x = cadd(x, xp[s]);
+          a.X[(size_t)c * m + r0 + r] = x;
+        }
+        sX[c * WF_LT + r] = x;
+      }
+      load_tile(r0);
+      __syncthreads();
+#pragma unroll
+      for (int kk = 0; kk < WF_TR; kk += 8) {
+        const int ka = kk + tq, kb = ka + 4;
+        const double2 v0 = sV[col * WF_LT + ka], v1 = sV[col * WF_LT + kb];
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+          // left operand, conjugate transposed: V, then Wacc (C1), then Vacc (C2)
+          const double2* L = b == 0 ? sV : (b <= KB ? sL + (K + 32 * (b - 1)) * WF_LT : sL + 32 * (b - 1 - KB) * WF_LT);
+          const double2 x00 = cconj(L[(ih + gq) * WF_LT + ka]), x10 = cconj(L[(ih + gq + 8) * WF_LT + ka]);
+          const double2 x01 = cconj(L[(ih + gq) * WF_LT + kb]), x11 = cconj(L[(ih + gq + 8) * WF_LT + kb]);
+          if (b == 0) cmma(cr[b], ci[b], x00, x10, x01, x11, sX[col * WF_LT + ka], sX[col * WF_LT + kb]);
+          else cmma(cr[b], ci[b], x00, x10, x01, x11, v0, v1);
+        }
+      }
     }
 #pragma unroll
-    for (int k = 0; k < 4; ++k) Gpart[(size_t)blockIdx.x * 1024 + i + 32 * (j0 + 8 * k)] = g4[k];
-  }
-}
-
-// M = T^H G, G = sum of the block partials (one CTA, fixed summation order)
-__global__ void __launch_bounds__(1024) k_mform(const double2* __restrict__ Gpart, int nb, const double2* __restrict__ T,
-                                                double2* __restrict__ M) {
-  __shared__ double2 sG[1024];
-  __shared__ double2 sT[1024];
-  const int e = threadIdx.x;
-  double2 t = make_double2(0, 0);
-  for (int b0 = 0; b0 < nb; b0 += 8) {   // in block order, 8 loads issued together
-    double2 pv[8];
+    for (int b = 0; b < NB; ++b)
 #pragma unroll
-    for (int u = 0; u < 8; ++u) pv[u] = (b0 + u < nb) ? __ldcg(Gpart + (size_t)(b0 + u) * 1024 + e) : make_double2(0, 0);
-#pragma unroll
-    for (int u = 0; u < 8; ++u)
-      if (b0 + u < nb) t = cadd(t, pv[u]);
+      for (int k = 0; k < 4; ++k)
+        a.part[((size_t)bid * NB + b) * 1024 + ih + gq + 8 * (k >> 1) + 32 * ((wp >> 1) * 8 + 2 * tq + (k & 1))] =
+            make_double2(cr[b][k], ci[b][k]);
   }
-  sG[e] = t;
-  sT[e] = T[e];
+  if (!grid_sync(a.cnt, G, a.err)) return;
+  // (2)
+  for (int g = bid; g < 32 * NB; g += G) {
+    const double2* p = a.part + (size_t)g * 32 + lane;
+    double2 t = make_double2(0, 0);
+    for (int b0 = wp; b0 < G; b0 += 64) {
+      double2 pv[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) pv[u] = (b0 + 8 * u < G) ? ldcg2(p + (size_t)(b0 + 8 * u) * NB * 1024) : make_double2(0, 0);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) t = cadd(t, pv[u]);
+    }
+    sP[wp * 32 + lane] = t;
+    __syncthreads();
+    if (wp == 0) {
+#pragma unroll
+      for (int u = 1; u < 8; ++u) t = cadd(t, sP[u * 32 + lane]);
+      a.red[g * 32 + lane] = t;
+    }
+    __syncthreads();
+  }
+  if (!grid_sync(a.cnt, 2 * G, a.err)) return;
+  // (3)
+  const double2* B = a.red;
+  if constexpr (KB > 0) {
+    for (int o = bid * 8 + wp; o < 1024; o += G * 8) {
+      const int i = o & 31, j = o >> 5;
+      double2 t = make_double2(0, 0);
+#pragma unroll
+      for (int b = 0; b < KB; ++b) {
+        const double2* c1 = a.red + (1 + b) * 1024 + lane;
+        const double2* c2 = a.red + (1 + KB + b) * 1024 + lane;
+        t = cadd(t, cmulc(ldcg2(c2 + 32 * i), ldcg2(c1 + 32 * j)));
+        t = cadd(t, cmulc(ldcg2(c1 + 32 * i), ldcg2(c2 + 32 * j)));
+      }
+      t = warp_sum2(t);
+      if (lane == 0) a.red[NB * 1024 + o] = csub(ldcg2(a.red + o), t);
+    }
+    if (!grid_sync(a.cnt, 3 * G, a.err)) return;
+    B = a.red + NB * 1024;
+  }
+  // (4) T, B (over the row tiles, which come later), C1, C2; Z / 2 = T^H B / 2
+  for (int e = tid; e < 1024; e += 256) {
+    const int i = e & 31, j = e >> 5;
+    sT[j * WF_LS + i] = i <= j ? a.T[e] : make_double2(0, 0);
+    sL[j * WF_LS + i] = ldcg2(B + e);
+  }
+  for (int e = tid; e < 2 * K * 32; e += 256) {
+    const int b = e >> 10, i = e & 31, j = (e >> 5) & 31;
+    sC[j * LDC + 32 * b + i] = ldcg2(a.red + 1024 + e);
+  }
   __syncthreads();
-  const int i = e & 31, j = e >> 5;
-  double2 s = make_double2(0, 0);
-  for (int l = 0; l <= i; ++l) s = cadd(s, cmulc(sT[l + i * 32], sG[l + j * 32]));   // conj(T[l][i]) G[l][j]
-  M[i + 32 * j] = s;
+  {
+    const int ih = (wp & 1) * 16, cb = (wp >> 1) * 8;
+    double zr[4] = {0, 0, 0, 0}, zi[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int kk = 0; kk < 32; kk += 8) {
+      const int ka = kk + tq, kb = ka + 4;
+      cmma(zr, zi, cconj(sT[(ih + gq) * WF_LS + ka]), cconj(sT[(ih + gq + 8) * WF_LS + ka]),
+           cconj(sT[(ih + gq) * WF_LS + kb]), cconj(sT[(ih + gq + 8) * WF_LS + kb]), sL[(cb + gq) * WF_LS + ka],
+           sL[(cb + gq) * WF_LS + kb]);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      sC[(cb + 2 * tq + (k & 1)) * LDC + 2 * K + ih + gq + 8 * (k >> 1)] = make_double2(0.5 * zr[k], 0.5 * zi[k]);
+  }
+  const int cb = (wp & 3) * 8, kh = wp >> 2;
+  for (int t = bid; t < ntile; t += G) {
+    const long long r0 = (long long)t * WF_TR;
+    __syncthreads();
+    load_tile(r0);
+    for (int e = tid; e < 32 * WF_TR; e += 256) {
+      const int r = e % WF_TR, c = e / WF_TR;
+      sX[c * WF_LT + r] = r0 + r < m ? a.X[(size_t)c * m + r0 + r] : make_double2(0, 0);
+    }
+    __syncthreads();
+    double cr[4] = {0, 0, 0, 0}, ci[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int q = 0; q < (2 * K + 32) / 16; ++q) {
+      const int ka = 8 * (2 * q + kh) + tq, kb = ka + 4;
+      cmma(cr, ci, sL[ka * WF_LT + gq], sL[ka * WF_LT + gq + 8], sL[kb * WF_LT + gq], sL[kb * WF_LT + gq + 8],
+           sC[(cb + gq) * LDC + ka], sC[(cb + gq) * LDC + kb]);
+    }
+    auto at = [&](int k) { return (cb + 2 * tq + (k & 1)) * WF_TR + gq + 8 * (k >> 1); };
+    if (kh == 1) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) sP[at(k)] = make_double2(cr[k], ci[k]);
+    }
+    __syncthreads();
+    if (kh == 0) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int i = (cb + 2 * tq + (k & 1)) * WF_LT + gq + 8 * (k >> 1);
+        sX[i] = csub(sX[i], cadd(make_double2(cr[k], ci[k]), sP[at(k)]));
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 4; ++k) cr[k] = ci[k] = 0.0;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int ka = 8 * (2 * q + kh) + tq, kb = ka + 4;
+      cmma(cr, ci, sX[ka * WF_LT + gq], sX[ka * WF_LT + gq + 8], sX[kb * WF_LT + gq], sX[kb * WF_LT + gq + 8],
+           sT[(cb + gq) * WF_LS + ka], sT[(cb + gq) * WF_LS + kb]);
+    }
+    if (kh == 1) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) sP[at(k)] = make_double2(cr[k], ci[k]);
+    }
+    __syncthreads();
+    if (kh == 0) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const long long r = r0 + gq + 8 * (k >> 1);
+        if (r < m) a.W[a.k0 + r + (long long)(cb + 2 * tq + (k & 1)) * a.N] = cadd(make_double2(cr[k], ci[k]), sP[at(k)]);
+      }
+    }
+  }
 }
-
-// W = Y - 1/2 V M (in place in Wp, rows k0..N-1): 32 rows per CTA, V staged column by column
-// with coalesced loads; element (r, j) sums i in order as before
-constexpr int WF_LD = 33;
-__global__ void __launch_bounds__(256) k_wform(long long N, long long k0, const double2* __restrict__ V,
-                                               const double2* __restrict__ M, double2* __restrict__ Wp) {
-  __shared__ double2 sM[1024];
-  __shared__ double2 sVb[32 * WF_LD];
-  const int tid = threadIdx.x;
-  const long long r0 = k0 + (long long)blockIdx.x * 32;
-  for (int e = tid; e < 1024; e += 256) sM[e] = M[e];
-  for (int e = tid; e < 32 * 32; e += 256) {
-    const int rr = e & 31, i = e >> 5;
-    sVb[i * WF_LD + rr] = (r0 + rr < N) ? V[r0 + rr + (long long)i * N] : make_double2(0, 0);
-  }
-  __syncthreads();
-  const int rr = tid & 31, jg = tid >> 5;   // columns j = jg + 8u, u < 4
-  if (r0 + rr >= N) return;
-  double2 t[4];
-#pragma unroll
-  for (int u = 0; u < 4; ++u) t[u] = make_double2(0, 0);
-  for (int i = 0; i < 32; ++i) {
-    const double2 vi = sVb[i * WF_LD + rr];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) t[u] = cadd(t[u], cmul(vi, sM[i + 32 * (jg + 8 * u)]));
-  }
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    double2* w = Wp + r0 + rr + (long long)(jg + 8 * u) * N;
-    *w = csub(*w, cscale(t[u], 0.5));
-  }
-}
-
 
 // Look-ahead group of panels.  Vacc, Wacc hold the group's V and W side by side (32 columns per
 // panel, leading dimension N); K = 32 * (panels already factored in the group).
@@ -982,96 +1068,6 @@ __global__ void __launch_bounds__(256) k_strip_update(double2* __restrict__ A, l
     double2 a = csub(A[idx], cadd(t0, t1));
     if (r == c0 + c) a.y = 0.0;
     A[idx] = a;
-  }
-}
-
-// Correction Gram matrices over 64-row blocks from row k1: which = 0: C1 = Wacc^H V2,
-// which = 1: C2 = Vacc^H V2 (K x 32 each, part[b][which][i + K j]).  Rows staged in shared memory.
-constexpr int CP_LD = 65;
-__global__ void __launch_bounds__(256) k_cpart(long long N, long long k1, int K, const double2* __restrict__ Vacc,
-                                               const double2* __restrict__ Wacc, const double2* __restrict__ V2,
-                                               double2* __restrict__ part) {
-  // sL [K][CP_LD], sV [32][CP_LD]: the odd row stride keeps a warp's K different rows of sL on
-  // distinct banks
-  extern __shared__ __align__(16) double2 csm[];
-  const int which = blockIdx.y;
-  const double2* L = which ? Vacc : Wacc;
-  double2* sL = csm;
-  double2* sV = csm + (size_t)K * CP_LD;
-  const long long rb = k1 + (long long)blockIdx.x * 64;
-  for (int e = threadIdx.x; e < K * 64; e += 256) {
-    const int u = e & 63, i = e >> 6;
-    const long long r = rb + u;
-    sL[i * CP_LD + u] = r < N ? L[r + (long long)i * N] : make_double2(0, 0);
-  }
-  for (int e = threadIdx.x; e < 32 * 64; e += 256) {
-    const int u = e & 63, j = e >> 6;
-    const long long r = rb + u;
-    sV[j * CP_LD + u] = r < N ? V2[r + (long long)j * N] : make_double2(0, 0);
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < K * 32; e += 256) {
-    const int i = e % K, j = e / K;
-    double2 t0 = make_double2(0, 0), t1 = t0;
-    for (int u = 0; u < 64; u += 2) {
-      t0 = cadd(t0, cmulc(sL[i * CP_LD + u], sV[j * CP_LD + u]));
-      t1 = cadd(t1, cmulc(sL[i * CP_LD + u + 1], sV[j * CP_LD + u + 1]));
-    }
-    part[((size_t)blockIdx.x * 2 + which) * K * 32 + e] = cadd(t0, t1);
-  }
-}
-// C12[which][i + K j] = sum over the blocks (fixed order); grid over entries
-__global__ void __launch_bounds__(256) k_creduce(const double2* __restrict__ part, int nb, int K, double2* __restrict__ C12) {
-  const int e = blockIdx.x * 256 + threadIdx.x;
-  if (e >= 2 * K * 32) return;
-  double2 t0 = make_double2(0, 0), t1 = t0;
-  int b = 0;
-  for (; b + 1 < nb; b += 2) {
-    t0 = cadd(t0, part[(size_t)b * 2 * K * 32 + e]);
-    t1 = cadd(t1, part[(size_t)(b + 1) * 2 * K * 32 + e]);
-  }
-  if (b < nb) t0 = cadd(t0, part[(size_t)b * 2 * K * 32 + e]);
-  C12[e] = cadd(t0, t1);
-}
-// X (the first split partial, [32][m]) -= Vacc C1 + Wacc C2 for the rows from k1: one warp per
-// row, lane = column; C1, C2 in shared memory.
-__global__ void __launch_bounds__(256) k_xcorr(double2* __restrict__ X0, long long N, long long k1, int K,
-                                               const double2* __restrict__ Vacc, const double2* __restrict__ Wacc,
-                                               const double2* __restrict__ C12) {
-  // C1 [K][32] (i + K j), C2, then the 32 rows of Vacc and Wacc [K][33] (staged with coalesced
-  // loads); element (rr, c) sums i in order as before, 32 rows per CTA, lanes along the rows
-  extern __shared__ __align__(16) double2 xsm2[];
-  double2* sVa = xsm2 + 2 * K * 32;
-  double2* sWa = sVa + (size_t)K * 33;
-  const long long m = N - k1;
-  const long long rr0 = (long long)blockIdx.x * 32;
-  for (int e = threadIdx.x; e < 2 * K * 32; e += 256) xsm2[e] = C12[e];
-  for (int e = threadIdx.x; e < K * 32; e += 256) {
-    const int u = e & 31, i = e >> 5;
-    const bool ok = rr0 + u < m;
-    sVa[i * 33 + u] = ok ? Vacc[k1 + rr0 + u + (long long)i * N] : make_double2(0, 0);
-    sWa[i * 33 + u] = ok ? Wacc[k1 + rr0 + u + (long long)i * N] : make_double2(0, 0);
-  }
-  __syncthreads();
-  const int u = threadIdx.x & 31, cg = threadIdx.x >> 5;   // columns c = cg + 8v, v < 4
-  const long long rr = rr0 + u;
-  if (rr >= m) return;
-  double2 t0[4], t1[4];
-#pragma unroll
-  for (int v = 0; v < 4; ++v) t0[v] = t1[v] = make_double2(0, 0);
-  for (int i = 0; i < K; ++i) {
-    const double2 va = sVa[i * 33 + u], wa = sWa[i * 33 + u];
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const int c = cg + 8 * v;
-      t0[v] = cadd(t0[v], cmul(va, xsm2[i + K * c]));
-      t1[v] = cadd(t1[v], cmul(wa, xsm2[K * 32 + i + K * c]));
-    }
-  }
-#pragma unroll
-  for (int v = 0; v < 4; ++v) {
-    const int c = cg + 8 * v;
-    X0[(size_t)c * m + rr] = csub(X0[(size_t)c * m + rr], cadd(t0[v], t1[v]));
   }
 }
 
@@ -1880,11 +1876,11 @@ __global__ void __launch_bounds__(256) k_bt1_apply(const double2* __restrict__ A
 constexpr int PQ_MAX_R = 384;
 constexpr long long LA_FOUR_FROM = 20000;   // N from which groups of four are used
 constexpr int LOOKAHEAD = 4;   // largest number of panels applied per rank-2k update (K = 128)
-// the look-ahead corrections stage K = 32 (group - 1) rows in shared memory (200 KB at 4)
+// k_wfuse holds the K = 32 (group - 1) columns of the group in shared memory (220 KB at 4)
 static_assert(LOOKAHEAD >= 1 && LOOKAHEAD <= 4, "look-ahead groups of 1 to 4 panels");
 // Group size per reduction: the wider update pays off where the trailing matrices are large
 // (config 2, N = 36864: fours 11.75 s, pairs 11.86 s per step); at N = 8100 the update rate does
-// not rise and the corrections cost more (fours 228 ms, pairs 223 ms per config-4 Q).
+// not rise and the corrections cost more (solve: fours 251 ms, pairs 247; N = 2304: 33.1 and 32.0).
 inline int lookahead_group(long long N) { return N >= LA_FOUR_FROM ? 4 : 2; }
 static bool two_stage_fits(wtbg_ctx* ctx, long long N) {
   if (ctx->nsm <= 0) cudaDeviceGetAttribute(&ctx->nsm, cudaDevAttrMultiProcessorCount, ctx->device);
@@ -1902,19 +1898,18 @@ static int two_stage_buffers(wtbg_ctx* ctx, int nband) {
   const long long N = ctx->N;
   const int nsm = ctx->nsm > 0 ? ctx->nsm : 148;
   const long long npan = (N - BW - 1 + BW - 1) / BW;
-  const long long nI = (N + 63) / 64;
   ENSURE(ctx->d, (size_t)N * 8);
   ENSURE(ctx->e, (size_t)N * 8);
   ENSURE(ctx->g, (size_t)N * 16 * NGMAX);
   ENSURE(ctx->Wp, (size_t)N * 16 * LOOKAHEAD * BW);
   ENSURE(ctx->t2V, (size_t)N * 16 * LOOKAHEAD * BW);
   ENSURE(ctx->t2X, (size_t)8 * BW * N * 16);
-  ENSURE(ctx->t2D, (size_t)nI * 64 * 64 * 16);
-  ENSURE(ctx->t2G, (size_t)nI * 1024 * 16 + 1024 * 16 + (size_t)nI * 2 * (LOOKAHEAD - 1) * 1024 * 16 +
-                        (size_t)2 * (LOOKAHEAD - 1) * 1024 * 16);
+  const int la = lookahead_group(N);
+  const long long wfg = std::min<long long>(nsm, (N + WF_TR - 1) / WF_TR);   // CTAs of k_wfuse
+  ENSURE(ctx->t2G, (size_t)((wfg + 1) * (2 * la - 1) + 1) * 1024 * 16);
   ENSURE(ctx->t2T, (size_t)std::max<long long>(npan, 1) * 1024 * 16);
   ENSURE(ctx->t2P, (size_t)nsm * (16 + 2 * 16 * BW + 16 * BW * BW + 16 * BW * NGMAX) + 4096 +
-                        (size_t)std::max<long long>(npan, 1) * 4);
+                        (size_t)std::max<long long>(npan, 1) * 8);
   ENSURE(ctx->t2AB, (size_t)nband * (N + AB_PAD) * LDB * 16);
   ENSURE(ctx->t2prog, (size_t)nband * N * 4 + 64);
   ENSURE(ctx->triErr, 16);
@@ -2000,31 +1995,26 @@ static int run_stage1(wtbg_ctx* ctx, int ng, int band) {
   cudaStream_t s = ctx->stream;
   const int nsm = ctx->nsm > 0 ? ctx->nsm : 148;
   const long long npan = (N - BW - 1 + BW - 1) / BW;
-  const long long nI = (N + 63) / 64;
   const int SMAX = 8;
   double2* A = ctx->H.as<double2>();
   double2* g = ctx->g.as<double2>();
   double2* Vp = ctx->t2V.as<double2>();
   double2* Wp = ctx->Wp.as<double2>();
   double2* Xpart = ctx->t2X.as<double2>();
-  double2* Dsym = ctx->t2D.as<double2>();
-  double2* Gpart = ctx->t2G.as<double2>();
-  double2* Mbuf = Gpart + (size_t)nI * 1024;
-  double2* Cpart = Mbuf + 1024;                                        // look-ahead correction partials
-  double2* Cbuf = Cpart + (size_t)nI * 2 * (LOOKAHEAD - 1) * 1024;     // C1 (K x 32) then C2
+  const int la = std::min(LOOKAHEAD, lookahead_group(N));
+  double2* red = ctx->t2G.as<double2>();                     // sums of k_wfuse, then its CTAs' shares
+  double2* part = red + (size_t)(2 * la) * 1024;
   double2* Tbuf = ctx->t2T.as<double2>();
   char* pb = ctx->t2P.as<char>();
   double2* partW = reinterpret_cast<double2*>(pb + (size_t)nsm * 16);   // 16-byte aligned for any SM count
   double2* partG = partW + (size_t)2 * nsm * BW;
   double2* partVg = partG + (size_t)nsm * BW * BW;
   double2* alpha = partVg + (size_t)nsm * BW * NGMAX;
-  unsigned int* cnt = reinterpret_cast<unsigned int*>(alpha + 2 * BW);   // one barrier counter per panel launch
+  unsigned int* cnt = reinterpret_cast<unsigned int*>(alpha + 2 * BW);   // barrier counters, two per panel
   int* err = ctx->triErr.as<int>();
   if (int r = panel_cluster_limits(ctx)) return r;
-  CK(cudaMemsetAsync(cnt, 0, (size_t)std::max<long long>(npan, 1) * 4, s));
+  CK(cudaMemsetAsync(cnt, 0, (size_t)std::max<long long>(npan, 1) * 8, s));
   CK(cudaFuncSetAttribute(k_hemm2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HM_SMEM));
-  CK(cudaFuncSetAttribute(k_xreduce, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XR_SMEM));
-  CK(cudaFuncSetAttribute(k_symdiag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SD_SMEM));
   // profiling: event pairs around the panel QR, the Hermitian product and the rank-2k update
   // of every panel (read after the stage), and around the stage
   const bool prof = ctx->profiling != 0;
@@ -2079,27 +2069,35 @@ static int run_stage1(wtbg_ctx* ctx, int ng, int band) {
     }
     mark(pnl, 1);
     const int nIm = (int)((m + 63) / 64);
-    k_symdiag<<<nIm, 256, SD_SMEM, s>>>(A, N, k0, Dsym);
     int S = (int)std::min<long long>(SMAX, std::max<long long>(1, (4LL * nsm + nIm - 1) / nIm));
     S = std::min(S, nIm);
     const int chunkJ = (nIm + S - 1) / S;
     S = (nIm + chunkJ - 1) / chunkJ;
     mark(pnl, 2);
-    k_hemm2<<<dim3(nIm, S), 256, HM_SMEM, s>>>(A, N, k0, Dsym, V, nIm, chunkJ, Xpart);
+    k_hemm2<<<dim3(nIm, S), 256, HM_SMEM, s>>>(A, N, k0, V, nIm, chunkJ, Xpart);
     mark(pnl, 3);
-    if (K > 0) {
-      const size_t cps = ((size_t)K * CP_LD + 32 * CP_LD) * 16, xcs = ((size_t)2 * K * 32 + 2 * (size_t)K * 33) * 16;
-      CK(cudaFuncSetAttribute(k_cpart, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cps));
-      CK(cudaFuncSetAttribute(k_xcorr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)xcs));
-      k_cpart<<<dim3(nIm, 2), 256, cps, s>>>(N, k0, K, Vp, Wp, V, Cpart);
-      k_creduce<<<(2 * K * 32 + 255) / 256, 256, 0, s>>>(Cpart, nIm, K, Cbuf);
-      k_xcorr<<<(int)((m + 31) / 32), 256, xcs, s>>>(Xpart, N, k0, K, Vp, Wp, Cbuf);
-      WTBG_COUNT(ctx, 3);
-    }
-    k_xreduce<<<nIm, 256, XR_SMEM, s>>>(Xpart, S, N, k0, Tbuf + (size_t)pnl * 1024, V, Wout, Gpart);
-    k_mform<<<1, 1024, 0, s>>>(Gpart, nIm, Tbuf + (size_t)pnl * 1024, Mbuf);
-    k_wform<<<(int)((m + 31) / 32), 256, 0, s>>>(N, k0, V, Mbuf, Wout);
-    WTBG_COUNT(ctx, 6);
+    WfArgs wa{};
+    wa.X = Xpart;
+    wa.S = S;
+    wa.N = N;
+    wa.k0 = k0;
+    wa.V = V;
+    wa.T = Tbuf + (size_t)pnl * 1024;
+    wa.Vacc = Vp;
+    wa.Wacc = Wp;
+    wa.W = Wout;
+    wa.part = part;
+    wa.red = red;
+    wa.cnt = cnt + npan + pnl;
+    wa.err = err;
+    const long long ntile = (m + WF_TR - 1) / WF_TR, per = (ntile + nsm - 1) / nsm;
+    const void* const wf[LOOKAHEAD] = {(const void*)k_wfuse<0>, (const void*)k_wfuse<1>, (const void*)k_wfuse<2>,
+                                       (const void*)k_wfuse<3>};
+    const size_t wsm = wf_smem(K / 32);
+    CK(cudaFuncSetAttribute(wf[K / 32], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wsm));
+    void* wargs[] = {&wa};
+    CK(cudaLaunchCooperativeKernel(wf[K / 32], dim3((unsigned)((ntile + per - 1) / per)), dim3(256), wargs, wsm, s));
+    WTBG_COUNT(ctx, 3);
     CKL("two-stage panel");
     return 0;
   };
@@ -2108,7 +2106,6 @@ static int run_stage1(wtbg_ctx* ctx, int ng, int band) {
   // its product from the matrix that still lacks those updates (corrected); one rank-2k update
   // with K = 32 x (panels in the group) then applies the whole group to the trailing matrix.
   std::vector<double> her2k_flops(npan, 0.0);
-  const int la = std::min(LOOKAHEAD, lookahead_group(N));
   for (long long p0 = 0; p0 < npan; p0 += la) {
     const int gsz = (int)std::min<long long>(la, npan - p0);
     for (int j = 0; j < gsz; ++j) {
