@@ -523,10 +523,12 @@ template <int N_>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N_) : "memory"); }
 
 // V (row, q) = Vs[row + (vc0 + q) * N]: the panel columns of A in the one-stage reduction, the
-// dense V of the two-stage panel otherwise.
+// dense V of the two-stage panel otherwise.  BESIDE: runs beside the kernel launched before it (the next
+// panel's QR, which shares no data with it) as soon as all CTAs of that one have started; the grid ends after it.
+template <bool BESIDE>
 __global__ void __launch_bounds__(256, 2) k_her2k(double2* A, long long N, const double2* Wp, const double2* Vs,
                                                   int vc0, int jb, int k0) {
-  pdl_enter();
+  if constexpr (!BESIDE) pdl_enter();
   extern __shared__ __align__(16) double2 hsm[];
   const long long t = blockIdx.x;
   int bi = (int)floor((sqrt(8.0 * (double)t + 1.0) - 1.0) * 0.5);
@@ -627,6 +629,9 @@ __global__ void __launch_bounds__(256, 2) k_her2k(double2* A, long long N, const
         A[row + col * N] = v;
       }
     }
+  }
+  if constexpr (BESIDE) {
+    if (blockIdx.x == gridDim.x - 1) asm volatile("griddepcontrol.wait;" ::: "memory");
   }
 }
 
@@ -754,14 +759,16 @@ int autotune_hemv(wtbg_ctx* ctx, int* hs_out) {
   return 0;
 }
 
-// Trailing update of the two-stage panel: A22 -= V W^H + W V^H with V (row, q) = V[row + (vc0 + q) vld]
+// Trailing update of the two-stage panel: A22 -= V W^H + W V^H with V (row, q) = V[row + (vc0 + q) vld];
+// beside: beside the kernel launched last, whose CTAs must leave it room (HER2K_SMEM a CTA) or SMs
 int launch_her2k_v(wtbg_ctx* ctx, double2* A, long long N, const double2* Wp, const double2* V, long long vld, int vc0,
-                   int jb, long long k0) {
+                   int jb, long long k0, bool beside) {
   if (vld != N) return set_err(ctx, WTBG_ERR_ARG, "her2k: V must have leading dimension N");
-  CK(cudaFuncSetAttribute(k_her2k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HER2K_SMEM));
+  const auto fn = beside ? k_her2k<true> : k_her2k<false>;
+  CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HER2K_SMEM));
   const long long T = (N - k0 + TB - 1) / TB;
   const long long ntile = T * (T + 1) / 2;
-  CK(launch_pdl(k_her2k, dim3((unsigned)ntile), dim3(256), HER2K_SMEM, ctx->stream, A, N, Wp, V, vc0, jb, (int)k0));
+  CK(launch_pdl(fn, dim3((unsigned)ntile), dim3(256), HER2K_SMEM, ctx->stream, A, N, Wp, V, vc0, jb, (int)k0));
   WTBG_COUNT(ctx, 1);
   return 0;
 }
@@ -810,7 +817,7 @@ static int run_tridiagonalise1(wtbg_ctx* ctx) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   CK(cudaStreamIsCapturing(s, &cap));
   if (cap == cudaStreamCaptureStatusNone) {
-    CK(cudaFuncSetAttribute(k_her2k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HER2K_SMEM));
+    CK(cudaFuncSetAttribute(k_her2k<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)HER2K_SMEM));
     if (int r = prepare_hemv(ctx)) return r;
     if (int r = autotune_hemv(ctx, &hs)) return r;
   } else {
@@ -865,7 +872,7 @@ static int run_tridiagonalise1(wtbg_ctx* ctx) {
       const long long T = (N - k0 + TB - 1) / TB;
       const long long ntile = T * (T + 1) / 2;
       if (prof) cudaEventRecord(ctx->evpool[evh + 2 * (j0 / NB)], s);
-      CK(launch_pdl(k_her2k, dim3((unsigned)ntile), dim3(256), HER2K_SMEM, s, A, N, (const double2*)Wp,
+      CK(launch_pdl(k_her2k<false>, dim3((unsigned)ntile), dim3(256), HER2K_SMEM, s, A, N, (const double2*)Wp,
                     (const double2*)A, (int)j0, jb, (int)k0)); WTBG_COUNT(ctx, 1);
       if (prof) cudaEventRecord(ctx->evpool[evh + 2 * (j0 / NB) + 1], s);
       CKL("k_her2k");

@@ -31,7 +31,7 @@
 
 // implemented in tridiag.cu
 int launch_her2k_v(wtbg_ctx* ctx, double2* A, long long N, const double2* Wp, const double2* V, long long vld, int vc0,
-                   int jb, long long k0);
+                   int jb, long long k0, bool beside);
 
 namespace {
 
@@ -134,8 +134,11 @@ struct PanelArgs {
 };
 
 __device__ __forceinline__ double2 ldcg2(const double2* p) { return __ldcg(p); }
+// a following kernel launched to run beside this one may start (any other still waits for the end)
+__device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 __global__ void __launch_bounds__(PQ_THREADS, 1) k_panel_qr(PanelArgs a) {
+  pdl_release();
   extern __shared__ __align__(16) double2 P[];   // [jb][R]
   __shared__ double2 s_tau[BW];
   __shared__ double2 s_w[BW];
@@ -474,6 +477,7 @@ __device__ __forceinline__ void cluster_sync() {
 
 template <int NR>
 __global__ void __launch_bounds__(PC_THREADS, 1) k_panel_qr_cl(PanelArgs a, int C) {
+  pdl_release();
   constexpr int R = 8 * NR, VS = R + 1;
   extern __shared__ __align__(16) double2 psm[];
   double2(*s_part)[PC_MAXC][PC_COLS] = reinterpret_cast<double2(*)[PC_MAXC][PC_COLS]>(psm);   // dot products, by parity of p
@@ -1054,18 +1058,24 @@ __global__ void __launch_bounds__(256) k_strip_update(double2* __restrict__ A, l
   const int u = threadIdx.x & 31, cg = threadIdx.x >> 5;
   const long long r = rb + u;
   if (r >= N) return;
+  double2 t0[4], t1[4];
+#pragma unroll
+  for (int v = 0; v < 4; ++v) t0[v] = t1[v] = make_double2(0, 0);
+  for (int q = 0; q < K; q += 2) {
+    const double2 v0 = sVr[q * 33 + u], w0 = sWr[q * 33 + u], v1 = sVr[(q + 1) * 33 + u], w1 = sWr[(q + 1) * 33 + u];
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const int c = cg + 8 * v;
+      t0[v] = cadd(t0[v], cadd(cmulc(sWc[q * 32 + c], v0), cmulc(sVc[q * 32 + c], w0)));
+      t1[v] = cadd(t1[v], cadd(cmulc(sWc[(q + 1) * 32 + c], v1), cmulc(sVc[(q + 1) * 32 + c], w1)));
+    }
+  }
 #pragma unroll
   for (int v = 0; v < 4; ++v) {
     const int c = cg + 8 * v;
     if (c0 + c >= N || r < c0 + c) continue;
-    double2 t0 = make_double2(0, 0), t1 = t0;
-    for (int q = 0; q < K; q += 2) {
-      t0 = cadd(t0, cadd(cmulc(sWc[q * 32 + c], sVr[q * 33 + u]), cmulc(sVc[q * 32 + c], sWr[q * 33 + u])));
-      t1 = cadd(t1, cadd(cmulc(sWc[(q + 1) * 32 + c], sVr[(q + 1) * 33 + u]),
-                         cmulc(sVc[(q + 1) * 32 + c], sWr[(q + 1) * 33 + u])));
-    }
     const long long idx = r + (c0 + c) * N;
-    double2 a = csub(A[idx], cadd(t0, t1));
+    double2 a = csub(A[idx], cadd(t0[v], t1[v]));
     if (r == c0 + c) a.y = 0.0;
     A[idx] = a;
   }
@@ -1901,8 +1911,8 @@ static int two_stage_buffers(wtbg_ctx* ctx, int nband) {
   ENSURE(ctx->d, (size_t)N * 8);
   ENSURE(ctx->e, (size_t)N * 8);
   ENSURE(ctx->g, (size_t)N * 16 * NGMAX);
-  ENSURE(ctx->Wp, (size_t)N * 16 * LOOKAHEAD * BW);
-  ENSURE(ctx->t2V, (size_t)N * 16 * LOOKAHEAD * BW);
+  ENSURE(ctx->Wp, (size_t)N * 16 * 2 * lookahead_group(N) * BW);   // two groups: see run_stage1
+  ENSURE(ctx->t2V, (size_t)N * 16 * 2 * lookahead_group(N) * BW);
   ENSURE(ctx->t2X, (size_t)8 * BW * N * 16);
   const int la = lookahead_group(N);
   const long long wfg = std::min<long long>(nsm, (N + WF_TR - 1) / WF_TR);   // CTAs of k_wfuse
@@ -1934,6 +1944,9 @@ static PanelClFn panel_cl_fn(int nr) {
     default: return k_panel_qr_cl<24>;
   }
 }
+// Shared memory that keeps a panel CTA alone on its SM while the rank-2k update runs beside it (the update
+// takes 66 KB a CTA of the SM's 228).
+constexpr size_t ALONE_SMEM = 168 * 1024;
 static int launch_panel_cluster(wtbg_ctx* ctx, const PanelArgs& pa) {
   const long long m = pa.N - pa.k0;
   int C = 1;
@@ -1941,7 +1954,7 @@ static int launch_panel_cluster(wtbg_ctx* ctx, const PanelArgs& pa) {
   int nr = (int)((m + 8 * C - 1) / (8 * C));
   nr = std::max(4, (nr + 1) & ~1);
   PanelClFn fn = panel_cl_fn(nr);
-  const size_t smem = pc_smem(nr);
+  const size_t smem = std::max(pc_smem(nr), ALONE_SMEM);
   CK(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   if (C > 8) CK(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   cudaLaunchConfig_t cfg{};
@@ -1964,7 +1977,7 @@ static int launch_panel_cluster(wtbg_ctx* ctx, const PanelArgs& pa) {
 static int panel_cluster_limits(wtbg_ctx* ctx) {
   if (ctx->panel_cl_max > 0) return 0;
   PanelClFn fn = panel_cl_fn(PC_MAX_NR);
-  const size_t smem = pc_smem(PC_MAX_NR);
+  const size_t smem = std::max(pc_smem(PC_MAX_NR), ALONE_SMEM);
   CK(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   CK(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   cudaLaunchConfig_t cfg{};
@@ -2030,7 +2043,7 @@ static int run_stage1(wtbg_ctx* ctx, int ng, int band) {
   // Panel QR of panel pnl into V (its 32 columns), then X = A22 V (split K) and W.  Inside a
   // look-ahead group (K > 0) A22 still lacks the updates of the group's K/32 earlier panels
   // (Vacc, Wacc) and the product is corrected by -Vacc C1 - Wacc C2.
-  auto panel = [&](long long pnl, double2* V, double2* Wout, int K) -> int {
+  auto factor = [&](long long pnl, double2* V) -> int {
     const int j0 = (int)(pnl * BW), k0 = j0 + BW;
     const long long m = N - k0;
     const int nref = (int)std::min<long long>(BW, m);
@@ -2061,13 +2074,19 @@ static int run_stage1(wtbg_ctx* ctx, int ng, int band) {
       pa.alpha = alpha;
       pa.cnt = cnt + pnl;
       pa.err = err;
-      const size_t psm = (size_t)BW * (R | 1) * 16;
+      const size_t psm = std::max((size_t)BW * (R | 1) * 16, ALONE_SMEM);
       CK(cudaFuncSetAttribute(k_panel_qr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm));
       if (G > PQ_MAXG) return set_err(ctx, WTBG_ERR_UNSUPPORTED, "panel QR: more CTAs than the column reduction holds");
       void* args[] = {&pa};
       CK(cudaLaunchCooperativeKernel((const void*)k_panel_qr, dim3(G), dim3(PQ_THREADS), args, psm, s));
     }
     mark(pnl, 1);
+    WTBG_COUNT(ctx, 1);
+    return 0;
+  };
+  auto product = [&](long long pnl, const double2* V, const double2* Vacc, const double2* Wacc, double2* Wout, int K) -> int {
+    const int k0 = (int)(pnl * BW) + BW;
+    const long long m = N - k0;
     const int nIm = (int)((m + 63) / 64);
     int S = (int)std::min<long long>(SMAX, std::max<long long>(1, (4LL * nsm + nIm - 1) / nIm));
     S = std::min(S, nIm);
@@ -2083,8 +2102,8 @@ static int run_stage1(wtbg_ctx* ctx, int ng, int band) {
     wa.k0 = k0;
     wa.V = V;
     wa.T = Tbuf + (size_t)pnl * 1024;
-    wa.Vacc = Vp;
-    wa.Wacc = Wp;
+    wa.Vacc = Vacc;
+    wa.Wacc = Wacc;
     wa.W = Wout;
     wa.part = part;
     wa.red = red;
@@ -2097,40 +2116,63 @@ static int run_stage1(wtbg_ctx* ctx, int ng, int band) {
     CK(cudaFuncSetAttribute(wf[K / 32], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wsm));
     void* wargs[] = {&wa};
     CK(cudaLaunchCooperativeKernel(wf[K / 32], dim3((unsigned)((ntile + per - 1) / per)), dim3(256), wargs, wsm, s));
-    WTBG_COUNT(ctx, 3);
+    WTBG_COUNT(ctx, 2);
     CKL("two-stage panel");
+    return 0;
+  };
+  // pending updates of kc columns of V, W on the 32 columns from c0
+  auto strip = [&](long long c0, int kc, const double2* V, const double2* W) -> int {
+    for (int q = 0; q < kc; q += 64) {   // as much as shared memory holds
+      const int kq = std::min(64, kc - q);
+      const size_t sss = ((size_t)2 * 32 * kq + (size_t)2 * 33 * kq) * 16;
+      CK(cudaFuncSetAttribute(k_strip_update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sss));
+      k_strip_update<<<(int)((N - c0 + 31) / 32), 256, sss, s>>>(A, N, c0, kq, V + (size_t)q * N, W + (size_t)q * N);
+      WTBG_COUNT(ctx, 1);
+    }
     return 0;
   };
   // Panels in look-ahead groups of la (up to LOOKAHEAD): panel j of a group first gets the pending
   // updates of the group's earlier panels on its own 32 columns (strip), is factored, and forms
   // its product from the matrix that still lacks those updates (corrected); one rank-2k update
   // with K = 32 x (panels in the group) then applies the whole group to the trailing matrix.
+  // The QR of the next group's first panel, a latency chain on one cluster or 64 CTAs, needs only its own 32
+  // columns: they are updated first (strip), and the rank-2k update of the rest runs beside it.  V and W
+  // of the two groups in turn.  Solve: N = 1156 14.6 -> 14.3 ms, 2304 32.0 -> 30.7, 3600 60.5 -> 57.0,
+  // 8100 247 -> 236, 14400 870 -> 843.
   std::vector<double> her2k_flops(npan, 0.0);
-  for (long long p0 = 0; p0 < npan; p0 += la) {
+  bool factored = false;
+  for (long long p0 = 0, grp = 0; p0 < npan; p0 += la, ++grp) {
     const int gsz = (int)std::min<long long>(la, npan - p0);
+    double2* Vg = Vp + (size_t)(grp & 1) * la * BW * N;
+    double2* Wg = Wp + (size_t)(grp & 1) * la * BW * N;
     for (int j = 0; j < gsz; ++j) {
       const long long pnl = p0 + j;
+      const int K = BW * j;
+      double2* V = Vg + (size_t)K * N;
       if (j > 0) {
-        const long long c0 = pnl * BW;   // the panel's first column (= the previous panel's k0)
-        const long long mc = N - c0;
-        const size_t sss = ((size_t)2 * 32 * j * 32 + (size_t)2 * 32 * j * 33) * 16;
-        CK(cudaFuncSetAttribute(k_strip_update, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sss));
         mark(pnl - 1, 4);
-        k_strip_update<<<(int)((mc + 31) / 32), 256, sss, s>>>(A, N, c0, 32 * j, Vp, Wp);
-        WTBG_COUNT(ctx, 1);
+        if (int r = strip(pnl * BW, K, Vg, Wg)) return r;   // the panel's first column (= the previous panel's k0)
         mark(pnl - 1, 5);
-        her2k_flops[pnl - 1] = 8.0 * (double)mc * 32 * 2 * 32 * j;
+        her2k_flops[pnl - 1] = 8.0 * (double)(N - pnl * BW) * 32 * 2 * K;
       }
-      if (int r = panel(pnl, Vp + (size_t)32 * j * N, Wp + (size_t)32 * j * N, 32 * j)) return r;
+      if (j > 0 || !factored)
+        if (int r = factor(pnl, V)) return r;
+      if (int r = product(pnl, V, Vg, Wg, Wg + (size_t)K * N, K)) return r;
     }
     const long long pl = p0 + gsz - 1;
     const long long kl = (pl + 1) * BW;
     const long long ml = N - kl;
     const int Kg = 32 * (gsz - 1) + (int)std::min<long long>(BW, ml);
-    mark(pl, 4);
-    if (int r = launch_her2k_v(ctx, A, N, Wp, Vp, N, 0, Kg, kl)) return r;
+    factored = pl + 1 < npan;
+    if (factored) {
+      if (int r = strip(kl, Kg, Vg, Wg)) return r;
+      if (int r = factor(pl + 1, Vp + (size_t)((grp + 1) & 1) * la * BW * N)) return r;
+    }
+    mark(pl, 4);   // with profiling the events keep the two apart
+    if (int r = launch_her2k_v(ctx, A, N, Wg, Vg, N, 0, Kg, factored ? kl + BW : kl, factored)) return r;
     mark(pl, 5);
-    her2k_flops[pl] = (double)ml * (ml + 1.0) * 0.5 * 16.0 * Kg;
+    const double mu = (double)(factored ? ml - BW : ml);
+    her2k_flops[pl] = mu * (mu + 1.0) * 0.5 * 16.0 * Kg;
   }
   k_band_extract<<<(unsigned)(N + AB_PAD), BW * 2, 0, s>>>(A, N, ctx->t2AB.as<double2>() + (size_t)band * (N + AB_PAD) * LDB);
   WTBG_COUNT(ctx, 1);
