@@ -15,8 +15,8 @@
 //   * eigenvalues closer than 1e-7 * ||T|| form a cluster: its vectors are orthonormalised in
 //     order (k_cluster), so degenerate excitons get orthogonal vectors;
 //   * what neither makes well (a residual that is too large, a cluster of nearly parallel
-//     vectors) and the vectors of BSE_WF are made by inverse iteration with a partial-pivoting
-//     tridiagonal LU, three steps from a deterministic pseudo-random start vector (k_inviter).
+//     vectors) is made by inverse iteration with a partial-pivoting tridiagonal LU, three steps
+//     from a deterministic pseudo-random start vector (k_inviter).
 // Selected exciton eigenvectors (BSE_WF) are back-transformed A_n = Q z_n panel by panel
 // with the compact-WY form I - V T V^H of each panel's reflectors.
 #include <algorithm>
@@ -255,6 +255,7 @@ struct TwistArgs {
   double* act;
   int dtfull, cpol;
   double rtol;          // largest residual of the joined row, ||sc T|| <= 1
+  bool keep;            // vectors are wanted, not only the sums: k_cluster normalises all of them in t
 };
 
 // Eigenvector m of T without a factorisation, one lane each.  From the top z_{k+1} = -((d_k - lam) z_k + e_{k-1}
@@ -403,7 +404,7 @@ __global__ void __launch_bounds__(32) k_twist(TwistArgs a) {
   cp_async_wait<0>();
   __syncwarp();
   // ---- from the bottom again, joined with the top at r and scaled to z_r = 1
-  const bool member = a.csize[m] != 1, members = __any_sync(0xffffffffu, member);
+  const bool member = a.keep || a.csize[m] != 1, members = __any_sync(0xffffffffu, member);
   const double st = 1.0 / bT, sb = 1.0 / bB;
   const int rmax = __reduce_max_sync(0xffffffffu, r);
   double2 sg[NGT];
@@ -480,7 +481,7 @@ __global__ void __launch_bounds__(32) k_twist(TwistArgs a) {
 
 // The vectors of a cluster, one block each: modified Gram-Schmidt in order against the earlier members, then
 // the sums again.  Where less than a third of a vector is left the members were nearly parallel (eigenvalues
-// equal to rounding), and inverse iteration makes the cluster.
+// equal to rounding), and inverse iteration makes the cluster.  With keep also a vector by itself: normalised.
 constexpr int CL_T = 256;
 __device__ __forceinline__ double block_sum(double x, double* red) {
 #pragma unroll
@@ -497,7 +498,7 @@ template <int NGT>
 __global__ void __launch_bounds__(CL_T) k_cluster(TwistArgs a) {
   __shared__ double red[CL_T / 32];
   const int m = a.m0 + blockIdx.x, cs = a.csize[m], n = a.n, tid = threadIdx.x;
-  if (cs < 2 || a.todo[m] != 0) return;
+  if (cs < (a.keep ? 1 : 2) || a.todo[m] != 0) return;
   double* __restrict__ X = a.t + blockIdx.x;
   const size_t M = (size_t)a.M;
   for (int s = 0; s < cs; ++s) {
@@ -539,13 +540,21 @@ __global__ void __launch_bounds__(CL_T) k_cluster(TwistArgs a) {
   }
 }
 
+// vectors zs0 .. zs1 of the chunk as columns of zsel, except those that k_inviter has made
+__global__ void k_take_vectors(TwistArgs a, int zs0, double* zsel) {
+  const int c = blockIdx.y, m = zs0 + c, k = blockIdx.x * blockDim.x + threadIdx.x;
+  int l = m;
+  while (l > 0 && a.csize[l] == 0) --l;
+  if (k < a.n && a.todo[l] == 0) zsel[(size_t)c * a.n + k] = a.t[(size_t)k * a.M + (m - a.m0)];
+}
+
 template <int NGT>
 static int launch_twist(wtbg_ctx* ctx, const TwistArgs& a, bool clusters) {
   const int cnt = a.m1 - a.m0, smem = TW_ST * (int)sizeof(TwTile<NGT>);
   CK(cudaFuncSetAttribute(k_twist<NGT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   k_twist<NGT><<<(cnt + 31) / 32, 32, smem, ctx->stream>>>(a); WTBG_COUNT(ctx, 1);
   CKL("k_twist");
-  if (clusters) {
+  if (clusters || a.keep) {
     k_cluster<NGT><<<cnt, CL_T, 0, ctx->stream>>>(a); WTBG_COUNT(ctx, 1);
     CKL("k_cluster");
   }
@@ -826,6 +835,13 @@ __global__ void k_gauge_last(double2* X, long long n, int nvec) {
 
 static int tridiagonal_solve_body(wtbg_ctx* ctx, int dtfull, int cpol, bool vectors);
 
+// the recurrences run on T scaled by a power of two to ||T|| <= 1
+static double td_scale(double tnorm) {
+  int ex = 0;
+  if (tnorm > 0.0 && std::isfinite(tnorm)) (void)std::frexp(tnorm, &ex);
+  return std::ldexp(1.0, -std::min(std::max(ex, -1000), 1000));
+}
+
 // Eigenvalues (bisection) and, with vectors, the fused oscillator sums of the tridiagonal
 // form; timed as a whole when profiling.
 int run_tridiagonal_solve(wtbg_ctx* ctx, int dtfull, int cpol, bool vectors) {
@@ -869,10 +885,7 @@ static int tridiagonal_solve_body(wtbg_ctx* ctx, int dtfull, int cpol, bool vect
   lo -= pad;
   hi += pad;
   ENSURE(ctx->lam, (size_t)n * 8);
-  // the recurrences run on T scaled by a power of two to ||T|| <= 1
-  int ex = 0;
-  if (tnorm > 0.0 && std::isfinite(tnorm)) (void)std::frexp(tnorm, &ex);
-  const double sc = std::ldexp(1.0, -std::min(std::max(ex, -1000), 1000));
+  const double sc = td_scale(tnorm);
   const int npad = (int)((n + TD_TILE - 1) / TD_TILE * TD_TILE), ntile = npad / TD_TILE;
   ENSURE(ctx->tmp2, (size_t)npad * 48);
   double2* rcnt = ctx->tmp2.as<double2>();
@@ -957,6 +970,7 @@ static int tridiagonal_solve_body(wtbg_ctx* ctx, int dtfull, int cpol, bool vect
   tw.cpol = cpol;
   // the residual of the joined row is |lambda's error| / |z_r|, and |z_r| >= ||z|| / sqrt(n)
   tw.rtol = 8.0 * DBL_EPSILON * std::sqrt((double)n);
+  tw.keep = false;
   for (long long m0 = 0; m0 < n;) {
     // end the chunk at a cluster start
     long long m1 = std::min(n, m0 + M);
@@ -983,8 +997,8 @@ int run_eigvecs(wtbg_ctx* ctx, int n0, int n1, double2* d_out) {
   const int nvec = n1 - n0 + 1;
   if (nvec > 32) return set_err(ctx, WTBG_ERR_UNSUPPORTED, "eigvecs: at most 32 vectors per launch");
   cudaStream_t s = ctx->stream;
-  // tridiagonal eigenvectors of the requested range, recomputed by inverse iteration over
-  // the whole clusters that contain n0-1 .. n1-1 (0-based)
+  // tridiagonal eigenvectors of the requested range, recomputed over the whole clusters that contain
+  // n0-1 .. n1-1 (0-based)
   {
     const std::vector<int>& cs = ctx->csize_host;
     long long lead = n0 - 1;
@@ -995,16 +1009,44 @@ int run_eigvecs(wtbg_ctx* ctx, int n0, int n1, double2* d_out) {
       while (l2 > 0 && cs[l2] == 0) --l2;
       end = l2 + cs[l2];
     }
-    const long long M = end - lead;
-    ENSURE(ctx->ws, (size_t)4 * 8 * n * M);
+    const long long M = end - lead, tM = (M + 31) / 32 * 32;
+    const int npad = (int)((n + TD_TILE - 1) / TD_TILE * TD_TILE);
+    ENSURE(ctx->ws, (size_t)4 * 8 * n * M + (size_t)npad * tM * 8 + (size_t)npad / 8 * tM * 4);
     ENSURE(ctx->zsel, (size_t)8 * n * nvec);
-    ENSURE(ctx->tmp2, (size_t)8 * 8 * n);
+    ENSURE(ctx->tmp2, (size_t)npad * 48 + (size_t)8 * 8 * n);
+    double2* rec = ctx->tmp2.as<double2>();
+    int* todo = ctx->csz.as<int>() + n;
+    TwistArgs tw;
+    tw.rec = rec + npad;
+    tw.n = (int)n;
+    tw.npad = npad;
+    tw.sc = td_scale(ctx->tnorm);
+    tw.lam = ctx->lam.as<double>();
+    tw.csize = ctx->csz.as<int>();
+    tw.todo = todo;
+    tw.m0 = (int)lead;
+    tw.m1 = (int)end;
+    tw.M = (int)tM;
+    tw.t = ctx->ws.as<double>() + (size_t)4 * n * M;
+    tw.te = reinterpret_cast<int*>(tw.t + (size_t)npad * tM);
+    tw.g = ctx->g.as<double2>();
+    tw.act = reinterpret_cast<double*>(rec + 3 * (size_t)npad);   // not kept
+    tw.dtfull = 0;
+    tw.cpol = 0;
+    tw.rtol = 8.0 * DBL_EPSILON * std::sqrt((double)n);
+    tw.keep = true;
+    k_td_records<<<(npad + 255) / 256, 256, 0, s>>>(ctx->d.as<double>(), ctx->e.as<double>(), (int)n, npad, tw.sc, rec,
+                                                    rec + npad);
+    WTBG_COUNT(ctx, 1);
+    CKL("k_td_records");
+    CK(cudaMemsetAsync(todo, 0, (size_t)n * 4, s));
+    if (int r = ctx->ng == 10 ? launch_twist<10>(ctx, tw, true) : launch_twist<5>(ctx, tw, true)) return r;
     InvArgs a;
     a.d = ctx->d.as<double>();
     a.e = ctx->e.as<double>();
     a.n = n;
     a.lam = ctx->lam.as<double>();
-    a.csize = ctx->csz.as<int>();
+    a.csize = todo;
     a.m0 = lead;
     a.m1 = end;
     a.M = (int)M;
@@ -1012,7 +1054,7 @@ int run_eigvecs(wtbg_ctx* ctx, int n0, int n1, double2* d_out) {
     a.pert = DBL_EPSILON * std::max(ctx->tnorm, DBL_MIN);
     a.g = ctx->g.as<double2>();
     a.ng = ctx->ng;
-    a.act = ctx->tmp2.as<double>();
+    a.act = tw.act;
     a.dtfull = 0;
     a.cpol = 0;
     a.zsel = ctx->zsel.as<double>();
@@ -1020,6 +1062,9 @@ int run_eigvecs(wtbg_ctx* ctx, int n0, int n1, double2* d_out) {
     a.zs1 = n1 - 1;
     k_inviter<<<(int)((M + 63) / 64), 64, 0, s>>>(a); WTBG_COUNT(ctx, 1);
     CKL("k_inviter(eigvecs)");
+    k_take_vectors<<<dim3((unsigned)((n + 255) / 256), nvec), 256, 0, s>>>(tw, n0 - 1, ctx->zsel.as<double>());
+    WTBG_COUNT(ctx, 1);
+    CKL("k_take_vectors");
   }
   const long long cnt = (long long)nvec * n;
   k_real_to_complex<<<(int)((cnt + 255) / 256), 256, 0, s>>>(ctx->zsel.as<double>(), d_out, cnt); WTBG_COUNT(ctx, 1);

@@ -1784,98 +1784,183 @@ __global__ void k_band_to_tridiag(const double2* __restrict__ AB, long long N, d
   if (j < N - 1) e[j] = AB[j * LDB + 1].x;
 }
 
-// ----------------------------------------------------------------------------- back-transform
-// Stage-2 reflectors in reverse: sweeps from the last, each step after the next sweep has
-// finished its steps up to t (the ranges are then disjoint); X (n x nvec, column-major).
-__global__ void __launch_bounds__(32 * BG_WARPS, 1) k_bulge_back(const double2* __restrict__ A, long long N,
-                                                                  const double2* __restrict__ tau2, double2* X, int nvec,
-                                                                  unsigned int* prog, int* err) {
+// Exciton vectors through stage 2: X <- Q2 X.  The reflectors of sweep s act on rows s + 1 + 32 t ..; a warp
+// takes one vector through the 32 sweeps s0 .. s0 + 31 of a group, last sweep first, block t by block t: its 63
+// rows are two numbers a lane (rows l and l + 32 of the window), of which sweep s0 + p uses the first where
+// l >= p and the second where not, so nothing moves between the lanes.  Block t needs block t of the group
+// behind (s0 + 32), whose rows start 32 further on.  One chain of dot products a block: N / 32 groups and as many
+// blocks one after the other instead of N sweeps with a flag each: 8 vectors of N = 2916 14.6 -> 1.7 ms.
+constexpr int BB_WARPS = 8;
+__global__ void __launch_bounds__(32 * BB_WARPS, 2) k_bulge_back(const double2* __restrict__ A, long long N,
+                                                                const double2* __restrict__ tau2, double2* X, int nvec,
+                                                                unsigned int* prog, int* err) {
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long W = (long long)gridDim.x * BG_WARPS;
-  for (long long u = (long long)blockIdx.x * BG_WARPS + wid; u < N - 1; u += W) {
-    const long long s = N - 2 - u;
-    const long long ns = nsteps_of(N, s);
-    const long long nnext = (s + 1 < N - 1) ? nsteps_of(N, s + 1) : 0;
-    for (long long t = 0; t < ns; ++t) {
-      if (s + 1 < N - 1) {
-        const unsigned int need = (unsigned int)min(t + 1, nnext);
+  const long long ng = (N - 1 + BW - 1) / BW;
+  const int nch = (nvec + BB_WARPS - 1) / BB_WARPS;
+  for (long long u = blockIdx.x; u < ng * nch; u += gridDim.x) {   // later sweeps first: no task waits for a later one
+    const long long g = ng - 1 - u / nch, s0 = g * BW;
+    const int c = (int)(u % nch) * BB_WARPS + wid;
+    if (c >= nvec) continue;
+    const int np = (int)min((long long)BW, N - 1 - s0);   // sweeps of the group
+    const long long nblk = nsteps_of(N, s0), nnext = (g + 1 < ng) ? nsteps_of(N, s0 + BW) : 0;
+    unsigned int* mine = prog + g * 32 + c;
+    const long long toff = lane < np ? tau2_offset(N, s0 + lane) : 0;
+    const int tn = lane < np ? (int)nsteps_of(N, s0 + lane) : 0;
+    double2* xc = X + (long long)c * N + s0 + 1 + lane;
+    auto row_ok = [&](long long r) { return s0 + 1 + r + lane < N; };
+    double2 x0 = row_ok(0) ? __ldcg(xc) : make_double2(0, 0);
+    for (long long t = 0; t < nblk; ++t) {
+      const double2 tau = t < tn ? tau2[toff + t] : make_double2(0, 0);
+      // v of sweep s0 + p in the window: element (lane - p) mod 32 of the stored reflector
+      auto ldv = [&](int p) {
+        const int i = (lane - p) & 31;
+        return (p < np && s0 + p + 1 + t * BW + i < N) ? A[t * BW + i + (N - 1 - s0 - p) * N] : make_double2(0, 0);
+      };
+      double2 v[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v[q] = ldv(31 - q);
+      const long long need = min(t + 1, nnext);
+      if (need > 0) {
         int bad = 0;
-        if (lane == 0) bad = wait_at_least(prog + s + 1, need, err) ? 0 : 1;
-        bad = __shfl_sync(0xffffffffu, bad, 0);
-        if (bad) return;
+        if (lane == 0) bad = wait_at_least(prog + (g + 1) * 32 + c, (unsigned int)need, err) ? 0 : 1;
+        if (__shfl_sync(0xffffffffu, bad, 0)) return;
       }
-      const long long r0 = s + 1 + t * BW;
-      const int L = (int)min((long long)BW, N - r0);
-      const double2 v = (lane < L) ? A[(r0 + lane - s - 1) + (N - 1 - s) * N] : make_double2(0, 0);
-      const double2 tau = tau2[tau2_offset(N, s) + t];
-      for (int c = 0; c < nvec; ++c) {
-        double2* xp = X + (long long)c * N + r0;
-        const double2 xv = (lane < L) ? __ldcg(xp + lane) : make_double2(0, 0);
-        const double2 sv = warp_sum2(cmulc(v, xv));   // v^H x
-        if (lane < L) xp[lane] = csub(xv, cmul(tau, cmul(v, sv)));
+      double2 x1 = row_ok((t + 1) * BW) ? __ldcg(xc + (t + 1) * BW) : make_double2(0, 0);
+#pragma unroll 1
+      for (int p8 = 31; p8 > 0; p8 -= 8) {
+        double2 vn[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) vn[q] = p8 >= 8 ? ldv(p8 - 8 - q) : make_double2(0, 0);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const int p = p8 - q;
+          const bool lo = lane >= p;
+          const double2 xs = lo ? x0 : x1;
+          const double2 sv = warp_sum2(cmulc(v[q], xs));   // v^H x
+          const double2 tv = cmul(shfl2(tau, p), v[q]);
+          const double2 xn = csub(xs, cmul(tv, sv));
+          if (lo) x0 = xn;
+          else x1 = xn;
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = vn[q];
       }
+      if (row_ok(t * BW)) xc[t * BW] = x0;
+      if (t + 1 == nblk && row_ok((t + 1) * BW)) xc[(t + 1) * BW] = x1;
+      x0 = x1;
       __syncwarp();
-      if (lane == 0) st_release(prog + s, (unsigned int)(t + 1));
+      if (lane == 0) st_release(mine, (unsigned int)(t + 1));
     }
   }
 }
 
-// Stage-1 block reflectors in reverse: X[k0:] -= V (T (V^H X[k0:])).  V from the panel's
-// columns of A (unit at row k0+q, v below, zero above).
-constexpr int BT1_RB = 128;
+// ... and through stage 1: X <- Q1 X, the panels' block reflectors in reverse, X[k0:] -= V (T (V^H X[k0:])), all in
+// one cooperative launch.  V from the panel's columns of A (unit at row k0+q, v below, zero above).  CTA b owns
+// the 32-row tiles b, b + G, ... counted from the end of the matrix; per panel its share of V^H X, a grid
+// barrier, the sum and the product with T (one CTA a vector, fixed order), a barrier, and its rows.  8 vectors of
+// N = 2916 (91 panels): 6.5 -> 1.3 ms (three launches a panel, V read across its columns).
+constexpr int BT_LD = 33;
+constexpr size_t BT1_SMEM = (size_t)(32 * BT_LD + 2 * 32 * 32 + 32 * 32) * sizeof(double2);
 __device__ __forceinline__ double2 panel_v(const double2* A, long long N, int j0, int k0, int q, long long r) {
   const long long rq = (long long)k0 + q;
   if (r < rq) return make_double2(0, 0);
   if (r == rq) return make_double2(1.0, 0.0);
   return A[r + (long long)(j0 + q) * N];
 }
-__global__ void __launch_bounds__(256) k_bt1_partial(const double2* __restrict__ A, long long N, int j0, int k0, int nref,
-                                                     const double2* __restrict__ X, int nvec, double2* __restrict__ part) {
-  // part[b][q + 32 c] = sum over this block's rows of conj(V[r][q]) X[r][c]
-  const long long rb = (long long)k0 + (long long)blockIdx.x * BT1_RB;
-  for (int e = threadIdx.x; e < 32 * nvec; e += 256) {
-    const int q = e & 31, c = e >> 5;
-    double2 t = make_double2(0, 0);
-    if (q < nref)
-      for (int i = 0; i < BT1_RB; ++i) {
-        const long long r = rb + i;
-        if (r >= N) break;
-        t = cadd(t, cmulc(panel_v(A, N, j0, k0, q, r), X[r + (long long)c * N]));
+__global__ void __launch_bounds__(256, 1) k_bt1(const double2* __restrict__ A, long long N, const double2* __restrict__ Tbuf,
+                                                double2* X, int nvec, double2* part, double2* Y, unsigned int* cnt,
+                                                int* err) {
+  extern __shared__ __align__(16) double2 bsm[];
+  double2* sV = bsm;                    // [q][row]
+  double2* sX = sV + 32 * BT_LD;        // [row][c]
+  double2* sY = sX + 32 * 32;           // [q][c]
+  double2* sP = sY + 32 * 32;
+  const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5, G = gridDim.x, b = blockIdx.x;
+  const int npan = (int)((N - BW - 1 + BW - 1) / BW);
+  unsigned int target = 0;
+  for (int pnl = npan - 1; pnl >= 0; --pnl) {
+    const int j0 = pnl * BW, k0 = j0 + BW;
+    const int nref = (int)min((long long)BW, N - k0);
+    const int ntile = (int)((N - k0 + 31) / 32), na = min(ntile, G);   // CTAs with rows
+    const double2* T = Tbuf + (size_t)pnl * 1024;
+    auto load = [&](int t) {   // tile t: rows N - 32 (t + 1) .. + 31, those from k0 on
+      const long long r0 = N - 32LL * (t + 1);
+      __syncthreads();
+      for (int e = tid; e < 1024; e += 256) {
+        const int i = e & 31, q = e >> 5;
+        const long long r = r0 + i;
+        sV[q * BT_LD + i] = (r >= k0 && q < nref) ? panel_v(A, N, j0, k0, q, r) : make_double2(0, 0);
+        if (q < nvec) sX[i * 32 + (q ^ i)] = r >= k0 ? __ldcg(X + r + (long long)q * N) : make_double2(0, 0);
       }
-    part[(size_t)blockIdx.x * 32 * 32 + e] = t;
-  }
-}
-__global__ void __launch_bounds__(1024) k_bt1_tmat(const double2* __restrict__ part, int nb, int nvec,
-                                                   const double2* __restrict__ T, double2* __restrict__ Y) {
-  __shared__ double2 sY[32 * 32];
-  const int e = threadIdx.x;
-  const int q = e & 31, c = e >> 5;
-  double2 t = make_double2(0, 0);
-  if (c < nvec)
-    for (int b = 0; b < nb; ++b) t = cadd(t, part[(size_t)b * 32 * 32 + e]);
-  sY[e] = t;
-  __syncthreads();
-  if (c < nvec) {   // (T Y)[q][c] = sum_{l >= q} T[q][l] Y[l][c]
-    double2 s = make_double2(0, 0);
-    for (int l = q; l < 32; ++l) s = cadd(s, cmul(T[q + 32 * l], sY[l + 32 * c]));
-    Y[e] = s;
-  }
-}
-__global__ void __launch_bounds__(256) k_bt1_apply(const double2* __restrict__ A, long long N, int j0, int k0, int nref,
-                                                   double2* X, int nvec, const double2* __restrict__ Y) {
-  __shared__ double2 sY[32 * 32];
-  for (int e = threadIdx.x; e < 32 * nvec; e += 256) sY[e] = Y[e];
-  __syncthreads();
-  const long long r = (long long)k0 + (long long)blockIdx.x * 256 + threadIdx.x;
-  if (r >= N) return;
-  double2 vq[32];
+      __syncthreads();
+    };
+    // share of V^H X: thread (q = lane, vectors wp + 8 u)
+    double2 acc[4];
 #pragma unroll
-  for (int q = 0; q < 32; ++q) vq[q] = (q < nref) ? panel_v(A, N, j0, k0, q, r) : make_double2(0, 0);
-  for (int c = 0; c < nvec; ++c) {
-    double2 t = make_double2(0, 0);
+    for (int u = 0; u < 4; ++u) acc[u] = make_double2(0, 0);
+    for (int t = b; t < ntile; t += G) {
+      load(t);
+      for (int i = 0; i < 32; ++i) {
+        const double2 v = sV[lane * BT_LD + i];
 #pragma unroll
-    for (int q = 0; q < 32; ++q) t = cadd(t, cmul(vq[q], sY[q + 32 * c]));
-    X[r + (long long)c * N] = csub(X[r + (long long)c * N], t);
+        for (int u = 0; u < 4; ++u)
+          if (wp + 8 * u < nvec) acc[u] = cfmac(v, sX[i * 32 + ((wp + 8 * u) ^ i)], acc[u]);
+      }
+    }
+    if (b < na) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (wp + 8 * u < nvec) part[((size_t)(wp + 8 * u) * G + b) * 32 + lane] = acc[u];
+    }
+    if (!grid_sync(cnt, target += G, err)) return;
+    // Y[:, c] = T sum of the shares
+    for (int c = b; c < nvec; c += G) {
+      double2 t = make_double2(0, 0);
+      const double2* p = part + (size_t)c * G * 32 + lane;
+      for (int i0 = wp; i0 < na; i0 += 64) {
+        double2 pv[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) pv[u] = i0 + 8 * u < na ? ldcg2(p + (size_t)(i0 + 8 * u) * 32) : make_double2(0, 0);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) t = cadd(t, pv[u]);
+      }
+      sP[tid] = t;
+      __syncthreads();
+      if (wp == 0) {
+#pragma unroll
+        for (int u = 1; u < 8; ++u) t = cadd(t, sP[u * 32 + lane]);
+        double2 y = make_double2(0, 0);   // (T P)[q] = sum_{l >= q} T[q][l] P[l]
+        for (int l = 0; l < 32; ++l) {
+          const double2 pl = shfl2(t, l);
+          if (l >= lane) y = cfma(T[lane + 32 * l], pl, y);
+        }
+        Y[c * 32 + lane] = y;
+      }
+      __syncthreads();
+    }
+    if (!grid_sync(cnt, target += G, err)) return;
+    if (b < na) {
+      for (int e = tid; e < 32 * nvec; e += 256) sY[(e & 31) * 32 + (e >> 5)] = ldcg2(Y + e);
+      for (int t = b; t < ntile; t += G) {
+        if (t != b || ntile > G) load(t);   // else the tile is still here
+        else __syncthreads();
+        const long long r = N - 32LL * (t + 1) + lane;
+        double2 x[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) x[u] = make_double2(0, 0);
+        for (int q = 0; q < 32; ++q) {
+          const double2 v = sV[q * BT_LD + lane];
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (wp + 8 * u < nvec) x[u] = cfma(v, sY[q * 32 + wp + 8 * u], x[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int c = wp + 8 * u;
+          if (c < nvec && r >= k0) X[r + (long long)c * N] = csub(sX[lane * 32 + (c ^ lane)], x[u]);
+        }
+      }
+    }
   }
 }
 
@@ -1921,7 +2006,7 @@ static int two_stage_buffers(wtbg_ctx* ctx, int nband) {
   ENSURE(ctx->t2P, (size_t)nsm * (16 + 2 * 16 * BW + 16 * BW * BW + 16 * BW * NGMAX) + 4096 +
                         (size_t)std::max<long long>(npan, 1) * 8);
   ENSURE(ctx->t2AB, (size_t)nband * (N + AB_PAD) * LDB * 16);
-  ENSURE(ctx->t2prog, (size_t)nband * N * 4 + 64);
+  ENSURE(ctx->t2prog, (size_t)nband * N * 4 + 512);
   ENSURE(ctx->triErr, 16);
   return 0;
 }
@@ -2317,32 +2402,32 @@ int run_backtransform2(wtbg_ctx* ctx, double2* X, int nvec) {
   const int nsm = ctx->nsm > 0 ? ctx->nsm : 148;
   unsigned int* prog = ctx->t2prog.as<unsigned int>();
   int* err = ctx->triErr.as<int>();
-  CK(cudaMemsetAsync(prog, 0, (size_t)N * 4, s));
+  const long long ng = (N - 1 + BW - 1) / BW;
+  CK(cudaMemsetAsync(prog, 0, (size_t)(ng + 1) * 32 * 4, s));   // and the barrier counter of k_bt1
   CK(cudaMemsetAsync(err, 0, 4, s));
-  const long long nsweep = N - 1;
-  const int gb = (int)std::max<long long>(1, std::min<long long>(nsm, (nsweep + BG_WARPS - 1) / BG_WARPS));
+  const double2* A = ctx->H.as<double2>();
+  long long NN = N;
   {
-    const double2* A = ctx->H.as<double2>();
+    int per = 1;
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_bulge_back, 32 * BB_WARPS, 0));
+    const long long tasks = ng * ((nvec + BB_WARPS - 1) / BB_WARPS);
+    const int gb = (int)std::max<long long>(1, std::min<long long>((long long)nsm * std::max(per, 1), tasks));
     const double2* tau2 = ctx->tau.as<double2>();
-    long long NN = N;
     void* args[] = {(void*)&A, (void*)&NN, (void*)&tau2, (void*)&X, (void*)&nvec, (void*)&prog, (void*)&err};
-    CK(cudaLaunchCooperativeKernel((const void*)k_bulge_back, dim3(gb), dim3(32 * BG_WARPS), args, 0, s));
+    CK(cudaLaunchCooperativeKernel((const void*)k_bulge_back, dim3(gb), dim3(32 * BB_WARPS), args, 0, s));
   }
-  const long long npan = (N - BW - 1 + BW - 1) / BW;
-  const int nbmax = (int)((N + BT1_RB - 1) / BT1_RB);
-  ENSURE(ctx->t2G, (size_t)nbmax * 1024 * 16 + 1024 * 16);
-  double2* part = ctx->t2G.as<double2>();
-  double2* Y = part + (size_t)nbmax * 1024;
-  for (long long pnl = npan - 1; pnl >= 0; --pnl) {
-    const int j0 = (int)(pnl * BW), k0 = j0 + BW;
-    const long long m = N - k0;
-    const int nref = (int)std::min<long long>(BW, m);
-    const int nb = (int)((m + BT1_RB - 1) / BT1_RB);
-    k_bt1_partial<<<nb, 256, 0, s>>>(ctx->H.as<double2>(), N, j0, k0, nref, X, nvec, part);
-    k_bt1_tmat<<<1, 1024, 0, s>>>(part, nb, nvec, ctx->t2T.as<double2>() + (size_t)pnl * 1024, Y);
-    k_bt1_apply<<<(int)((m + 255) / 256), 256, 0, s>>>(ctx->H.as<double2>(), N, j0, k0, nref, X, nvec, Y);
+  {
+    const int gt = (int)std::max<long long>(1, std::min<long long>(nsm, (N - BW + 31) / 32));
+    ENSURE(ctx->t2G, (size_t)(gt + 1) * 1024 * 16);
+    double2* Y = ctx->t2G.as<double2>();
+    double2* part = Y + 1024;
+    const double2* T = ctx->t2T.as<double2>();
+    unsigned int* cnt = prog + ng * 32;
+    CK(cudaFuncSetAttribute(k_bt1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BT1_SMEM));
+    void* args[] = {(void*)&A, (void*)&NN, (void*)&T, (void*)&X, (void*)&nvec, (void*)&part, (void*)&Y, (void*)&cnt, (void*)&err};
+    CK(cudaLaunchCooperativeKernel((const void*)k_bt1, dim3(gt), dim3(256), args, BT1_SMEM, s));
   }
-  WTBG_COUNT(ctx, 1 + 3 * npan);
+  WTBG_COUNT(ctx, 2);
   CKL("two-stage back-transform");
   int herr = 0;
   CK(cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, s));
