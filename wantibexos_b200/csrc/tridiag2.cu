@@ -457,7 +457,7 @@ constexpr int PC_COLS = BW + NGMAX;
 constexpr int PC_MAXC = 16;
 constexpr int PC_MAX_NR = 24;
 constexpr size_t pc_smem(int nr) {
-  return sizeof(double2) * (size_t)(2 * PC_MAXC * PC_COLS + 2 * BW * BW + BW * BW / 4 + 2 * BW * NGMAX + BW * (8 * nr + 1));
+  return sizeof(double2) * (size_t)(2 * PC_MAXC * PC_COLS + 2 * BW * BW + 2 * BW * NGMAX + BW * (8 * nr + 1));
 }
 
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -465,11 +465,37 @@ __device__ __forceinline__ uint32_t cluster_rank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
-// one 16-byte store into the same shared-memory place of CTA `cta` of the cluster
-__device__ __forceinline__ void st_cluster(double2* p, uint32_t cta, double2 v) {
-  uint32_t a;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(tc::smem_u32(p)), "r"(cta));
-  asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(a), "d"(v.x), "d"(v.y) : "memory");
+// shared::cluster address in CTA `cta` of the cluster of what lies at p here
+__device__ __forceinline__ uint32_t cluster_map(const void* p, uint32_t cta) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(cta));
+  return r;
+}
+// 16 bytes into another CTA's shared memory, counted by its mbarrier
+__device__ __forceinline__ void st_async16(uint32_t addr, uint32_t mbar, double2 v) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];" ::"r"(addr),
+               "d"(v.x), "d"(v.y), "r"(mbar)
+               : "memory");
+}
+// arrive for a phase of the own mbarrier that `bytes` will come to
+__device__ __forceinline__ void mbar_expect(uint32_t mbar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mbar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t mbar, uint32_t parity) {
+  unsigned long long t0 = 0;
+  for (unsigned int spins = 1;; ++spins) {
+    uint32_t ok;
+    asm volatile(
+        "{ .reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p; }"
+        : "=r"(ok)
+        : "r"(mbar), "r"(parity)
+        : "memory");
+    if (ok) return true;
+    if ((spins & 63u) == 0u) {
+      if (t0 == 0) t0 = globaltimer();
+      if (globaltimer() - t0 > kWaitNs) return false;
+    }
+  }
 }
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -483,14 +509,14 @@ __global__ void __launch_bounds__(PC_THREADS, 1) k_panel_qr_cl(PanelArgs a, int 
   double2(*s_part)[PC_MAXC][PC_COLS] = reinterpret_cast<double2(*)[PC_MAXC][PC_COLS]>(psm);   // dot products, by parity of p
   double2* s_G = psm + 2 * PC_MAXC * PC_COLS;
   double2* s_T = s_G + BW * BW;
-  double2* s_w = s_T + BW * BW;
-  double2* s_y = s_w + BW * BW / 4;
+  double2* s_y = s_T + BW * BW;
   double2* s_z = s_y + BW * NGMAX;
   double2* Vs = s_z + BW * NGMAX;                      // [32][VS]: V of the own rows, at the end
   __shared__ double2 s_x[2][R];                        // pivot column by parity of p
   __shared__ double2 s_al[2][PC_COLS];                 // row p
   __shared__ double2 s_tau[BW];
   __shared__ double2 s_sc[2][3];                       // kappa; (beta, 0); 1/u_p
+  __shared__ __align__(8) unsigned long long s_bar[2]; // arrivals for column p, by parity of p
   const int tid = threadIdx.x, lane = tid & 31, sl = tid & 7, q = tid >> 3;
   const int c = (int)cluster_rank();
   const long long N = a.N;
@@ -518,11 +544,44 @@ __global__ void __launch_bounds__(PC_THREADS, 1) k_panel_qr_cl(PanelArgs a, int 
     for (int o = 4; o > 0; o >>= 1) v = cadd(v, shfl2_xor(v, o));
     return v;
   };
+  // T(0:p, p) = -tau_p T(0:p, 0:p) G(0:p, p), lane = row
+  auto t_column = [&](int p) {
+    const double2 tau = s_tau[p];
+    double2 t0 = make_double2(0, 0), t1 = t0;
+    int l = 0;
+    for (; l + 1 < p; l += 2) {   // T is zero below its diagonal
+      t0 = cfma(s_T[lane + l * BW], s_G[l + p * BW], t0);
+      t1 = cfma(s_T[lane + (l + 1) * BW], s_G[l + 1 + p * BW], t1);
+    }
+    if (l < p) t0 = cfma(s_T[lane + l * BW], s_G[l + p * BW], t0);
+    const double2 t = cmul(tau, cadd(t0, t1));
+    if (lane <= p) s_T[lane + p * BW] = lane == p ? tau : make_double2(-t.x, -t.y);
+    __syncwarp();
+  };
   for (int e = tid; e < BW * BW; e += PC_THREADS) s_G[e] = s_T[e] = make_double2(0, 0);
   for (int e = tid; e < BW * NGMAX; e += PC_THREADS) s_y[e] = make_double2(0, 0);
   if (tid < BW) s_tau[tid] = make_double2(0, 0);
   if (q == 0) post(0);
-  cluster_sync();   // every CTA of the cluster runs (its shared memory is written below)
+  const uint32_t bar = (uint32_t)__cvta_generic_to_shared(s_bar);
+  const int nq = BW + ng;                                   // columns that are exchanged
+  const uint32_t bytes = (uint32_t)((C + 1) * nq * 16);     // their sums from every CTA, and row p from CTA 0
+  if (tid == 0) {
+    for (int b = 0; b < 2; ++b) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar + 8 * b) : "memory");
+      mbar_expect(bar + 8 * b, bytes);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  cluster_sync();   // every CTA of the cluster runs and has its mbarriers (both are written below)
+  uint32_t rpart[2], ral[2], rbar[2];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const uint32_t cta = (uint32_t)min(sl + 8 * k, C - 1);
+    rpart[k] = cluster_map(&s_part[0][c][min(q, PC_COLS - 1)], cta);
+    ral[k] = cluster_map(&s_al[0][min(q, PC_COLS - 1)], cta);
+    rbar[k] = cluster_map(s_bar, cta);
+  }
+  bool late = false;
   for (int p = 0; p < nref; ++p) {
     const int buf = p & 1;
     double2* xs = s_x[buf];
@@ -534,22 +593,30 @@ __global__ void __launch_bounds__(PC_THREADS, 1) k_panel_qr_cl(PanelArgs a, int 
         if (u + 1 < NR) s1 = cfmac(xs[8 * u + 8 + sl], P[u + 1], s1);
       }
       const double2 S = sum8(cadd(s0, s1));
-      if (q < PC_COLS) {
-        if (sl < C) st_cluster(&s_part[buf][c][q], sl, S);
-        if (sl + 8 < C) st_cluster(&s_part[buf][c][q], sl + 8, S);
+      const uint32_t po = buf * (uint32_t)sizeof(s_part[0]), ao = buf * (uint32_t)sizeof(s_al[0]);
+      if (q < nq) {
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+          if (sl + 8 * k < C) st_async16(rpart[k] + po, rbar[k] + 8 * buf, S);
       }
       if (c == 0) {   // row p of every column, held by the thread sl = p mod 8 at u = p / 8 (rows < 32: u < 4)
         const double2 v = (p >> 3) == 0 ? P[0] : ((p >> 3) == 1 ? P[1] : ((p >> 3) == 2 ? P[2] : P[3]));
         const double2 r = shfl2(v, (lane & 24) | (p & 7));
-        if (q < PC_COLS) {
-          if (sl < C) st_cluster(&s_al[buf][q], sl, r);
-          if (sl + 8 < C) st_cluster(&s_al[buf][q], sl + 8, r);
+        if (q < nq) {
+#pragma unroll
+          for (int k = 0; k < 2; ++k)
+            if (sl + 8 * k < C) st_async16(ral[k] + ao, rbar[k] + 8 * buf, r);
         }
       }
     }
-    cluster_sync();
+    if ((tid >> 5) == PC_THREADS / 32 - 1) {   // the last warp holds no column: it forms T column by column
+      if (p > 0) t_column(p - 1);
+    } else if (!late) {
+      late = !mbar_wait_cluster(bar + 8 * buf, (p >> 1) & 1);
+    }
+    if (tid == 0) mbar_expect(bar + 8 * buf, bytes);   // for column p + 2
     double2 S = make_double2(0, 0);
-    if (q < PC_COLS) {
+    if (q < nq) {
       if (sl < C) S = s_part[buf][sl][q];
       if (sl + 8 < C) S = cadd(S, s_part[buf][sl + 8][q]);
     }
@@ -574,7 +641,7 @@ __global__ void __launch_bounds__(PC_THREADS, 1) k_panel_qr_cl(PanelArgs a, int 
     const double beta = s_sc[buf][1].x;
     // w_q = S_q + conj(u_p) P_pq
     const double2 al = s_al[buf][p];
-    const double2 w = q < PC_COLS ? cfmac(make_double2(al.x - beta, al.y), s_al[buf][q], S) : S;
+    const double2 w = q < nq ? cfmac(make_double2(al.x - beta, al.y), s_al[buf][q], S) : S;
     if (panel && q > p) {
       const double2 cw = cmulc(kap, w);
 #pragma unroll
@@ -594,6 +661,10 @@ __global__ void __launch_bounds__(PC_THREADS, 1) k_panel_qr_cl(PanelArgs a, int 
     }
     __syncthreads();
   }
+  if (late) atomicExch(a.err, 1);
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // waited for at the end
+  if ((tid >> 5) == PC_THREADS / 32 - 1) t_column(nref - 1);
   // write back: A keeps R (rows <= k0+q) and v below; Vp and Vs get V with its unit and zeros
   if (panel) {
 #pragma unroll
@@ -609,33 +680,10 @@ __global__ void __launch_bounds__(PC_THREADS, 1) k_panel_qr_cl(PanelArgs a, int 
       }
     }
   }
-  // T factor: T_ii = tau_i, and for neighbouring diagonal blocks of size h, T_12 = -T_11 (G_12 T_22)
-  if (tid < BW) s_T[tid + tid * BW] = s_tau[tid];
   __syncthreads();
-  for (int h = 1; h < BW; h *= 2) {
-    const int cnt = BW / (2 * h) * h * h;   // entries of all pairs' T_12
-    int b = 0, i = 0, j = 0;
-    if (tid < cnt) {
-      b = tid / (h * h) * 2 * h;
-      i = tid % h;
-      j = (tid / h) % h;
-      double2 t = make_double2(0, 0);
-      for (int l = 0; l <= j; ++l) t = cfma(s_G[(b + i) + (b + h + l) * BW], s_T[(b + h + l) + (b + h + j) * BW], t);
-      s_w[tid] = t;
-    }
-    __syncthreads();
-    if (tid < cnt) {
-      double2 t = make_double2(0, 0);
-      const double2* wj = s_w + tid - i;   // column j of the pair's product
-      for (int l = i; l < h; ++l) t = cfms(s_T[(b + i) + (b + l) * BW], wj[l], t);
-      s_T[(b + i) + (b + h + j) * BW] = t;
-    }
-    __syncthreads();
-  }
   if (c == 0)
     for (int e = tid; e < BW * BW; e += PC_THREADS) a.Tout[e] = s_T[e];
   // g <- g - conj(V) T^T (V^T g)
-  if (ng == 0) return;
   for (int e = tid; e < BW * ng; e += PC_THREADS) {
     const int j = e % BW, al = e / BW;
     double2 t = make_double2(0, 0);
@@ -654,6 +702,9 @@ __global__ void __launch_bounds__(PC_THREADS, 1) k_panel_qr_cl(PanelArgs a, int 
     double2* gp = a.g + (long long)al * N + rbeg + i;
     *gp = csub(*gp, cadd(t0, t1));
   }
+  // no CTA leaves while another may still write to it (after a wait that ran out)
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 
@@ -2143,6 +2194,7 @@ static int run_stage1(wtbg_ctx* ctx, int ng, int band) {
     pa.Tout = Tbuf + (size_t)pnl * 1024;
     pa.g = g;
     pa.ng = ng;
+    pa.err = err;
     mark(pnl, 0);
     if (m <= ctx->panel_cl_rows) {
       if (int r = launch_panel_cluster(ctx, pa)) return r;
@@ -2158,7 +2210,6 @@ static int run_stage1(wtbg_ctx* ctx, int ng, int band) {
       pa.partVg = partVg;
       pa.alpha = alpha;
       pa.cnt = cnt + pnl;
-      pa.err = err;
       const size_t psm = std::max((size_t)BW * (R | 1) * 16, ALONE_SMEM);
       CK(cudaFuncSetAttribute(k_panel_qr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm));
       if (G > PQ_MAXG) return set_err(ctx, WTBG_ERR_UNSUPPORTED, "panel QR: more CTAs than the column reduction holds");
