@@ -188,6 +188,19 @@ __device__ __forceinline__ double fast_rcp(double x) {
   return fma(r, fma(g, g, g), r);
 }
 
+// a, b scaled by the power of two that brings the larger to [1, 2); returns the exponent taken out
+__device__ __forceinline__ int pow2_rescale(double& a, double& b) {
+  const int h = max(__double2hiint(a) & 0x7ff00000, __double2hiint(b) & 0x7ff00000);
+  const double f = __hiloint2double(0x7fe00000 - h, 0);
+  a *= f;
+  b *= f;
+  return (h >> 20) - 1023;
+}
+// 2^x, 0 below 2^-1022, at most 2^1000
+__device__ __forceinline__ double pow2_clamped(int x) {
+  return __hiloint2double((min(max(x, -1023), 1000) + 1023) << 20, 0);
+}
+
 // ---- kernel launchers (implemented in the .cu files)
 int launch_bands(wtbg_ctx* ctx, bool q_mesh);
 int launch_velocity(wtbg_ctx* ctx, double eta_f32);

@@ -11,8 +11,10 @@
 // bse_subs.f90:336-378, no conjugate on the eigenvector).
 #include <algorithm>
 #include <cfloat>
+#include <climits>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include <cub/cub.cuh>
@@ -444,48 +446,55 @@ __global__ void __launch_bounds__(512) k_chol_inv(const double2* G, int q, doubl
 
 // One-CTA Hermitian eigensolver for the Rayleigh-Ritz matrix (n <= kMaxRR, nb wanted pairs):
 //  1. Householder reduction to real tridiagonal form in shared memory (lower reflectors as in
-//     ZHETRD: H = I - tau v v^H, v(1) = 1, beta real), the A22 v product with four threads a row;
+//     ZHETRD: H = I - tau v v^H, v(1) = 1, beta real): three barriers a column, every warp forming the
+//     norm, the scalars and p^H v for itself, the A22 v product with four threads a row;
 //  2. multisection Sturm bisection: blockDim/nb threads per wanted eigenvalue each evaluate one
 //     point of the current interval, shrinking it (G+1)-fold per round, a fixed number of rounds
 //     down to ~eps |T|;
-//  3. inverse iteration with partial pivoting (3 steps) for the eigenvectors of T, eigenvalues
-//     closer than 1e-7 |T| handled in order by one thread with Gram-Schmidt;
-//  4. back-transform y = H_0 H_1 ... H_{n-2} z, one warp per vector in shared memory.
+//  3. eigenvectors of T, a thread each: the recurrence from the top and from the bottom joined where
+//     their product is largest, twice, the second time at the Rayleigh quotient of the first; where
+//     the residual of the joined row says no, and for eigenvalues closer than 1e-7 |T| (in order by one
+//     thread with Gram-Schmidt), inverse iteration with partial pivoting (3 steps);
+//  4. back-transform y = H_0 H_1 ... H_{n-2} z, up to three vectors a warp in registers.
+// One chain of latencies, in it 64 % the reduction at n = 80: 40 vectors of n = 80 0.37 ms, of n = 56 0.16; over a
+// solve of N = 14400 (61 of them) 31.7 -> 19.8 ms.
 constexpr int RR_THREADS = 512;
 
+// leading dimension = 2 mod 8: the product's 2 rows x 4 columns of a quarter-warp fall on distinct banks
+__host__ __device__ constexpr int rr_ld(int n) { return n + (10 - n % 8) % 8; }
 __host__ __device__ constexpr size_t rr_smem_bytes(int n, int nb) {
-  return (size_t)16 * ((size_t)n * n + 3 * n + (size_t)n * nb) + (size_t)8 * (2 * n + 3 * kMaxRR + (size_t)n * nb) +
-         (size_t)4 * RR_THREADS + 64;
+  return (size_t)16 * ((size_t)n * rr_ld(n) + 3 * n) +
+         (size_t)8 * (5 * (n + 8) + 3 * kMaxRR + (size_t)n * (nb + 1)) + (size_t)4 * (RR_THREADS + 10 * (nb + 1)) + 64;
 }
 
 // Number of eigenvalues of the symmetric tridiagonal (d, e) below x from the sign changes of
-// the leading principal minors p_i = (d_i - x) p_{i-1} - e_{i-1}^2 p_{i-2} (two FMAs a step,
-// no division), rescaled by exact powers of two; a zero minor counts as a sign change.
-__device__ __forceinline__ int sturm_count(const double* dd, const double* ee, int n, double x) {
-  double pm = 0.0, p = 1.0, sgn = 1.0;
+// the leading principal minors p_i = (d_i - x) p_{i-1} - e_{i-1}^2 p_{i-2} (e2[i] = e_{i-1}^2, held above
+// 2^-160 |T|^2 so that no two minors in a row vanish), scaled by a power of two every eight steps;
+// d and e2 are padded to a multiple of eight by rows that change no sign.
+__device__ __forceinline__ int sturm_count(const double* dd, const double* e2, int n, double x) {
+  double pm = 0.0, p = 1.0;
   int cnt = 0;
-  for (int i = 0; i < n; ++i) {
-    const double e2 = (i > 0) ? ee[i - 1] * ee[i - 1] : 0.0;
-    const double pn = fma(dd[i] - x, p, -e2 * pm);
-    pm = p;
-    p = pn;
-    const double ap = fabs(p);
-    if (ap > 0x1p+500) {
-      p *= 0x1p-500;
-      pm *= 0x1p-500;
-    } else if (ap < 0x1p-500 && ap > 0.0) {
-      p *= 0x1p+500;
-      pm *= 0x1p+500;
+  for (int i0 = 0; i0 < n; i0 += 8) {
+    double d[8], e[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      d[q] = dd[i0 + q];
+      e[q] = e2[i0 + q];
     }
-    const double s = (p == 0.0) ? -sgn : (p < 0.0 ? -1.0 : 1.0);
-    cnt += (s != sgn);
-    sgn = s;
-    if (p == 0.0) p = sgn * (fabs(pm) * 0x1p-60 + 0x1p-1000);   // a zero minor: pivot -> sign change
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const double pn = fma(d[q] - x, p, -e[q] * pm);
+      cnt += (unsigned)(__double2hiint(pn) ^ __double2hiint(p)) >> 31;
+      pm = p;
+      p = pn;
+    }
+    pow2_rescale(p, pm);
   }
   return cnt;
 }
 
 __device__ __forceinline__ double2 warp_sum2(double2 t) {
+#pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     t.x += __shfl_xor_sync(0xffffffffu, t.x, o);
     t.y += __shfl_xor_sync(0xffffffffu, t.y, o);
@@ -493,121 +502,144 @@ __device__ __forceinline__ double2 warp_sum2(double2 t) {
   return t;
 }
 
+template <int RPL>   // rows per lane: n <= 32 RPL
 __global__ void __launch_bounds__(RR_THREADS) k_rr_tridiag(const double2* Min, int n, int nb, int descending,
                                                            double* theta, double2* Yout, int* status) {
   extern __shared__ __align__(16) unsigned char smem[];
-  double2* A = reinterpret_cast<double2*>(smem);   // n x n, column-major; reflectors kept below the diagonal
-  double2* vv = A + n * n;
+  const int ld = rr_ld(n), ldz = nb + 1;
+  double2* A = reinterpret_cast<double2*>(smem);   // n columns, reflectors kept below the diagonal
+  double2* vv = A + n * ld;
   double2* pp = vv + n;
   double2* taus = pp + n;
-  double2* Ys = taus + n;                           // n x nb back-transformed vectors
-  double* dd = reinterpret_cast<double*>(Ys + n * nb);
-  double* ee = dd + n;
-  double* lam = ee + n;                             // kMaxRR
+  double* dd = reinterpret_cast<double*>(taus + n);
+  const int np = (n + 7) / 8 * 8;
+  double* ee = dd + np;
+  double* es = ee + np;                             // e held off zero, -1 / es, es^2 (from index 1)
+  double* ne = es + np;
+  double* e2 = ne + np;
+  double* lam = e2 + np;                            // kMaxRR
   double* blo = lam + kMaxRR;                       // kMaxRR
   double* bhi = blo + kMaxRR;                       // kMaxRR
-  double* Z = bhi + kMaxRR;                         // n x nb eigenvectors of T
-  int* cnt = reinterpret_cast<int*>(Z + n * nb);    // RR_THREADS
-  __shared__ double red[RR_THREADS / 32];
-  __shared__ double2 redc[RR_THREADS / 32];
-  __shared__ double2 s_tau, s_scal, s_a2;
-  __shared__ int s_triv;
+  double* Z = bhi + kMaxRR;                         // [n][ldz] eigenvectors of T
+  int* cnt = reinterpret_cast<int*>(Z + n * ldz);   // RR_THREADS
+  int* tex = cnt + RR_THREADS;                      // [10][ldz] exponents of the recurrence from the top
   __shared__ double s_lo, s_hi, s_tn;
   const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
   constexpr int bs = RR_THREADS, NW = RR_THREADS / 32;
+  constexpr int RR_RED = RPL == 2 ? 256 : 512;      // threads of the reduction
   for (int it = tid; it < n * n; it += bs) {
     const int a = it % n, b = it / n;
     double2 v = Min[it];
     if (a == b) v.y = 0.0;
     if (a < b) v = cconj(Min[b + a * n]);
-    A[it] = v;
+    A[a + b * ld] = v;
   }
   __syncthreads();
-  // ---- 1. tridiagonal reduction
-  for (int j = 0; j < n - 1; ++j) {
+  // ---- 1. tridiagonal reduction, by RR_RED threads (what every warp does for itself costs each sub-partition
+  //         its share of FP64 issue)
+  auto red_sync = [] { asm volatile("bar.sync 1, %0;" ::"n"(RR_RED) : "memory"); };
+  for (int j = 0; j < (tid < RR_RED ? n - 1 : 0); ++j) {
     const int m = n - j - 1;
-    double s = 0.0;
-    for (int i = 1 + tid; i < m; i += bs) {
-      const double2 x = A[(j + 1 + i) + j * n];
-      s += x.x * x.x + x.y * x.y;
+    const double2* x = A + (j + 1) + j * ld;
+    double xn2 = 0.0;
+#pragma unroll
+    for (int u = 0; u < RPL; ++u) {
+      const int i = lane + 32 * u;
+      if (i > 0 && i < m) xn2 = fma(x[i].x, x[i].x, fma(x[i].y, x[i].y, xn2));
     }
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) red[wp] = s;
-    __syncthreads();
-    if (wp == 0) {
-      double xn2 = (lane < NW) ? red[lane] : 0.0;
-      for (int o = 16; o > 0; o >>= 1) xn2 += __shfl_xor_sync(0xffffffffu, xn2, o);
-      if (lane == 0) {
-        const double2 al = A[(j + 1) + j * n];
-        if (xn2 == 0.0 && al.y == 0.0) {
-          s_triv = 1;
-          s_tau = make_double2(0, 0);
-          ee[j] = al.x;
-        } else {
-          s_triv = 0;
-          const double beta = -copysign(sqrt(al.x * al.x + al.y * al.y + xn2), al.x);
-          const double ib = 1.0 / beta;
-          s_tau = make_double2((beta - al.x) * ib, -al.y * ib);
-          const double2 den = make_double2(al.x - beta, al.y);
-          const double idn = 1.0 / (den.x * den.x + den.y * den.y);
-          s_scal = make_double2(den.x * idn, -den.y * idn);
-          ee[j] = beta;
-        }
-        dd[j] = A[j + j * n].x;
-        taus[j] = s_tau;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) xn2 += __shfl_xor_sync(0xffffffffu, xn2, o);
+    const double2 al = x[0];
+    const bool triv = xn2 == 0.0 && al.y == 0.0;
+    double2 tau = make_double2(0, 0), scal = tau;
+    double beta = al.x;
+    if (!triv) {
+      const double q = al.x * al.x + al.y * al.y + xn2;
+      double ib;
+      if (q >= DBL_MIN && q < 1e300) {
+        const double y = fast_rsqrt(q);
+        beta = -copysign(q * y, al.x);
+        ib = -copysign(y, al.x);
+      } else {
+        beta = -copysign(sqrt(q), al.x);
+        ib = 1.0 / beta;
       }
+      tau = make_double2((beta - al.x) * ib, -al.y * ib);
+      const double2 den = make_double2(al.x - beta, al.y);
+      const double dn = den.x * den.x + den.y * den.y;
+      const double idn = (dn >= DBL_MIN && dn < 1e300) ? fast_rcp(dn) : 1.0 / dn;
+      scal = make_double2(den.x * idn, -den.y * idn);
     }
-    __syncthreads();
-    const int triv = s_triv;
-    const double2 tau = s_tau;
-    for (int i = tid; i < m; i += bs) {
-      const double2 v = (i == 0) ? make_double2(1, 0) : (triv ? make_double2(0, 0) : cmul(A[(j + 1 + i) + j * n], s_scal));
-      vv[i] = v;
-      A[(j + 1 + i) + j * n] = v;
+    if (tid < m) vv[tid] = (tid == 0) ? make_double2(1, 0) : (triv ? make_double2(0, 0) : cmul(x[tid], scal));
+    if (tid == 0) {
+      dd[j] = A[j + j * ld].x;
+      ee[j] = beta;
+      taus[j] = tau;
     }
-    __syncthreads();
-    if (triv) continue;
-    // p = tau A22 v: four threads per row; the partial p^H v of each row group on the fly
-    double2 t = make_double2(0, 0);
+    red_sync();
+    if (tid < m) A[(j + 1 + tid) + j * ld] = vv[tid];
+    if (triv) continue;   // (the next column's first barrier comes before anything else is written)
+    // p = tau A22 v: four threads per row
     {
       const int part = tid & 3;
       const unsigned gmask = 0xFu << (lane & ~3);
-      for (int i = tid >> 2; i < m; i += bs / 4) {
+      for (int i = tid >> 2; i < m; i += RR_RED / 4) {
         double2 acc = make_double2(0, 0);
-        for (int k = part; k < m; k += 4) acc = cadd(acc, cmul(A[(j + 1 + i) + (j + 1 + k) * n], vv[k]));
+        const double2* row = A + (j + 1 + i) + (j + 1) * ld;
+#pragma unroll 4
+        for (int k = part; k < m; k += 4) acc = cadd(acc, cmul(row[k * ld], vv[k]));
         acc.x += __shfl_xor_sync(gmask, acc.x, 1);
         acc.y += __shfl_xor_sync(gmask, acc.y, 1);
         acc.x += __shfl_xor_sync(gmask, acc.x, 2);
         acc.y += __shfl_xor_sync(gmask, acc.y, 2);
-        const double2 pi = cmul(tau, acc);
-        if (part == 0) {
-          pp[i] = pi;
-          t = cadd(t, cmulc(pi, vv[i]));
+        if (part == 0) pp[i] = cmul(tau, acc);
+      }
+    }
+    red_sync();
+    // w = p + a2 v, a2 = -tau/2 p^H v; A22 -= v w^H + w v^H, a warp per column, a lane's rows in registers
+    double2 vr[RPL], wr[RPL], t = make_double2(0, 0);
+#pragma unroll
+    for (int u = 0; u < RPL; ++u) {
+      const int i = lane + 32 * u;
+      vr[u] = i < m ? vv[i] : make_double2(0, 0);
+      wr[u] = i < m ? pp[i] : make_double2(0, 0);
+      t = cadd(t, cmulc(wr[u], vr[u]));
+    }
+    const double2 a2 = cscale(cmul(tau, warp_sum2(t)), -0.5);
+#pragma unroll
+    for (int u = 0; u < RPL; ++u) wr[u] = cadd(wr[u], cmul(a2, vr[u]));
+    for (int c0 = wp; c0 < m; c0 += RR_RED / 8) {   // four columns' loads together
+      double2 vc[4], wc[4], x4[4][RPL];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int c = min(c0 + k * (RR_RED / 32), m - 1);
+        vc[k] = vv[c];
+        wc[k] = pp[c];
+#pragma unroll
+        for (int u = 0; u < RPL; ++u)
+          if (32 * u < m) x4[k][u] = A[(j + 1) + min(lane + 32 * u, m - 1) + (j + 1 + c) * ld];
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int c = c0 + k * (RR_RED / 32);
+        if (c >= m) break;
+        wc[k] = cconj(cadd(wc[k], cmul(a2, vc[k])));
+        vc[k] = cconj(vc[k]);
+#pragma unroll
+        for (int u = 0; u < RPL; ++u) {
+          const int r = lane + 32 * u;
+          if (32 * u < m) {
+            x4[k][u] = csub(x4[k][u], cadd(cmul(vr[u], wc[k]), cmul(wr[u], vc[k])));
+            if (r < m) A[(j + 1) + r + (j + 1 + c) * ld] = x4[k][u];
+          }
         }
       }
     }
-    t = warp_sum2(t);
-    if (lane == 0) redc[wp] = t;
-    __syncthreads();
-    if (wp == 0) {
-      double2 sum = (lane < NW) ? redc[lane] : make_double2(0, 0);
-      sum = warp_sum2(sum);
-      if (lane == 0) s_a2 = cscale(cmul(tau, sum), -0.5);
-    }
-    __syncthreads();
-    const double2 a2 = s_a2;
-    for (int i = tid; i < m; i += bs) pp[i] = cadd(pp[i], cmul(a2, vv[i]));   // w
-    __syncthreads();
-    for (int it = tid; it < m * m; it += bs) {
-      const int r = it % m, c = it / m;
-      double2 x = A[(j + 1 + r) + (j + 1 + c) * n];
-      x = csub(x, cadd(cmul(vv[r], cconj(pp[c])), cmul(pp[r], cconj(vv[c]))));
-      A[(j + 1 + r) + (j + 1 + c) * n] = x;
-    }
-    __syncthreads();
+    red_sync();
   }
+  __syncthreads();
   if (tid == 0) {
-    dd[n - 1] = A[(n - 1) + (n - 1) * n].x;
+    dd[n - 1] = A[(n - 1) + (n - 1) * ld].x;
     double lo = 0.0, hi = 0.0;
     for (int i = 0; i < n; ++i) {
       const double r = (i > 0 ? fabs(ee[i - 1]) : 0.0) + (i < n - 1 ? fabs(ee[i]) : 0.0);
@@ -618,6 +650,17 @@ __global__ void __launch_bounds__(RR_THREADS) k_rr_tridiag(const double2* Min, i
     const double pad = 4.0 * DBL_EPSILON * s_tn + 1e-300;
     s_lo = lo - pad;
     s_hi = hi + pad;
+  }
+  __syncthreads();
+  if (tid < n) {
+    const double floor_e = 0x1p-80 * fmax(s_tn, 0x1p-400);
+    auto off = [&](int k) { return fabs(ee[k]) < floor_e ? copysign(floor_e, ee[k]) : ee[k]; };
+    es[tid] = tid < n - 1 ? off(tid) : 1.0;
+    ne[tid] = -1.0 / es[tid];
+    e2[tid] = tid > 0 ? off(tid - 1) * off(tid - 1) : 0.0;
+  } else if (tid < np) {
+    dd[tid] = 4.0 * s_tn;
+    e2[tid] = 0.0;
   }
   __syncthreads();
   // ---- 2. multisection bisection down to ~2^-44 of the Gershgorin width
@@ -641,7 +684,7 @@ __global__ void __launch_bounds__(RR_THREADS) k_rr_tridiag(const double2* Min, i
     if (e < nb) {
       const double lo = blo[e], hi = bhi[e];
       const double x = lo + (hi - lo) * ((double)(g + 1) * ig);
-      cnt[tid] = sturm_count(dd, ee, n, x);
+      cnt[tid] = sturm_count(dd, e2, n, x);
     }
     __syncthreads();
     if (e < nb && g == 0) {
@@ -672,12 +715,80 @@ __global__ void __launch_bounds__(RR_THREADS) k_rr_tridiag(const double2* Min, i
     if (leader) {
       int cs = 1;
       while (tid + cs < nb && fabs(lam[tid + cs] - lam[tid + cs - 1]) <= ctol) ++cs;
+      bool good = false;
+      if (cs == 1) {
+        double lm = lam[tid], res = 0.0, nrm = 1.0;
+        for (int rd = 0; rd < 2; ++rd) {
+          lm += res / nrm;   // Rayleigh quotient of the joined vector (its one nonzero residual over |z|^2)
+          // from the top, stored with an exponent per eight rows
+          double z = 1.0, zp = 0.0;
+          int E = 0;
+          for (int k = 0; k < n; ++k) {
+            if ((k & 7) == 0) {
+              E += pow2_rescale(z, zp);
+              tex[(k >> 3) * ldz + tid] = E;
+            }
+            Z[k * ldz + tid] = z;
+            const double zn = fma(dd[k] - lm, z, (k > 0 ? es[k - 1] : 0.0) * zp) * ne[k];
+            zp = z;
+            z = zn;
+          }
+          // from the bottom: the row where |top bottom| is largest
+          int r = n - 1, bE = INT_MIN, tEr = 0, bEr = 0;
+          double bM = 0.0, tr = 1.0, br = 1.0;
+          z = 1.0, zp = 0.0, E = 0;
+          for (int k = n - 1; k >= 0; --k) {
+            if ((k & 7) == 7) E += pow2_rescale(z, zp);
+            const double tv = Z[k * ldz + tid], v = fabs(tv * z);
+            const int tE = tex[(k >> 3) * ldz + tid], h = __double2hiint(v), ve = tE + E + (h >> 20) - 1023;
+            const double vm = __hiloint2double((h & 0x000fffff) | 0x3ff00000, __double2loint(v));
+            if (v > 0.0 && (ve > bE || (ve == bE && vm > bM))) {
+              bE = ve;
+              bM = vm;
+              r = k;
+              tr = tv;
+              tEr = tE;
+              br = z;
+              bEr = E;
+            }
+            const double zn = fma(dd[k] - lm, z, es[k] * zp) * (k > 0 ? ne[k - 1] : 0.0);
+            zp = z;
+            z = zn;
+          }
+          // joined and scaled to z_r = 1
+          const double st = 1.0 / tr, sb = 1.0 / br;
+          double fb = sb * pow2_clamped(-bEr), up = 0.0, dn = 0.0;
+          nrm = 0.0;
+          z = 1.0, zp = 0.0, E = 0;
+          for (int k = n - 1; k >= 0; --k) {
+            if ((k & 7) == 7) {
+              E += pow2_rescale(z, zp);
+              fb = sb * pow2_clamped(E - bEr);
+            }
+            const double y = k > r ? z * fb : Z[k * ldz + tid] * (st * pow2_clamped(tex[(k >> 3) * ldz + tid] - tEr));
+            if (k == r + 1) dn = y;
+            if (k == r - 1) up = y;
+            nrm = fma(y, y, nrm);
+            Z[k * ldz + tid] = y;
+            const double zn = fma(dd[k] - lm, z, es[k] * zp) * (k > 0 ? ne[k - 1] : 0.0);
+            zp = z;
+            z = zn;
+          }
+          res = fma(r > 0 ? es[r - 1] : 0.0, up, (dd[r] - lm) + (r < n - 1 ? es[r] : 0.0) * dn);
+        }
+        good = fabs(res) <= 16.0 * DBL_EPSILON * s_tn * sqrt(nrm) && nrm < 1e300;
+        if (good) {
+          const double c = 1.0 / sqrt(nrm);
+          for (int k = 0; k < n; ++k) Z[k * ldz + tid] *= c;
+        }
+      }
       const double pert = DBL_EPSILON * fmax(s_tn, 1e-300);
       double r1[kMaxRR], u2[kMaxRR], u3[kMaxRR], ml[kMaxRR];
       unsigned char sw[kMaxRR];
-      for (int sidx = 0; sidx < cs; ++sidx) {
+      for (int sidx = 0; sidx < (good ? 0 : cs); ++sidx) {
         const int col = tid + sidx;
-        double* x = Z + col * n;
+        double* zc = Z + col;
+        auto x = [&](int k) -> double& { return zc[k * ldz]; };
         const double lm = lam[col];
         double diag = dd[0] - lm, sup = (n > 1) ? ee[0] : 0.0;
         for (int k = 0; k < n - 1; ++k) {
@@ -707,41 +818,41 @@ __global__ void __launch_bounds__(RR_THREADS) k_rr_tridiag(const double2* Min, i
         }
         if (fabs(diag) < pert) diag = copysign(pert, diag);
         const double rlast = 1.0 / diag;
-        for (int k = 0; k < n; ++k) x[k] = 1.0 + 0.1 * (double)((k * 7 + col * 13) % 17) / 17.0;
+        for (int k = 0; k < n; ++k) x(k) = 1.0 + 0.1 * (double)((k * 7 + col * 13) % 17) / 17.0;
         for (int itr = 0; itr < 3; ++itr) {
-          double cur = x[0];
+          double cur = x(0);
           for (int k = 0; k < n - 1; ++k) {
-            const double nxt = x[k + 1];
+            const double nxt = x(k + 1);
             if (sw[k]) {
-              x[k] = nxt;
+              x(k) = nxt;
               cur = cur - ml[k] * nxt;
             } else {
-              x[k] = cur;
+              x(k) = cur;
               cur = nxt - ml[k] * cur;
             }
           }
           double x2 = 0.0, x1 = cur * rlast, nrm = x1 * x1;
-          x[n - 1] = x1;
+          x(n - 1) = x1;
           for (int k = n - 2; k >= 0; --k) {
-            const double xk = (x[k] - u2[k] * x1 - u3[k] * x2) * r1[k];
-            x[k] = xk;
+            const double xk = (x(k) - u2[k] * x1 - u3[k] * x2) * r1[k];
+            x(k) = xk;
             nrm += xk * xk;
             x2 = x1;
             x1 = xk;
           }
           double sc = 1.0 / sqrt(nrm);
-          for (int k = 0; k < n; ++k) x[k] *= sc;
+          for (int k = 0; k < n; ++k) x(k) *= sc;
           if (sidx > 0) {
             for (int t2 = 0; t2 < sidx; ++t2) {
-              const double* y = Z + (tid + t2) * n;
+              const double* yc = Z + (tid + t2);
               double dot = 0.0;
-              for (int k = 0; k < n; ++k) dot += x[k] * y[k];
-              for (int k = 0; k < n; ++k) x[k] -= dot * y[k];
+              for (int k = 0; k < n; ++k) dot += x(k) * yc[k * ldz];
+              for (int k = 0; k < n; ++k) x(k) -= dot * yc[k * ldz];
             }
             double n2 = 0.0;
-            for (int k = 0; k < n; ++k) n2 += x[k] * x[k];
+            for (int k = 0; k < n; ++k) n2 += x(k) * x(k);
             sc = 1.0 / sqrt(n2);
-            for (int k = 0; k < n; ++k) x[k] *= sc;
+            for (int k = 0; k < n; ++k) x(k) *= sc;
           }
         }
       }
@@ -750,37 +861,50 @@ __global__ void __launch_bounds__(RR_THREADS) k_rr_tridiag(const double2* Min, i
   __syncthreads();
   // ---- 4. back-transform y = H_0 H_1 ... H_{n-2} z: each warp carries its vectors together
   {
-    constexpr int VPW = (kMaxRR / 2 + NW - 1) / NW;   // vectors per warp (nb <= kMaxRR / 2)
-    int cols[VPW];
-    int nv = 0;
-    for (int c = wp; c < nb && nv < VPW; c += NW) cols[nv++] = c;
-    for (int q = 0; q < nv; ++q)
-      for (int k = lane; k < n; k += 32) Ys[cols[q] * n + k] = make_double2(Z[cols[q] * n + k], 0.0);
-    __syncwarp();
-    for (int j = n - 2; j >= 0; --j) {
-      const double2 tau = taus[j];
-      if (tau.x == 0.0 && tau.y == 0.0) continue;
-      double2 dot[VPW];
+    static_assert(kMaxRR / 2 <= 3 * NW, "three vectors a warp");
+    auto back = [&](auto vpw) {
+      constexpr int VPW = decltype(vpw)::value;   // vectors per warp
+      double2 y[VPW][RPL];
 #pragma unroll
-      for (int q = 0; q < VPW; ++q) dot[q] = make_double2(0, 0);
-      for (int k = j + 1 + lane; k < n; k += 32) {
-        const double2 v = A[k + j * n];
+      for (int q = 0; q < VPW; ++q)
+#pragma unroll
+        for (int u = 0; u < RPL; ++u) {
+          const int c = wp + q * NW, k = lane + 32 * u;
+          y[q][u] = make_double2(c < nb && k < n ? Z[k * ldz + c] : 0.0, 0.0);
+        }
+      for (int j = n - 2; j >= 0; --j) {
+        const double2 tau = taus[j];
+        double2 v[RPL], dot[VPW];
+#pragma unroll
+        for (int u = 0; u < RPL; ++u) {
+          const int k = lane + 32 * u;
+          v[u] = (k > j && k < n) ? A[k + j * ld] : make_double2(0, 0);
+        }
+#pragma unroll
+        for (int q = 0; q < VPW; ++q) {
+          dot[q] = make_double2(0, 0);
+#pragma unroll
+          for (int u = 0; u < RPL; ++u) dot[q] = cadd(dot[q], cmulc(v[u], y[q][u]));
+        }
 #pragma unroll
         for (int q = 0; q < VPW; ++q)
-          if (q < nv) dot[q] = cadd(dot[q], cmulc(v, Ys[cols[q] * n + k]));
-      }
-#pragma unroll
-      for (int q = 0; q < VPW; ++q) dot[q] = warp_sum2(dot[q]);
-      for (int k = j + 1 + lane; k < n; k += 32) {
-        const double2 v = A[k + j * n];
+          dot[q] = cmul(tau, warp_sum2(dot[q]));
 #pragma unroll
         for (int q = 0; q < VPW; ++q)
-          if (q < nv) Ys[cols[q] * n + k] = csub(Ys[cols[q] * n + k], cmul(v, cmul(tau, dot[q])));
+#pragma unroll
+          for (int u = 0; u < RPL; ++u) y[q][u] = csub(y[q][u], cmul(v[u], dot[q]));
       }
-      __syncwarp();
-    }
-    for (int q = 0; q < nv; ++q)
-      for (int k = lane; k < n; k += 32) Yout[(long long)cols[q] * n + k] = Ys[cols[q] * n + k];
+#pragma unroll
+      for (int q = 0; q < VPW; ++q)
+#pragma unroll
+        for (int u = 0; u < RPL; ++u) {
+          const int c = wp + q * NW, k = lane + 32 * u;
+          if (c < nb && k < n) Yout[(long long)c * n + k] = y[q][u];
+        }
+    };
+    if (nb <= NW) back(std::integral_constant<int, 1>{});
+    else if (nb <= 2 * NW) back(std::integral_constant<int, 2>{});
+    else back(std::integral_constant<int, 3>{});
   }
   if (tid < nb) theta[tid] = lam[tid];
   if (tid == 0) *status = 0;
@@ -1012,13 +1136,15 @@ int run_davidson(wtbg_ctx* ctx, int nev, int nb, int largest, int max_iter, doub
   if (int r = hemm(ctx, X, (int)N, nb, HX, (int)N, w.Yp)) return r;
   // first Rayleigh-Ritz on X alone
   const size_t rrsm = rr_smem_bytes(kMaxRR, kMaxRR / 2);
-  CK(cudaFuncSetAttribute(k_rr_tridiag, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rrsm));
+  CK(cudaFuncSetAttribute(k_rr_tridiag<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rrsm));
+  CK(cudaFuncSetAttribute(k_rr_tridiag<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rrsm));
   double2* Mm = w.small;
   double2* Y = w.small + kMaxRR * kMaxRR;
   auto rr = [&](const double2* Vb, const double2* HVb, int n) -> int {
     if (int r = gram(ctx, Vb, (int)N, n, HVb, (int)N, n, Mm, w.part)) return r;
     const size_t sm = rr_smem_bytes(n, nb);
-    k_rr_tridiag<<<1, RR_THREADS, sm, s>>>(Mm, n, nb, largest, w.theta, Y, w.istat + 1); WTBG_COUNT(ctx, 1);
+    (n <= 64 ? k_rr_tridiag<2> : k_rr_tridiag<3>)<<<1, RR_THREADS, sm, s>>>(Mm, n, nb, largest, w.theta, Y, w.istat + 1);
+    WTBG_COUNT(ctx, 1);
     CKL("k_rr_tridiag");
     // X = V Y(:, :nb), HX = HV Y(:, :nb)
     if (int r = tall(ctx, Vb, (int)N, n, Y, nb, w.Xn, (int)N, false)) return r;

@@ -59,15 +59,6 @@ __global__ void k_td_records(const double* __restrict__ d, const double* __restr
   vec[2 * k + 1] = make_double2(-1.0 / ek, (k >= 1 && k < n) ? -1.0 / ep : 0.0);
 }
 
-// a, b scaled by the power of two that brings the larger to [1, 2); returns the exponent taken out
-__device__ __forceinline__ int rescale(double& a, double& b) {
-  const int h = max(__double2hiint(a) & 0x7ff00000, __double2hiint(b) & 0x7ff00000);
-  const double f = __hiloint2double(0x7fe00000 - h, 0);
-  a *= f;
-  b *= f;
-  return (h >> 20) - 1023;
-}
-
 // Number of eigenvalues of the scaled T below x, one point per thread: the sign changes of the leading
 // minors p_{k+1} = (d_k - x) p_k - e_{k-1}^2 p_{k-1} (the counts of the pivots p_{k+1} / p_k, and as backward
 // stable: each step is exact for d_k - x and e_{k-1}^2 changed by a few roundings).  Without a division the chain
@@ -103,7 +94,7 @@ __device__ __forceinline__ int block_sturm(const double2* __restrict__ rec, int 
         pp = p;
         p = pn;
       }
-      rescale(p, pp);
+      pow2_rescale(p, pp);
     };
     load(a, 0);
 #pragma unroll 1
@@ -279,9 +270,6 @@ struct __align__(16) TwTile {
 __device__ __forceinline__ double tw_step(double a, double z, double e, double zp, double nie) {
   return __dmul_rn(__fma_rn(a, z, __dmul_rn(e, zp)), nie);
 }
-__device__ __forceinline__ double pow2_clamped(int x) {
-  return __hiloint2double((min(max(x, -1023), 1000) + 1023) << 20, 0);   // 0 below 2^-1022
-}
 
 template <int NGT>
 __global__ void __launch_bounds__(32) k_twist(TwistArgs a) {
@@ -322,7 +310,7 @@ __global__ void __launch_bounds__(32) k_twist(TwistArgs a) {
       issue(t + TW_ST - 1, (t + TW_ST - 1) % TW_ST, 1);
       const TwTile<NGT>& s = ring[t % TW_ST];
       for (int b = 0; b < TW; b += 8) {
-        E += rescale(z, zp);
+        E += pow2_rescale(z, zp);
         TE[(size_t)((t * TW + b) >> 3) * M] = E;
         double2 de[8];
         double nie[8];
@@ -362,7 +350,7 @@ __global__ void __launch_bounds__(32) k_twist(TwistArgs a) {
       const int k0 = (nt - 1 - t) * TW;
       for (int b = TW - 8; b >= 0; b -= 8) {
         if (k0 + b >= n) continue;
-        E += rescale(z, zp);
+        E += pow2_rescale(z, zp);
         double vb = 0.0, tb = 1.0, bb = 1.0, tv[8], nie[8];
         double2 de[8];
         int kb = 0;
@@ -425,7 +413,7 @@ __global__ void __launch_bounds__(32) k_twist(TwistArgs a) {
       const int k0 = (nt - 1 - t) * TW;
       for (int b = TW - 8; b >= 0; b -= 8) {
         if (k0 + b >= n) continue;
-        E += rescale(z, zp);
+        E += pow2_rescale(z, zp);
         const double fb = sb * pow2_clamped(E - bBE);
         const double ft = st * pow2_clamped(s.te[b >> 3][lane] - bTE);
         double x[8], nie[8];
