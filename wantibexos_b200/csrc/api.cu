@@ -153,6 +153,11 @@ int wtbg_destroy(wtbg_ctx* ctx) {
                     &ctx->pHk, &ctx->pOc, &ctx->pOv, &ctx->pErr, &ctx->triErr, &ctx->gwork,
                     &ctx->t2V, &ctx->t2X, &ctx->t2G, &ctx->t2T, &ctx->t2P, &ctx->t2AB, &ctx->t2prog, &ctx->t2de};
   for (DevBuf* b : bufs) free_buf(*b);
+  for (auto& l : ctx->qlane) {
+    DevBuf* lb[] = {&l.H, &l.V, &l.W, &l.X, &l.T, &l.P, &l.G};
+    for (DevBuf* b : lb) free_buf(*b);
+    if (l.stream) cudaStreamDestroy(l.stream);
+  }
   for (cudaEvent_t e : ctx->evpool) cudaEventDestroy(e);
   if (ctx->tri_exec) cudaGraphExecDestroy(ctx->tri_exec);
   cudaEventDestroy(ctx->ev0);
@@ -933,17 +938,52 @@ static int q_group_two_stage(wtbg_ctx* ctx, int nk, int g0, int gn, const double
   long long N = 0;
   const bool hv = ctx->have_velocity;
   cudaEventRecord(e0, ctx->stream);
+  // Q point i on lane i mod lanes: its build (which ends synchronised, so the buffers that builds share are free
+  // again) and stage 1 run beside stage 1 of the other lanes
+  const int lanes = two_stage_lanes(ctx, (long long)nk * ctx->nc * ctx->nv, gn);
+  for (int l = 1; l < lanes && !r; ++l)
+    if (!ctx->qlane[l - 1].stream) {
+      const cudaError_t ce = cudaStreamCreateWithFlags(&ctx->qlane[l - 1].stream, cudaStreamNonBlocking);
+      if (ce != cudaSuccess) r = cuda_fail(ctx, ce, "Q group: stream");
+    }
+  auto swap_lane = [&](int l) {
+    if (l == 0) return;
+    auto& q = ctx->qlane[l - 1];
+    std::swap(ctx->H, q.H);
+    std::swap(ctx->t2V, q.V);
+    std::swap(ctx->Wp, q.W);
+    std::swap(ctx->t2X, q.X);
+    std::swap(ctx->t2T, q.T);
+    std::swap(ctx->t2P, q.P);
+    std::swap(ctx->t2G, q.G);
+    std::swap(ctx->stream, q.stream);
+  };
+  ctx->nlane = lanes;
   for (int i = 0; i < gn && !r; ++i) {
-    const int iq = g0 + i;
+    const int iq = g0 + i, lane = i % lanes;
+    swap_lane(lane);
+    struct Back {
+      decltype(swap_lane)& f;
+      int l;
+      ~Back() { f(l); }
+    } back{swap_lane, lane};
     if ((r = wtbg_bse_build_q(ctx, nk, kptq + (size_t)iq * nk * 3, q4 + (size_t)iq * 4, p))) break;
     if (i == 0) {
       N = ctx->N;
       if ((r = two_stage_group_begin(ctx, gn))) break;
+      const cudaError_t ce = lanes > 1 ? cudaStreamSynchronize(ctx->stream) : cudaSuccess;   // the error word is clear
+      if (ce != cudaSuccess && (r = cuda_fail(ctx, ce, "Q group"))) break;
     }
     ctx->have_velocity = false;
-    r = two_stage_group_add(ctx, i);
+    r = two_stage_group_add(ctx, i, gn);
     ctx->have_velocity = hv;
   }
+  ctx->nlane = 1;
+  for (int l = 1; l < lanes; ++l)
+    if (ctx->qlane[l - 1].stream) {
+      const cudaError_t ce = cudaStreamSynchronize(ctx->qlane[l - 1].stream);
+      if (ce != cudaSuccess && !r) r = cuda_fail(ctx, ce, "Q group");
+    }
   double* dd = nullptr;
   double* ee = nullptr;
   if (!r) r = two_stage_group_finish(ctx, gn, &dd, &ee);

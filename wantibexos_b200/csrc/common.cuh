@@ -103,6 +103,13 @@ struct wtbg_ctx {
   int panel_cl_max = 0;          // largest cluster of the panel QR (0: not asked yet)
   long long panel_cl_rows = 0;   // panels of up to so many rows run on one cluster
   DevBuf t2V, t2X, t2G, t2T, t2P, t2AB, t2prog, t2de;
+  // matrix, panel buffers and stream of the further Q points whose stage 1 runs side by side (swapped with
+  // H, t2V, Wp, t2X, t2T, t2P, t2G and stream while such a Q is at work), and how many run at a time now
+  struct QLane {
+    DevBuf H, V, W, X, T, P, G;
+    cudaStream_t stream = nullptr;
+  } qlane[3];
+  int nlane = 1;
   cudaGraphExec_t tri_exec = nullptr;
   std::vector<const void*> tri_sig;
   long long tri_launches = 0;
@@ -251,7 +258,8 @@ int launch_dos(wtbg_ctx* ctx, const double* d_etb, const double* d_w, long long 
 int autotune_hemv(wtbg_ctx* ctx, int* hs_out);
 int run_backtransform2(wtbg_ctx* ctx, double2* X, int nvec);
 int two_stage_group_begin(wtbg_ctx* ctx, int nq);
-int two_stage_group_add(wtbg_ctx* ctx, int slot);
+int two_stage_group_add(wtbg_ctx* ctx, int slot, int nq);
+int two_stage_lanes(wtbg_ctx* ctx, long long N, int nq);
 int two_stage_group_finish(wtbg_ctx* ctx, int nq, double** dd, double** ee);
 bool use_two_stage(wtbg_ctx* ctx);
 // C^T (N x M, ldc) (+)= A (M x K, lda) B (N x K, ldb)^T, bf16 operands, FP32 accumulation on the

@@ -856,7 +856,8 @@ __global__ void __launch_bounds__(256, 2) k_hemm2(const double2* __restrict__ A,
 // three times over.  With C1 = Wacc^H V, C2 = Vacc^H V for the pending updates of the look-ahead group (K = 32 KB
 // columns), B = V^H X - C2^H C1 - C1^H C2 and Z = T^H B:
 //   W = (X - Vacc C1 - Wacc C2 - 1/2 V Z) T.
-// CTA b owns the 16-row tiles b, b + G, ...  (1) sums the split partials and takes its share of V^H X, C1 and C2;
+// A share is the 16-row tiles b, b + shares, ... and CTA c takes the shares c, c + G, ... (one, but where several
+// Q points run side by side).  (1) sums the split partials and takes the share of V^H X, C1 and C2;
 // (2) after a grid barrier the shares are summed, 32 entries a CTA, in a fixed order; (3, K > 0) after another the
 // 1024 entries of B, a warp each; (4) after the last W.  All products on the FP64 MMA; 16 rows so that up to
 // nsm * 16 rows run side by side.  The work itself is 1 to 7 us of FP64 an SM; as seven launches with their tails,
@@ -874,7 +875,8 @@ struct WfArgs {
   long long N, k0;
   const double2 *V, *T, *Vacc, *Wacc;
   double2* W;
-  double2* part;         // [G][1 + 2 KB][32 x 32]
+  int shares;            // partial sums: one per CTA of a full device, so the sums do not depend on the grid
+  double2* part;         // [shares][1 + 2 KB][32 x 32]
   double2* red;          // [1 + 2 KB][32 x 32], then B
   unsigned int* cnt;     // this launch's grid-barrier counter (zero at launch)
   int* err;
@@ -912,14 +914,14 @@ __global__ void __launch_bounds__(256, 1) k_wfuse(WfArgs a) {
     }
   };
   // (1)
-  {
+  for (int sh = bid; sh < a.shares; sh += G) {
     const int ih = (wp & 1) * 16, col = (wp >> 1) * 8 + gq;
     double cr[NB][4], ci[NB][4];
 #pragma unroll
     for (int b = 0; b < NB; ++b)
 #pragma unroll
       for (int k = 0; k < 4; ++k) cr[b][k] = ci[b][k] = 0.0;
-    for (int t = bid; t < ntile; t += G) {
+    for (int t = sh; t < ntile; t += a.shares) {
       const long long r0 = (long long)t * WF_TR;
       __syncthreads();
       for (int e = tid; e < 32 * WF_TR; e += 256) {
@@ -958,7 +960,7 @@ __global__ void __launch_bounds__(256, 1) k_wfuse(WfArgs a) {
     for (int b = 0; b < NB; ++b)
 #pragma unroll
       for (int k = 0; k < 4; ++k)
-        a.part[((size_t)bid * NB + b) * 1024 + ih + gq + 8 * (k >> 1) + 32 * ((wp >> 1) * 8 + 2 * tq + (k & 1))] =
+        a.part[((size_t)sh * NB + b) * 1024 + ih + gq + 8 * (k >> 1) + 32 * ((wp >> 1) * 8 + 2 * tq + (k & 1))] =
             make_double2(cr[b][k], ci[b][k]);
   }
   if (!grid_sync(a.cnt, G, a.err)) return;
@@ -966,10 +968,10 @@ __global__ void __launch_bounds__(256, 1) k_wfuse(WfArgs a) {
   for (int g = bid; g < 32 * NB; g += G) {
     const double2* p = a.part + (size_t)g * 32 + lane;
     double2 t = make_double2(0, 0);
-    for (int b0 = wp; b0 < G; b0 += 64) {
+    for (int b0 = wp; b0 < a.shares; b0 += 64) {
       double2 pv[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) pv[u] = (b0 + 8 * u < G) ? ldcg2(p + (size_t)(b0 + 8 * u) * NB * 1024) : make_double2(0, 0);
+      for (int u = 0; u < 8; ++u) pv[u] = (b0 + 8 * u < a.shares) ? ldcg2(p + (size_t)(b0 + 8 * u) * NB * 1024) : make_double2(0, 0);
 #pragma unroll
       for (int u = 0; u < 8; ++u) t = cadd(t, pv[u]);
     }
@@ -1028,7 +1030,8 @@ __global__ void __launch_bounds__(256, 1) k_wfuse(WfArgs a) {
       sC[(cb + 2 * tq + (k & 1)) * LDC + 2 * K + ih + gq + 8 * (k >> 1)] = make_double2(0.5 * zr[k], 0.5 * zi[k]);
   }
   const int cb = (wp & 3) * 8, kh = wp >> 2;
-  for (int t = bid; t < ntile; t += G) {
+  for (int sh = bid; sh < a.shares; sh += G)
+  for (int t = sh; t < ntile; t += a.shares) {
     const long long r0 = (long long)t * WF_TR;
     __syncthreads();
     load_tile(r0);
@@ -2246,12 +2249,13 @@ static int run_stage1(wtbg_ctx* ctx, int ng, int band) {
     wa.cnt = cnt + npan + pnl;
     wa.err = err;
     const long long ntile = (m + WF_TR - 1) / WF_TR, per = (ntile + nsm - 1) / nsm;
+    wa.shares = (int)((ntile + per - 1) / per);
     const void* const wf[LOOKAHEAD] = {(const void*)k_wfuse<0>, (const void*)k_wfuse<1>, (const void*)k_wfuse<2>,
                                        (const void*)k_wfuse<3>};
     const size_t wsm = wf_smem(K / 32);
     CK(cudaFuncSetAttribute(wf[K / 32], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wsm));
     void* wargs[] = {&wa};
-    CK(cudaLaunchCooperativeKernel(wf[K / 32], dim3((unsigned)((ntile + per - 1) / per)), dim3(256), wargs, wsm, s));
+    CK(cudaLaunchCooperativeKernel(wf[K / 32], dim3((unsigned)std::min(wa.shares, nsm / ctx->nlane)), dim3(256), wargs, wsm, s));
     WTBG_COUNT(ctx, 2);
     CKL("two-stage panel");
     return 0;
@@ -2436,7 +2440,26 @@ int two_stage_group_begin(wtbg_ctx* ctx, int nq) {
   CK(cudaMemsetAsync(ctx->triErr.p, 0, 4, ctx->stream));
   return 0;
 }
-int two_stage_group_add(wtbg_ctx* ctx, int slot) { return run_stage1(ctx, 0, slot); }
+int two_stage_group_add(wtbg_ctx* ctx, int slot, int nq) {
+  if (int r = two_stage_buffers(ctx, nq)) return r;   // the panel buffers of a further lane
+  return run_stage1(ctx, 0, slot);
+}
+// Q points whose stage 1 runs side by side, each on its own stream with its own matrix and buffers.  Stage 1 of
+// a small matrix is a chain of kernels that leave most of the device idle (the panel QR takes 16 SMs or 64), and at
+// large N the panels of one run beside the products of another.  The kernels that spin on a grid barrier are all
+// resident at once: k_wfuse takes nsm / lanes CTAs, and the grid-wide panel QR (64 CTAs up to N = 9216) runs only
+// where there are two lanes; four where every panel goes to a cluster.  A path of 12 Q points of N = 576 27.8 ->
+// 13.3 ms, 6 of 1156 34.8 -> 20.9, 4 of 2304 58.4 -> 38.2 (two lanes 43.8), 3 of 5625 240 -> 214, of 8100 526 -> 486.
+int two_stage_lanes(wtbg_ctx* ctx, long long N, int nq) {
+  const int nsm = ctx->nsm > 0 ? ctx->nsm : 148;
+  if (ctx->profiling || nq < 2 || N > 9216 || nsm < 128) return 1;
+  if (panel_cluster_limits(ctx)) return 1;
+  const int n = std::min(nq, N - BW <= ctx->panel_cl_rows ? 4 : 2);
+  size_t freeb = 0, totb = 0;
+  if (cudaMemGetInfo(&freeb, &totb) != cudaSuccess) return 1;
+  const size_t need = (size_t)(n - 1) * ((size_t)N * N * 16 + (size_t)N * 16 * BW * 32 + (64u << 20));
+  return need <= freeb / 2 ? n : 1;
+}
 int two_stage_group_finish(wtbg_ctx* ctx, int nq, double** dd, double** ee) {
   *dd = ctx->t2de.as<double>();
   *ee = *dd + (size_t)nq * ctx->N;
