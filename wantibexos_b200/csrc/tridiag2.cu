@@ -7,15 +7,15 @@
 // matrix-vector product, so half of its flops run at HBM speed.  Here:
 //
 // Stage 1 (dense -> band), per panel of b columns j0..j0+b-1 with k0 = j0 + b:
-//   (1) k_panel_qr: Householder QR of the panel A[k0:N, j0:j0+b] (ZLARFG reflectors, one
-//       cooperative launch whose CTAs keep their row slices in shared memory, two bounded grid
-//       barriers per column); the T factor of the block reflector Q = I - V T V^H; the velocity
+//   (1) k_panel_qr_cl, k_panel_qr: Householder QR of the panel A[k0:N, j0:j0+b] (ZLARFG reflectors,
+//       one cluster whose CTAs keep their rows in registers, or for long panels one cooperative
+//       launch with the row slices in shared memory); the T factor of the block reflector Q = I - V T V^H; the velocity
 //       vectors g <- Q^T g = g - conj(V) T^T (V^T g).
 //   (2) k_hemm2: X = A22 V on the FP64 tensor cores (mma.sync m16n8k16), A22 = A[k0:N, k0:N]
 //       read once from its stored lower triangle (tiles above the diagonal are read transposed
-//       and conjugated, the diagonal tiles from a symmetrised copy), split over K into
+//       and conjugated, the diagonal tiles mirrored on the way), split over K into
 //       deterministic partial sums.
-//   (3) k_xreduce / k_mform / k_wform: X <- X T, M = T^H V^H X, W = X - 1/2 V M.
+//   (3) k_wfuse: W = (X - 1/2 V T^H V^H X) T, with the corrections of the look-ahead group.
 //   (4) k_her2k (tridiag.cu): A22 -= V W^H + W V^H, so that A22 <- Q^H A22 Q.
 //   Both large products are GEMM-shaped, so the stage runs at tensor-core speed where the
 //   one-stage mat-vec runs at HBM speed.
@@ -443,15 +443,17 @@ __device__ __forceinline__ void reflector_scalars(double2 al, double xn2, double
 // [k0 + cR, k0 + (c+1)R), R = 8 NR, and keeps them in registers: eight threads per column hold its rows
 // i = 8u + sl, and the conjugated velocity vectors are further columns.  Column step p: every column's
 // dot product S_q = sum_{r > k0+p} conj(x_r) P_rq with the pivot column x (in shared memory, zero up to
-// row p), the CTAs' sums exchanged through distributed shared memory, one cluster barrier; then with the
+// row p), the CTAs' sums exchanged through distributed shared memory, counted by mbarriers; then with the
 // unscaled vector u = x - beta e_p the reflector is H = I - kappa u u^H and w_q = u^H P_q = S_q +
 // conj(u_p) P_pq (row p is posted by CTA 0) serves three ends: columns q > p are updated by P_q -=
 // conj(kappa) w_q u, finished columns q < p give the Gram entry v_q^H v_p = conj(w_q) / u_p that the T factor
-// needs, and the velocity columns give V^T g the same way.  T = T_1 + T_2 blocks by doubling.
+// needs, and the velocity columns give V^T g the same way.  The last warp, which holds no column, forms T
+// one column behind.
 // Bound by the latency of the column chain.  The grid-wide form (k_panel_qr, still used for longer
 // panels) pays a barrier and two round trips through L2 per column, keeps the slice in shared memory
 // (whose bandwidth bounds update and dot products) and forms Gram matrix and V^T g in passes of their
-// own.  Per panel, grid-wide against cluster: N = 576 170 / 68 us, 2304 189 / 91 us.
+// own.  Per panel, grid-wide against cluster: N = 576 170 / 68 us, 2304 189 / 91 us (with cluster barriers and T by
+// doubling; 59 us at 144 rows and 105 at 2272 against 70 and 115 since the exchange is counted and T formed along).
 constexpr int PC_THREADS = 384;   // 48 columns x 8 threads: 32 of the panel, up to 10 velocity vectors
 constexpr int PC_COLS = BW + NGMAX;
 constexpr int PC_MAXC = 16;
@@ -2039,7 +2041,8 @@ static bool two_stage_fits(wtbg_ctx* ctx, long long N) {
 // The reduction used for the current matrix: two-stage wherever it fits (auto).  Device time of a
 // solve, one-stage against two-stage: N = 36 1.01 / 0.49 ms, 144 4.1 / 2.3, 576 17.4 / 10.4, 1156 36.8 /
 // 22.0, 2304 83.7 / 47.6, 14400 2423 / 979 (the one-stage reduction is four launches per column, the
-// two-stage one ten per 32 columns and one for the chase).
+// two-stage one five per 32 columns and one for the chase).  Later steps brought the two-stage solve of N = 576 to
+// 6.5 ms, of 2304 to 30, of 14400 to 843.
 bool use_two_stage(wtbg_ctx* ctx) { return ctx->tri_mode != 1 && two_stage_fits(ctx, ctx->N); }
 
 // Work buffers of the two-stage reduction for N (nband bands side by side for Q groups).
