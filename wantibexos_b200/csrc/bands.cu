@@ -21,9 +21,8 @@
 // iteration cap and reports non-convergence per k instead of spinning.  A round is two block
 // barriers: w/2 threads form the rotations, then every 2 x 2 block between two rotated pairs is taken
 // through both sides at once (lower triangle only) while other threads rotate the vectors' columns.
-// The round is a latency chain (about 800 cycles with the rotation's square roots and reciprocal as one
-// third-order step each), so the block is sized to w and many k-points share an SM; odd column strides
-// keep the row accesses off one bank.
+// The round is a latency chain (the rotation's square roots and its division in it), so the block is sized
+// to w and many k-points share an SM; odd column strides keep the row accesses off one bank.
 #include <cfloat>
 #include <cub/cub.cuh>
 
@@ -174,10 +173,10 @@ __device__ __forceinline__ void bands_body(const BandsArgs& a, const int k, unsi
           const double ac2 = fma(c.x, c.x, __dmul_rn(c.y, c.y));
           if (ac2 > fmax(0.25 * DBL_EPSILON * DBL_EPSILON * fabs(aa * bb), tol2) && ac2 >= DBL_MIN) {
             // t = sign(d) 2|c| / (|d| + sqrt(d^2 + 4 |c|^2)), d = bb - aa
-            const double ia = fast_rsqrt(ac2), ac = ac2 * ia, d = bb - aa;
+            const double ia = rsqrt(ac2), ac = ac2 * ia, d = bb - aa;
             const double hh = fma(d, d, 4.0 * ac2);
-            const double tt = copysign(2.0 * ac, d) * fast_rcp(fma(hh, fast_rsqrt(hh), fabs(d)));
-            cs = fast_rsqrt(fma(tt, tt, 1.0));
+            const double tt = copysign(2.0 * ac, d) / (fabs(d) + sqrt(hh));
+            cs = rsqrt(fma(tt, tt, 1.0));
             const double sn = tt * cs * ia;
             sx = sn * c.x;
             sy = sn * c.y;
@@ -738,8 +737,7 @@ static size_t bands_smem(int w, int nvec) {
 }
 // Threads per k-point: on a mesh that fills the device few enough that several k-points share an SM, for
 // a few k-points (a path) one thread per item of a round.  Device time: 2304 points of w = 24 3.1 -> 0.77 ms,
-// 1296 of w = 40 8.8 -> 2.1 ms, 16 of w = 24 0.50 -> 0.20 ms (before: 256 threads, five barriers a round, the
-// rotations by library square roots and divisions).
+// 1296 of w = 40 8.8 -> 2.1 ms, 16 of w = 24 0.50 -> 0.20 ms (before: 256 threads, five barriers a round).
 static int bands_threads(wtbg_ctx* ctx, int w, long long nk) {
   if (ctx->nsm <= 0) cudaDeviceGetAttribute(&ctx->nsm, cudaDevAttrMultiProcessorCount, ctx->device);
   const int np = (w + 1) / 2, items = np * (np - 1) / 2 + np * w;

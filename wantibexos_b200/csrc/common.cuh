@@ -180,21 +180,6 @@ __host__ __device__ __forceinline__ double2 cscale(double2 a, double s) {
 }
 __host__ __device__ __forceinline__ double2 cconj(double2 a) { return make_double2(a.x, -a.y); }
 
-// 1/sqrt(x) and 1/x of a normal positive x (1/sqrt(x) also as sqrt(x) = x y): the hardware's first
-// approximation (relative error about 2^-20) and one third-order step, which leaves rounding errors only
-__device__ __forceinline__ double fast_rsqrt(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-(x * y), y, 1.0);   // 1/sqrt(x) = y (1 + e/2 + 3/8 e^2 + O(e^3))
-  return fma(y, e * fma(e, 0.375, 0.5), y);
-}
-__device__ __forceinline__ double fast_rcp(double x) {
-  double r;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-  const double g = fma(-x, r, 1.0);         // 1/x = r (1 + g + g^2 + O(g^3))
-  return fma(r, fma(g, g, g), r);
-}
-
 // a, b scaled by the power of two that brings the larger to [1, 2); returns the exponent taken out
 __device__ __forceinline__ int pow2_rescale(double& a, double& b) {
   const int h = max(__double2hiint(a) & 0x7ff00000, __double2hiint(b) & 0x7ff00000);

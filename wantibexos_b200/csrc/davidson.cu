@@ -545,19 +545,11 @@ __global__ void __launch_bounds__(RR_THREADS) k_rr_tridiag(const double2* Min, i
     double beta = al.x;
     if (!triv) {
       const double q = al.x * al.x + al.y * al.y + xn2;
-      double ib;
-      if (q >= DBL_MIN && q < 1e300) {
-        const double y = fast_rsqrt(q);
-        beta = -copysign(q * y, al.x);
-        ib = -copysign(y, al.x);
-      } else {
-        beta = -copysign(sqrt(q), al.x);
-        ib = 1.0 / beta;
-      }
+      beta = -copysign(sqrt(q), al.x);
+      const double ib = 1.0 / beta;
       tau = make_double2((beta - al.x) * ib, -al.y * ib);
       const double2 den = make_double2(al.x - beta, al.y);
-      const double dn = den.x * den.x + den.y * den.y;
-      const double idn = (dn >= DBL_MIN && dn < 1e300) ? fast_rcp(dn) : 1.0 / dn;
+      const double idn = 1.0 / (den.x * den.x + den.y * den.y);
       scal = make_double2(den.x * idn, -den.y * idn);
     }
     if (tid < m) vv[tid] = (tid == 0) ? make_double2(1, 0) : (triv ? make_double2(0, 0) : cmul(x[tid], scal));

@@ -413,9 +413,7 @@ __device__ __forceinline__ double2 caxpy(double a, double2 b, double2 c) {
 }
 // Reflector scalars of x (first entry al, xn2 = the squared norm of the others): beta =
 // -sign(Re al) |x|, kappa = -u_0 / (beta |u_0|^2), 1/beta, 1/|u_0|^2; no reflector (kappa = 0, al kept)
-// where x is already (real, 0, ..., 0).  The square root and the reciprocal start from the hardware's
-// first approximation (relative error about 2^-20) and take one third-order step each, which leaves
-// rounding errors only; both arguments are normal numbers (|u_0|^2 >= |x|^2).
+// where x is already (real, 0, ..., 0).
 __device__ __forceinline__ void reflector_scalars(double2 al, double xn2, double2& kap, double& beta, double& ib, double& rd) {
   const double ay2 = al.y * al.y;
   const double q = fma(al.x, al.x, ay2 + xn2);
@@ -423,17 +421,10 @@ __device__ __forceinline__ void reflector_scalars(double2 al, double xn2, double
   beta = al.x;
   ib = rd = 0.0;
   if (q >= DBL_MIN && !(xn2 == 0.0 && al.y == 0.0)) {
-    double y, r;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(q));
-    const double t = q * y, e = fma(-t, y, 1.0);         // 1/sqrt(q) = y (1 + e/2 + 3/8 e^2 + O(e^3))
-    const double c = e * fma(e, 0.375, 0.5);
-    const double nr = fma(t, c, t);
-    ib = -copysign(fma(y, c, y), al.x);
-    beta = -copysign(nr, al.x);
-    const double ux = al.x - beta, d = fma(ux, ux, ay2);
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-    const double g = fma(-d, r, 1.0);                    // 1/d = r (1 + g + g^2 + O(g^3))
-    rd = fma(r, fma(g, g, g), r);
+    ib = -copysign(rsqrt(q), al.x);
+    beta = -copysign(sqrt(q), al.x);
+    const double ux = al.x - beta;
+    rd = 1.0 / fma(ux, ux, ay2);
     const double f = -ib * rd;
     kap = make_double2(f * ux, f * al.y);
   }
