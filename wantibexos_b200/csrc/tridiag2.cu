@@ -413,7 +413,9 @@ __device__ __forceinline__ double2 caxpy(double a, double2 b, double2 c) {
 }
 // Reflector scalars of x (first entry al, xn2 = the squared norm of the others): beta =
 // -sign(Re al) |x|, kappa = -u_0 / (beta |u_0|^2), 1/beta, 1/|u_0|^2; no reflector (kappa = 0, al kept)
-// where x is already (real, 0, ..., 0).
+// where x is already (real, 0, ..., 0), or so small that |x|^2 is not a normal number.  kappa is of order |x|^-2 and
+// formed from factors that stay between |x|^-2 and 2, so it is finite for every |x| that is taken; of its products
+// only those with two vectors of order |x| are formed, never its square (which is infinite from |x| = 1e-77 down).
 __device__ __forceinline__ void reflector_scalars(double2 al, double xn2, double2& kap, double& beta, double& ib, double& rd) {
   const double ay2 = al.y * al.y;
   const double q = fma(al.x, al.x, ay2 + xn2);
@@ -425,8 +427,7 @@ __device__ __forceinline__ void reflector_scalars(double2 al, double xn2, double
     beta = -copysign(sqrt(q), al.x);
     const double ux = al.x - beta;
     rd = 1.0 / fma(ux, ux, ay2);
-    const double f = -ib * rd;
-    kap = make_double2(f * ux, f * al.y);
+    kap = make_double2(-(ib * ux) * rd, -(ib * al.y) * rd);
   }
 }
 
@@ -1786,10 +1787,12 @@ __global__ void __launch_bounds__(CH_THREADS, 1) k_chase(BulgeArgs a) {
           wait_warp(s_sr, CH_NX, n);
           const double2 kap = s_sc[xb][0];
           const double beta = s_sc[xb][1].x;
-          // lane = row: w = kappa y - 1/2 |kappa|^2 (u^H y) u, y = D u; then D <- D - u w^H - w u^H
+          // lane = row: w = kappa y - 1/2 |kappa|^2 (u^H y) u, y = D u; then D <- D - u w^H - w u^H.  |kappa|^2 =
+          // 1 / (beta^2 |u_0|^2), so the second term is 1/2 (u'^H y / |u_0|^2) u' with u' = u / beta
           if (lane == 0) ul.x -= beta;
           yl = caxpy(-beta, d0, yl);
-          const double hk = 0.5 * fma(kap.x, kap.x, kap.y * kap.y) * warp_sum(fma(ul.x, yl.x, ul.y * yl.y));
+          ul = cscale(ul, s_sc[xb][1].y);
+          const double hk = 0.5 * s_rd[xb] * warp_sum(fma(ul.x, yl.x, ul.y * yl.y));
           double2* wv = s_wv[wid];
           wv[lane] = caxpy(-hk, ul, cmul(kap, yl));
           __syncwarp();
