@@ -129,7 +129,7 @@ __device__ __forceinline__ void bands_body(const BandsArgs& a, const int k, unsi
       }
     }
     if (m == n) {
-      acc = make_double2(acc.x + (-a.ef32), a.Hk ? 0.0 : acc.y);
+      acc = make_double2(acc.x + (-a.ef32), 0.0);   // ZHEEV does not read the imaginary part
       lam[m] = acc.x;
     }
     A[m + n * ld] = acc;
