@@ -459,7 +459,7 @@ __host__ __device__ constexpr size_t rr_smem_bytes(int n, int nb) {
 
 // Number of eigenvalues of the symmetric tridiagonal (d, e) below x from the sign changes of
 // the leading principal minors p_i = (d_i - x) p_{i-1} - e_{i-1}^2 p_{i-2} (e2[i] = e_{i-1}^2, held above
-// 2^-160 |T|^2 so that no two minors in a row vanish), scaled by a power of two every eight steps;
+// 2^-160 |T|^2 so that no two minors in a row vanish; |T| < 1), scaled by a power of two every eight steps;
 // d and e2 are padded to a multiple of eight by rows that change no sign.
 __device__ __forceinline__ int sturm_count(const double* dd, const double* e2, int n, double x) {
   double pm = 0.0, p = 1.0;
@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(RR_THREADS) k_rr_tridiag(const double2* Min, i
   double* Z = bhi + kMaxRR;                         // [n][ldz] eigenvectors of T
   int* cnt = reinterpret_cast<int*>(Z + n * ldz);   // RR_THREADS
   int* tex = cnt + RR_THREADS;                      // [10][ldz] exponents of the recurrence from the top
-  __shared__ double s_lo, s_hi, s_tn;
+  __shared__ double s_lo, s_hi, s_tn, s_sc;
   const int tid = threadIdx.x, lane = tid & 31, wp = tid >> 5;
   constexpr int bs = RR_THREADS, NW = RR_THREADS / 32;
   constexpr int RR_RED = RPL == 2 ? 256 : 512;      // threads of the reduction
@@ -628,10 +628,21 @@ __global__ void __launch_bounds__(RR_THREADS) k_rr_tridiag(const double2* Min, i
       lo = (i == 0) ? dd[i] - r : fmin(lo, dd[i] - r);
       hi = (i == 0) ? dd[i] + r : fmax(hi, dd[i] + r);
     }
-    s_tn = fmax(fabs(lo), fabs(hi));
-    const double pad = 4.0 * DBL_EPSILON * s_tn + 1e-300;
-    s_lo = lo - pad;
-    s_hi = hi + pad;
+    // from here on T times the power of two that brings |T| to [1/2, 1), so that eight steps of a recurrence
+    // neither overflow nor vanish
+    double tn = fmax(fabs(lo), fabs(hi));
+    int ex = 0;
+    if (tn > 0.0 && tn < 1e300) (void)frexp(tn, &ex);
+    s_sc = ldexp(1.0, -max(ex, -1000));
+    s_tn = tn = tn * s_sc;
+    const double pad = 4.0 * DBL_EPSILON * tn + 1e-300;
+    s_lo = lo * s_sc - pad;
+    s_hi = hi * s_sc + pad;
+  }
+  __syncthreads();
+  if (tid < n) {
+    dd[tid] *= s_sc;
+    if (tid < n - 1) ee[tid] *= s_sc;
   }
   __syncthreads();
   if (tid < n) {
@@ -689,10 +700,11 @@ __global__ void __launch_bounds__(RR_THREADS) k_rr_tridiag(const double2* Min, i
   }
   for (int e = tid; e < nb; e += bs) lam[e] = 0.5 * (blo[e] + bhi[e]);
   __syncthreads();
-  // ---- 3. inverse iteration: T - lambda I = P L U factored once (partial pivoting), three
-  //         solves; eigenvalues closer than 1e-7 |T| are done in order by their first thread
+  // ---- 3. a thread each: the two recurrences joined; where that is not good, and for eigenvalues closer than
+  //         1e-7 |T| (in order by their first thread), inverse iteration: T - lambda I = P L U factored once
+  //         (partial pivoting), three solves
   if (tid < nb) {
-    const double ctol = 1e-7 * fmax(1e-3, s_tn);
+    const double ctol = 1e-7 * fmax(1e-3 * s_sc, s_tn);
     const bool leader = (tid == 0) || fabs(lam[tid] - lam[tid - 1]) > ctol;
     if (leader) {
       int cs = 1;
@@ -888,7 +900,7 @@ __global__ void __launch_bounds__(RR_THREADS) k_rr_tridiag(const double2* Min, i
     else if (nb <= 2 * NW) back(std::integral_constant<int, 2>{});
     else back(std::integral_constant<int, 3>{});
   }
-  if (tid < nb) theta[tid] = lam[tid];
+  if (tid < nb) theta[tid] = lam[tid] / s_sc;
   if (tid == 0) *status = 0;
 }
 
