@@ -4,6 +4,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <optional>
 #include <string>
 #include <vector>
 
@@ -937,6 +938,7 @@ static int q_group_two_stage(wtbg_ctx* ctx, int nk, int g0, int gn, const double
   int r = 0;
   long long N = 0;
   const bool hv = ctx->have_velocity;
+  std::optional<SpinSection> section(std::in_place, ctx);
   cudaEventRecord(e0, ctx->stream);
   // Q point i on lane i mod lanes: its build (which ends synchronised, so the buffers that builds share are free
   // again) and stage 1 run beside stage 1 of the other lanes
@@ -987,6 +989,7 @@ static int q_group_two_stage(wtbg_ctx* ctx, int nk, int g0, int gn, const double
   double* dd = nullptr;
   double* ee = nullptr;
   if (!r) r = two_stage_group_finish(ctx, gn, &dd, &ee);
+  section.reset();
   for (int i = 0; i < gn && !r; ++i) {
     cudaError_t ce = cudaMemcpyAsync(ctx->d.p, dd + (size_t)i * N, (size_t)N * 8, cudaMemcpyDeviceToDevice, ctx->stream);
     if (ce == cudaSuccess)

@@ -242,6 +242,21 @@ int launch_dos(wtbg_ctx* ctx, const double* d_etb, const double* d_w, long long 
                int nw, double sme, long long nkpt, double* d_out);
 int autotune_hemv(wtbg_ctx* ctx, int* hs_out);
 int run_backtransform2(wtbg_ctx* ctx, double2* X, int nvec);
+// Held while a context launches grids whose CTAs wait on one another (the chase, the panel QR, k_wfuse and the
+// back-transforms of the two-stage reduction).  Such a grid ends only when all its CTAs are resident; the launches
+// of one context are ordered, or sized to fit side by side, but two contexts of one device (host threads) could
+// each hold a part of the SMs and wait for the rest.  One context of the process at a time has a device's section, and
+// its stream is drained before it is given on.
+class SpinSection {
+ public:
+  explicit SpinSection(wtbg_ctx* ctx);
+  ~SpinSection();
+  SpinSection(const SpinSection&) = delete;
+  SpinSection& operator=(const SpinSection&) = delete;
+
+ private:
+  wtbg_ctx* ctx_;
+};
 int two_stage_group_begin(wtbg_ctx* ctx, int nq);
 int two_stage_group_add(wtbg_ctx* ctx, int slot, int nq);
 int two_stage_lanes(wtbg_ctx* ctx, long long N, int nq);

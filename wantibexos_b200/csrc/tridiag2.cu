@@ -27,6 +27,7 @@
 #include "tc_sm100.cuh"
 
 #include <algorithm>
+#include <mutex>
 #include <string>
 
 // implemented in tridiag.cu
@@ -2404,7 +2405,18 @@ static int run_stage2(wtbg_ctx* ctx, int nband, int ng, bool store, double* dd, 
   return 0;
 }
 
+static std::mutex& spin_mutex(int device) {
+  static std::mutex m[64];   // device ordinals; two that share one only wait for each other
+  return m[(unsigned)device % 64u];
+}
+SpinSection::SpinSection(wtbg_ctx* ctx) : ctx_(ctx) { spin_mutex(ctx->device).lock(); }
+SpinSection::~SpinSection() {
+  cudaStreamSynchronize(ctx_->stream);   // an error stays with the stream: the caller's next call returns it
+  spin_mutex(ctx_->device).unlock();
+}
+
 int run_tridiagonalise2(wtbg_ctx* ctx) {
+  SpinSection section(ctx);
   const long long N = ctx->N;
   cudaStream_t s = ctx->stream;
   if (int r = two_stage_buffers(ctx, 1)) return r;
@@ -2468,6 +2480,7 @@ int two_stage_group_finish(wtbg_ctx* ctx, int nq, double** dd, double** ee) {
 // Exciton vectors through both stages: X <- Q1 (Q2 X), Q2 the bulge-chasing reflectors in
 // reverse, Q1 the panels' block reflectors in reverse.
 int run_backtransform2(wtbg_ctx* ctx, double2* X, int nvec) {
+  SpinSection section(ctx);
   const long long N = ctx->N;
   cudaStream_t s = ctx->stream;
   const int nsm = ctx->nsm > 0 ? ctx->nsm : 148;
