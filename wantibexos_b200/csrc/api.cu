@@ -1,5 +1,6 @@
 // C-ABI of libwtbgpu.so: context management, argument checks, host <-> device transfers
 // and the order of kernel launches for each replaced reference stage (see wtbgpu.h).
+#include <array>
 #include <cfloat>
 #include <cmath>
 #include <cstdio>
@@ -30,6 +31,11 @@ int ensure(wtbg_ctx* c, DevBuf& b, size_t bytes) {
     b.bytes = 0;
   }
   cudaError_t e = cudaMalloc(&b.p, bytes);
+  if (e != cudaSuccess && c && c->nlane == 1 && lane_bytes(c) > 0) {   // with the Q lanes' memory
+    cudaGetLastError();
+    release_lanes(c);
+    e = cudaMalloc(&b.p, bytes);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     b.p = nullptr;
@@ -49,7 +55,24 @@ void free_buf(DevBuf& b) {
   b.bytes = 0;
 }
 
+template <class Lane>
+auto lane_bufs(Lane& l) {
+  return std::array{&l.H, &l.V, &l.W, &l.X, &l.T, &l.P, &l.G};
+}
+
 }  // namespace
+
+size_t lane_bytes(const wtbg_ctx* ctx) {
+  size_t n = 0;
+  for (const auto& l : ctx->qlane)
+    for (const DevBuf* b : lane_bufs(l)) n += b->bytes;
+  return n;
+}
+
+void release_lanes(wtbg_ctx* ctx) {
+  for (auto& l : ctx->qlane)
+    for (DevBuf* b : lane_bufs(l)) free_buf(*b);
+}
 
 int ensure_events(wtbg_ctx* ctx, size_t n) {
   while (ctx->evpool.size() < n) {
@@ -154,11 +177,9 @@ int wtbg_destroy(wtbg_ctx* ctx) {
                     &ctx->pHk, &ctx->pOc, &ctx->pOv, &ctx->pErr, &ctx->triErr, &ctx->gwork,
                     &ctx->t2V, &ctx->t2X, &ctx->t2G, &ctx->t2T, &ctx->t2P, &ctx->t2AB, &ctx->t2prog, &ctx->t2de};
   for (DevBuf* b : bufs) free_buf(*b);
-  for (auto& l : ctx->qlane) {
-    DevBuf* lb[] = {&l.H, &l.V, &l.W, &l.X, &l.T, &l.P, &l.G};
-    for (DevBuf* b : lb) free_buf(*b);
+  release_lanes(ctx);
+  for (auto& l : ctx->qlane)
     if (l.stream) cudaStreamDestroy(l.stream);
-  }
   for (cudaEvent_t e : ctx->evpool) cudaEventDestroy(e);
   if (ctx->tri_exec) cudaGraphExecDestroy(ctx->tri_exec);
   cudaEventDestroy(ctx->ev0);
@@ -177,6 +198,7 @@ int wtbg_set_model(wtbg_ctx* ctx, int w, int nvec, const double* hre, const doub
   for (int i = 0; i < nvec; ++i)
     if (deg[i] == 0) return set_err(ctx, WTBG_ERR_ARG, "set_model: zero degeneracy");
   if (int r = set_device(ctx)) return r;
+  release_lanes(ctx);   // of the last model's Q points
   ctx->w = w;
   ctx->nvec = nvec;
   for (int i = 0; i < 3; ++i)
@@ -930,7 +952,7 @@ static int tridiagonalise_graph(wtbg_ctx* ctx) {
 // slot (the N x N matrix buffer is reused), one bulge-chasing launch for the group's bands, then
 // the eigenvalues of each tridiagonal form.  ms_q gets the group's device time divided evenly.
 constexpr int kQGroup = 64;
-static int q_group_two_stage(wtbg_ctx* ctx, int nk, int g0, int gn, const double* kptq, const double* q4,
+static int q_group_two_stage(wtbg_ctx* ctx, int nk, int g0, int gn, int max_lanes, const double* kptq, const double* q4,
                              const wtbg_coulomb* p, double* W, double* ms_q) {
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   CK(cudaEventCreate(&e0));
@@ -942,7 +964,7 @@ static int q_group_two_stage(wtbg_ctx* ctx, int nk, int g0, int gn, const double
   cudaEventRecord(e0, ctx->stream);
   // Q point i on lane i mod lanes: its build (which ends synchronised, so the buffers that builds share are free
   // again) and stage 1 run beside stage 1 of the other lanes
-  const int lanes = two_stage_lanes(ctx, (long long)nk * ctx->nc * ctx->nv, gn);
+  const int lanes = std::min(max_lanes, two_stage_lanes(ctx, (long long)nk * ctx->nc * ctx->nv, gn));
   for (int l = 1; l < lanes && !r; ++l)
     if (!ctx->qlane[l - 1].stream) {
       const cudaError_t ce = cudaStreamCreateWithFlags(&ctx->qlane[l - 1].stream, cudaStreamNonBlocking);
@@ -1028,8 +1050,15 @@ int wtbg_bse_q_batch(wtbg_ctx* ctx, int nk, int nq, const double* kptq, const do
     const bool two = use_two_stage(ctx);
     ctx->N = N0;
     if (two) {
-      for (int g0 = 0; g0 < nq && !r; g0 += kQGroup)
-        r = q_group_two_stage(ctx, nk, g0, std::min(kQGroup, nq - g0), kptq, q4, p, W, ms_q);
+      for (int g0 = 0; g0 < nq && !r; g0 += kQGroup) {
+        const int gn = std::min(kQGroup, nq - g0);
+        r = q_group_two_stage(ctx, nk, g0, gn, 4, kptq, q4, p, W, ms_q);
+        if (r == WTBG_ERR_OOM) {   // as one Q point after the other if that fits
+          release_lanes(ctx);
+          ctx->have_velocity = hv;
+          r = q_group_two_stage(ctx, nk, g0, gn, 1, kptq, q4, p, W, ms_q);
+        }
+      }
       ctx->have_velocity = hv;
       ctx->have_matrix = false;
       ctx->fast_ready = false;

@@ -104,7 +104,8 @@ struct wtbg_ctx {
   long long panel_cl_rows = 0;   // panels of up to so many rows run on one cluster
   DevBuf t2V, t2X, t2G, t2T, t2P, t2AB, t2prog, t2de;
   // matrix, panel buffers and stream of the further Q points whose stage 1 runs side by side (swapped with
-  // H, t2V, Wp, t2X, t2T, t2P, t2G and stream while such a Q is at work), and how many run at a time now
+  // H, t2V, Wp, t2X, t2T, t2P, t2G and stream while such a Q is at work), and how many run at a time now.  Kept
+  // between calls, given back by release_lanes: with the next model, and when memory runs short
   struct QLane {
     DevBuf H, V, W, X, T, P, G;
     cudaStream_t stream = nullptr;
@@ -257,6 +258,9 @@ class SpinSection {
  private:
   wtbg_ctx* ctx_;
 };
+// Buffers of the Q lanes: what they hold, and giving them back (between groups only: ctx->nlane == 1)
+size_t lane_bytes(const wtbg_ctx* ctx);
+void release_lanes(wtbg_ctx* ctx);
 int two_stage_group_begin(wtbg_ctx* ctx, int nq);
 int two_stage_group_add(wtbg_ctx* ctx, int slot, int nq);
 int two_stage_lanes(wtbg_ctx* ctx, long long N, int nq);

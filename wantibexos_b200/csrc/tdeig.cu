@@ -913,6 +913,10 @@ static int tridiagonal_solve_body(wtbg_ctx* ctx, int dtfull, int cpol, bool vect
   CK(cudaMemGetInfo(&freeb, &totb));
   const double budget = std::min((double)freeb * 0.6 + (double)ctx->ws.bytes, 96e9);
   long long M = (long long)(budget / (4.0 * 8.0 * (double)n));
+  if (M < n && lane_bytes(ctx) > 0) {   // the Q lanes of an earlier call do not split this one
+    M = (long long)(std::min(budget + 0.6 * (double)lane_bytes(ctx), 96e9) / (4.0 * 8.0 * (double)n));
+    release_lanes(ctx);
+  }
   M = std::max<long long>(M, maxc);
   M = std::min<long long>(M, n);
   M = std::max<long long>(M, 1);

@@ -2467,7 +2467,7 @@ int two_stage_lanes(wtbg_ctx* ctx, long long N, int nq) {
   size_t freeb = 0, totb = 0;
   if (cudaMemGetInfo(&freeb, &totb) != cudaSuccess) return 1;
   const size_t need = (size_t)(n - 1) * ((size_t)N * N * 16 + (size_t)N * 16 * BW * 32 + (64u << 20));
-  return need <= freeb / 2 ? n : 1;
+  return need <= (freeb + lane_bytes(ctx)) / 2 ? n : 1;   // what the lanes hold from the last call counts as free
 }
 int two_stage_group_finish(wtbg_ctx* ctx, int nq, double** dd, double** ee) {
   *dd = ctx->t2de.as<double>();
