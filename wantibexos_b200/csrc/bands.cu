@@ -105,6 +105,7 @@ __device__ __forceinline__ void bands_body(const BandsArgs& a, const int k, unsi
     while (i * (i + 1) / 2 <= e) ++i;
     tri[e] = (unsigned short)(i << 8 | (e - i * (i - 1) / 2));
   }
+  if (tid < w) perm[tid] = tid;   // levels that are NaN all rank first: the places they leave stay indices
   const double kx = a.kpt[3 * k], ky = a.kpt[3 * k + 1], kz = a.kpt[3 * k + 2];
   for (int R = tid; R < nvec; R += bs) ph[R] = phase_of(kx, ky, kz, a.Rcart + 3 * R);
   __syncthreads();
