@@ -98,7 +98,9 @@ int wtbg_reset_stats(wtbg_ctx* ctx);
  * bulge chasing, wherever its panels fit on the device: 34 <= N <= 384 rows per SM; else one-stage),
  * 1 = one-stage (blocked Householder with a Hermitian mat-vec per column), 2 = two-stage
  * wherever it fits, 3 = as 2 with the bulge chasing run one warp per sweep instead of one CTA
- * per sweep (for comparison).  Both give the tridiagonal form of ZHETRD('L') up to rounding; the
+ * per sweep, 4 = as 2 with look-ahead groups of four panels at every N (automatic from N = 20000,
+ * below it pairs), 5 = as 2 with groups of three and every panel factored by the whole grid
+ * (automatic for panels of more than 3072 rows); 3 to 5 are for comparison.  Both give the tridiagonal form of ZHETRD('L') up to rounding; the
  * eigenvalues, oscillator strengths and vectors agree within the tolerances of the dense path.  No
  * counterpart in the reference (its ZHEEV is MKL's). */
 int wtbg_set_reduction(wtbg_ctx* ctx, int mode);

@@ -1,5 +1,6 @@
 // C-ABI of libwtbgpu.so: context management, argument checks, host <-> device transfers
 // and the order of kernel launches for each replaced reference stage (see wtbgpu.h).
+#include <algorithm>
 #include <array>
 #include <cfloat>
 #include <cmath>
@@ -100,9 +101,11 @@ int check_gemm_err(wtbg_ctx* ctx) {
 extern "C" {
 
 int wtbg_set_reduction(wtbg_ctx* ctx, int mode) {
-  if (!ctx || mode < 0 || mode > 3) return WTBG_ERR_ARG;
-  ctx->tri_mode = (mode == 3) ? 2 : mode;
+  if (!ctx || mode < 0 || mode > 5) return WTBG_ERR_ARG;
+  ctx->tri_mode = std::min(mode, 2);
   ctx->bulge_warp_mode = (mode == 3) ? 1 : 0;
+  ctx->panel_group = (mode == 4) ? 4 : (mode == 5 ? 3 : 0);
+  ctx->panel_wide = mode == 5;
   return WTBG_OK;
 }
 

@@ -100,6 +100,8 @@ struct wtbg_ctx {
   int tri_mode = 0;
   bool tri_two = false;
   int bulge_warp_mode = 0;   // stage 2: 0 = one CTA per sweep (k_chase), 1 = one warp per sweep (k_bulge)
+  int panel_group = 0;       // panels per look-ahead group (0: by N), and every panel grid-wide: modes 4 and 5
+  bool panel_wide = false;
   int panel_cl_max = 0;          // largest cluster of the panel QR (0: not asked yet)
   long long panel_cl_rows = 0;   // panels of up to so many rows run on one cluster
   DevBuf t2V, t2X, t2G, t2T, t2P, t2AB, t2prog, t2de;

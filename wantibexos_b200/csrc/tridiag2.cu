@@ -2027,7 +2027,9 @@ static_assert(LOOKAHEAD >= 1 && LOOKAHEAD <= 4, "look-ahead groups of 1 to 4 pan
 // Group size per reduction: the wider update pays off where the trailing matrices are large
 // (config 2, N = 36864: fours 11.75 s, pairs 11.86 s per step); at N = 8100 the update rate does
 // not rise and the corrections cost more (solve: fours 251 ms, pairs 247; N = 2304: 33.1 and 32.0).
-inline int lookahead_group(long long N) { return N >= LA_FOUR_FROM ? 4 : 2; }
+static int lookahead_group(const wtbg_ctx* ctx) {
+  return ctx->panel_group > 0 ? ctx->panel_group : (ctx->N >= LA_FOUR_FROM ? 4 : 2);
+}
 static bool two_stage_fits(wtbg_ctx* ctx, long long N) {
   if (ctx->nsm <= 0) cudaDeviceGetAttribute(&ctx->nsm, cudaDevAttrMultiProcessorCount, ctx->device);
   return N > BW + 1 && (N + ctx->nsm - 1) / ctx->nsm <= PQ_MAX_R;
@@ -2048,10 +2050,10 @@ static int two_stage_buffers(wtbg_ctx* ctx, int nband) {
   ENSURE(ctx->d, (size_t)N * 8);
   ENSURE(ctx->e, (size_t)N * 8);
   ENSURE(ctx->g, (size_t)N * 16 * NGMAX);
-  ENSURE(ctx->Wp, (size_t)N * 16 * 2 * lookahead_group(N) * BW);   // two groups: see run_stage1
-  ENSURE(ctx->t2V, (size_t)N * 16 * 2 * lookahead_group(N) * BW);
+  const int la = lookahead_group(ctx);
+  ENSURE(ctx->Wp, (size_t)N * 16 * 2 * la * BW);   // two groups: see run_stage1
+  ENSURE(ctx->t2V, (size_t)N * 16 * 2 * la * BW);
   ENSURE(ctx->t2X, (size_t)8 * BW * N * 16);
-  const int la = lookahead_group(N);
   const long long wfg = std::min<long long>(nsm, (N + WF_TR - 1) / WF_TR);   // CTAs of k_wfuse
   ENSURE(ctx->t2G, (size_t)((wfg + 1) * (2 * la - 1) + 1) * 1024 * 16);
   ENSURE(ctx->t2T, (size_t)std::max<long long>(npan, 1) * 1024 * 16);
@@ -2151,7 +2153,7 @@ static int run_stage1(wtbg_ctx* ctx, int ng, int band) {
   double2* Vp = ctx->t2V.as<double2>();
   double2* Wp = ctx->Wp.as<double2>();
   double2* Xpart = ctx->t2X.as<double2>();
-  const int la = std::min(LOOKAHEAD, lookahead_group(N));
+  const int la = std::min(LOOKAHEAD, lookahead_group(ctx));
   double2* red = ctx->t2G.as<double2>();                     // sums of k_wfuse, then its CTAs' shares
   double2* part = red + (size_t)(2 * la) * 1024;
   double2* Tbuf = ctx->t2T.as<double2>();
@@ -2197,12 +2199,13 @@ static int run_stage1(wtbg_ctx* ctx, int ng, int band) {
     pa.ng = ng;
     pa.err = err;
     mark(pnl, 0);
-    if (m <= ctx->panel_cl_rows) {
+    if (m <= ctx->panel_cl_rows && !ctx->panel_wide) {
       if (int r = launch_panel_cluster(ctx, pa)) return r;
     } else {
       // grid-wide: G CTAs of R rows (at most 64 CTAs while the rows fit: the panel is latency-bound,
-      // and fewer CTAs make the grid barrier and the cross-CTA reductions cheaper)
-      const int R = (int)std::min<long long>(PQ_MAX_R, std::max<long long>(64, (m + 63) / 64));
+      // and fewer CTAs make the grid barrier and the cross-CTA reductions cheaper; mode 5 as many as N = 56832 takes)
+      const int R = ctx->panel_wide ? (int)std::max<long long>(8, (m + nsm - 1) / nsm)
+                                    : (int)std::min<long long>(PQ_MAX_R, std::max<long long>(64, (m + 63) / 64));
       const int G = (int)((m + R - 1) / R);
       pa.R = R;
       pa.RS = R | 1;
@@ -2461,7 +2464,7 @@ int two_stage_group_add(wtbg_ctx* ctx, int slot, int nq) {
 // 13.3 ms, 6 of 1156 34.8 -> 20.9, 4 of 2304 58.4 -> 38.2 (two lanes 43.8), 3 of 5625 240 -> 214, of 8100 526 -> 486.
 int two_stage_lanes(wtbg_ctx* ctx, long long N, int nq) {
   const int nsm = ctx->nsm > 0 ? ctx->nsm : 148;
-  if (ctx->profiling || nq < 2 || N > 9216 || nsm < 128) return 1;
+  if (ctx->profiling || ctx->panel_wide || nq < 2 || N > 9216 || nsm < 128) return 1;
   if (panel_cluster_limits(ctx)) return 1;
   const int n = std::min(nq, N - BW <= ctx->panel_cl_rows ? 4 : 2);
   size_t freeb = 0, totb = 0;

@@ -289,7 +289,7 @@ class Context:
         return W, act, X, it.value, mr.value
 
     def set_reduction(self, mode: int) -> None:
-        """0 automatic, 1 one-stage, 2 two-stage reduction for the dense solves."""
+        """0 automatic, 1 one-stage, 2 two-stage reduction for the dense solves; 3 to 5: forms of 2 for comparison."""
         self._check(self.lib.wtbg_set_reduction(self.h, int(mode)))
 
     def bse_lowest(self, nev: int, nb: int = 40, max_iter: int = 200, tol: float = 1e-6, X0=None,
