@@ -65,9 +65,9 @@ __global__ void k_td_records(const double* __restrict__ d, const double* __restr
 // is one FMA a step (N = 576 0.41 -> 0.07 ms, 3600 3.6 -> 0.71 ms); scaled every eight steps.  The records stream through a four-stage ring shared by the
 // block of TD_TILE threads, all of which must call this.
 constexpr int TD_ST = 4;
-__device__ __forceinline__ int block_sturm(const double2* __restrict__ rec, int ntile, double x,
+__device__ __forceinline__ int block_sturm(const double2* __restrict__ rec, int n, double x,
                                            double2 (*ring)[TD_TILE]) {
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, ntile = (n + TD_TILE - 1) / TD_TILE;
   for (int t = 0; t < TD_ST - 1; ++t) {
     if (t < ntile) cp_async16(&ring[t][tid], rec + (size_t)t * TD_TILE + tid);
     cp_async_commit();
@@ -97,8 +97,9 @@ __device__ __forceinline__ int block_sturm(const double2* __restrict__ rec, int 
       pow2_rescale(p, pp);
     };
     load(a, 0);
+    const int rows = min(n - t * TD_TILE, TD_TILE);   // the padding counts nothing
 #pragma unroll 1
-    for (int g = 0; g < TD_TILE; g += 16) {
+    for (int g = 0; g < rows; g += 16) {
       load(b, g + 8);
       steps(a);
       load(a, (g + 16) & (TD_TILE - 1));
@@ -112,13 +113,13 @@ __device__ __forceinline__ int block_sturm(const double2* __restrict__ rec, int 
 // Coarse round: Sturm counts at the P + 1 points x_j = lo + (hi - lo) j / P of the Gershgorin
 // interval (count 0 at lo and n at hi by construction), one thread per point.
 constexpr int BIS_P = 32768;
-__global__ void __launch_bounds__(TD_TILE) k_bisect_grid(const double2* __restrict__ rec, int ntile, int n, double lo,
-                                                         double hi, double sc, double* __restrict__ xg,
+__global__ void __launch_bounds__(TD_TILE) k_bisect_grid(const double2* __restrict__ rec, int n, double lo, double hi,
+                                                         double sc, double* __restrict__ xg,
                                                          int* __restrict__ cg) {
   __shared__ __align__(16) double2 ring[TD_ST][TD_TILE];
   const int j = min(blockIdx.x * TD_TILE + (int)threadIdx.x, BIS_P);
   const double x = (j == BIS_P) ? hi : lo + (hi - lo) * ((double)j / (double)BIS_P);
-  const int c = block_sturm(rec, ntile, x * sc, ring);
+  const int c = block_sturm(rec, n, x * sc, ring);
   xg[j] = x;
   cg[j] = (j == 0) ? 0 : (j == BIS_P ? n : c);
 }
@@ -130,7 +131,7 @@ __global__ void __launch_bounds__(TD_TILE) k_bisect_grid(const double2* __restri
 // at the midpoint, for L = 1: plain bisection), so the chain of dependent Sturm passes per
 // eigenvalue is log2(L + 1) times shorter, for L times more total passes; the host picks L.
 // Stopping rule as in bisection: width <= 2 eps max(|a|, |b|) + pivmin, or no double between.
-__global__ void __launch_bounds__(TD_TILE) k_bisect(const double2* __restrict__ rec, int ntile, long long n,
+__global__ void __launch_bounds__(TD_TILE) k_bisect(const double2* __restrict__ rec, long long n,
                                                     const double* __restrict__ xg, const int* __restrict__ cg,
                                                     double pivmin, double sc, int L, double* lam) {
   __shared__ __align__(16) double2 ring[TD_ST][TD_TILE];
@@ -156,7 +157,7 @@ __global__ void __launch_bounds__(TD_TILE) k_bisect(const double2* __restrict__ 
     const bool done = !active || !(mid > a && mid < b) || (b - a <= 2.0 * DBL_EPSILON * fmax(fabs(a), fabs(b)) + pivmin);
     if (__syncthreads_and(done)) break;
     const double x = (L == 1) ? mid : a + (b - a) * ((double)(sl + 1) / (double)(L + 1));
-    const bool le = block_sturm(rec, ntile, x * sc, ring) <= m && !done;
+    const bool le = block_sturm(rec, (int)n, x * sc, ring) <= m && !done;
     const unsigned gb = (__ballot_sync(0xffffffffu, le) >> base) & (L == 32 ? 0xffffffffu : ((1u << L) - 1u));
     const int jhi = gb ? 31 - __clz(gb) : -1;   // highest point with count <= m
     const double xa = __shfl_sync(0xffffffffu, x, base + max(jhi, 0));
@@ -549,6 +550,10 @@ static int launch_twist(wtbg_ctx* ctx, const TwistArgs& a, bool clusters) {
   return 0;
 }
 
+// Below this the vectors are all made by inverse iteration: its chain is then no longer than the launches around
+// k_twist (vectors of N = 2 0.057 ms against 0.073, 8 0.117 / 0.126, 12 0.172 / 0.176, 16 0.245 both).
+constexpr long long TWIST_FROM = 16;
+
 constexpr int SB = 8;   // inverse-iteration steps whose loads are issued together
 
 __global__ void __launch_bounds__(64) k_inviter(InvArgs a) {
@@ -874,7 +879,7 @@ static int tridiagonal_solve_body(wtbg_ctx* ctx, int dtfull, int cpol, bool vect
   hi += pad;
   ENSURE(ctx->lam, (size_t)n * 8);
   const double sc = td_scale(tnorm);
-  const int npad = (int)((n + TD_TILE - 1) / TD_TILE * TD_TILE), ntile = npad / TD_TILE;
+  const int npad = (int)((n + TD_TILE - 1) / TD_TILE * TD_TILE);
   ENSURE(ctx->tmp2, (size_t)npad * 48);
   double2* rcnt = ctx->tmp2.as<double2>();
   double2* rvec = rcnt + npad;
@@ -885,9 +890,9 @@ static int tridiagonal_solve_body(wtbg_ctx* ctx, int dtfull, int cpol, bool vect
   ENSURE(ctx->bgrid, (size_t)(BIS_P + 1) * (8 + 4) + 64);
   double* xg = ctx->bgrid.as<double>();
   int* cg = reinterpret_cast<int*>(xg + BIS_P + 1);
-  k_bisect_grid<<<(BIS_P + TD_TILE) / TD_TILE, TD_TILE, 0, s>>>(rcnt, ntile, (int)n, lo, hi, sc, xg, cg);
+  k_bisect_grid<<<(BIS_P + TD_TILE) / TD_TILE, TD_TILE, 0, s>>>(rcnt, (int)n, lo, hi, sc, xg, cg);
   CKL("k_bisect_grid");
-  k_bisect<<<(int)((n * lanes + TD_TILE - 1) / TD_TILE), TD_TILE, 0, s>>>(rcnt, ntile, n, xg, cg, pivmin, sc, lanes,
+  k_bisect<<<(int)((n * lanes + TD_TILE - 1) / TD_TILE), TD_TILE, 0, s>>>(rcnt, n, xg, cg, pivmin, sc, lanes,
                                                                         ctx->lam.as<double>()); WTBG_COUNT(ctx, 3);
   CKL("k_bisect");
   ctx->lam_host.resize(n);
@@ -925,8 +930,13 @@ static int tridiagonal_solve_body(wtbg_ctx* ctx, int dtfull, int cpol, bool vect
   ENSURE(ctx->act, (size_t)8 * 8 * n);
   ENSURE(ctx->csz, (size_t)n * 8 + 64);
   int* todo = ctx->csz.as<int>() + n;
-  CK(cudaMemsetAsync(todo, 0, (size_t)n * 4, s));
-  CK(cudaMemcpyAsync(ctx->csz.as<int>(), csize.data(), n * 4, cudaMemcpyHostToDevice, s));
+  const bool twist = n >= TWIST_FROM;
+  if (twist) {
+    CK(cudaMemsetAsync(todo, 0, (size_t)n * 4, s));
+    CK(cudaMemcpyAsync(ctx->csz.as<int>(), csize.data(), n * 4, cudaMemcpyHostToDevice, s));
+  } else {
+    CK(cudaMemcpyAsync(todo, csize.data(), n * 4, cudaMemcpyHostToDevice, s));
+  }
   ctx->csize_host = csize;
   ctx->tnorm = tnorm;
   InvArgs a;
@@ -976,7 +986,8 @@ static int tridiagonal_solve_body(wtbg_ctx* ctx, int dtfull, int cpol, bool vect
     const int cnt = (int)(m1 - m0);
     tw.m0 = (int)m0;
     tw.m1 = (int)m1;
-    if (int r = a.ng == 10 ? launch_twist<10>(ctx, tw, maxc > 1) : launch_twist<5>(ctx, tw, maxc > 1)) return r;
+    if (twist)
+      if (int r = a.ng == 10 ? launch_twist<10>(ctx, tw, maxc > 1) : launch_twist<5>(ctx, tw, maxc > 1)) return r;
     k_inviter<<<(cnt + 63) / 64, 64, 0, s>>>(a); WTBG_COUNT(ctx, 1);
     CKL("k_inviter");
     m0 = m1;
@@ -1027,12 +1038,15 @@ int run_eigvecs(wtbg_ctx* ctx, int n0, int n1, double2* d_out) {
     tw.cpol = 0;
     tw.rtol = 8.0 * DBL_EPSILON * std::sqrt((double)n);
     tw.keep = true;
-    k_td_records<<<(npad + 255) / 256, 256, 0, s>>>(ctx->d.as<double>(), ctx->e.as<double>(), (int)n, npad, tw.sc, rec,
-                                                    rec + npad);
-    WTBG_COUNT(ctx, 1);
-    CKL("k_td_records");
-    CK(cudaMemsetAsync(todo, 0, (size_t)n * 4, s));
-    if (int r = ctx->ng == 10 ? launch_twist<10>(ctx, tw, true) : launch_twist<5>(ctx, tw, true)) return r;
+    const bool twist = n >= TWIST_FROM;   // else todo still holds the clusters of the solve
+    if (twist) {
+      k_td_records<<<(npad + 255) / 256, 256, 0, s>>>(ctx->d.as<double>(), ctx->e.as<double>(), (int)n, npad, tw.sc, rec,
+                                                      rec + npad);
+      WTBG_COUNT(ctx, 1);
+      CKL("k_td_records");
+      CK(cudaMemsetAsync(todo, 0, (size_t)n * 4, s));
+      if (int r = ctx->ng == 10 ? launch_twist<10>(ctx, tw, true) : launch_twist<5>(ctx, tw, true)) return r;
+    }
     InvArgs a;
     a.d = ctx->d.as<double>();
     a.e = ctx->e.as<double>();
@@ -1054,9 +1068,11 @@ int run_eigvecs(wtbg_ctx* ctx, int n0, int n1, double2* d_out) {
     a.zs1 = n1 - 1;
     k_inviter<<<(int)((M + 63) / 64), 64, 0, s>>>(a); WTBG_COUNT(ctx, 1);
     CKL("k_inviter(eigvecs)");
-    k_take_vectors<<<dim3((unsigned)((n + 255) / 256), nvec), 256, 0, s>>>(tw, n0 - 1, ctx->zsel.as<double>());
-    WTBG_COUNT(ctx, 1);
-    CKL("k_take_vectors");
+    if (twist) {
+      k_take_vectors<<<dim3((unsigned)((n + 255) / 256), nvec), 256, 0, s>>>(tw, n0 - 1, ctx->zsel.as<double>());
+      WTBG_COUNT(ctx, 1);
+      CKL("k_take_vectors");
+    }
   }
   const long long cnt = (long long)nvec * n;
   k_real_to_complex<<<(int)((cnt + 255) / 256), 256, 0, s>>>(ctx->zsel.as<double>(), d_out, cnt); WTBG_COUNT(ctx, 1);
