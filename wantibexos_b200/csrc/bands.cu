@@ -173,16 +173,20 @@ __device__ __forceinline__ void bands_body(const BandsArgs& a, const int k, unsi
           const double2 c = cconj(A[q + p * ld]);
           const double ac2 = fma(c.x, c.x, __dmul_rn(c.y, c.y));
           if (ac2 > fmax(0.25 * DBL_EPSILON * DBL_EPSILON * fabs(aa * bb), tol2) && ac2 >= DBL_MIN) {
-            // t = sign(d) 2|c| / (|d| + sqrt(d^2 + 4 |c|^2)), d = bb - aa
-            const double ia = rsqrt(ac2), ac = ac2 * ia, d = bb - aa;
-            const double hh = fma(d, d, 4.0 * ac2);
-            const double tt = copysign(2.0 * ac, d) / (fabs(d) + sqrt(hh));
-            cs = rsqrt(fma(tt, tt, 1.0));
-            const double sn = tt * cs * ia;
-            sx = sn * c.x;
-            sy = sn * c.y;
-            lam[p] = fma(-tt, ac, aa);
-            lam[q] = fma(tt, ac, bb);
+            // the angle by its double: cos 2t = |d| / h, h = sqrt(d^2 + 4 |c|^2), d = bb - aa, so cos^2 t = (1 + |d| / h) / 2
+            // without cancellation, and sin t = |c| / (h cos t): two reciprocal roots; then (cos, sin) to length 1
+            const double d = bb - aa, ih = rsqrt(fma(d, d, 4.0 * ac2));
+            const double c2 = fma(0.5 * fabs(d), ih, 0.5), ic = rsqrt(c2);
+            double f = copysign(ih * ic, d);   // sin t / |c|
+            const double dl = f * ic * ac2;    // tan t |c|
+            cs = c2 * ic;
+            const double off = 0.5 * fma(-f * f, ac2, fma(-cs, cs, 1.0));
+            cs = fma(cs, off, cs);
+            f = fma(f, off, f);
+            sx = f * c.x;
+            sy = f * c.y;
+            lam[p] = aa - dl;
+            lam[q] = bb + dl;
             A[q + p * ld] = make_double2(0.0, 0.0);
             act = 1;
           }
