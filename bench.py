@@ -517,7 +517,7 @@ def main():
                     help="plain FP64 path (the headline), the fast form, or both (default)")
     ap.add_argument("--no-learned", action="store_true", help="skip the learned warm-start and config-4 legs")
     ap.add_argument("--reduction", default="auto", choices=["auto", "one", "two", "two-warp"],
-                    help="tridiagonal reduction of the dense solve: automatic (two-stage for N >= 2048), "
+                    help="tridiagonal reduction of the dense solve: automatic (two-stage wherever it fits), "
                          "one-stage or two-stage")
     ap.add_argument("--device-only", action="store_true",
                     help="only the device-resident steps (no e2e run, no CPU baseline): profiling captures")

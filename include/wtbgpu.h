@@ -51,7 +51,10 @@ typedef struct wtbg_coulomb {
 
 typedef struct wtbg_ctx wtbg_ctx;
 
-/* ---- context ------------------------------------------------------------ */
+/* ---- context ------------------------------------------------------------
+ * A context is used by one host thread at a time; different contexts, also of one device, by different
+ * threads at the same time.  The two-stage reductions and the exciton vectors of one device are
+ * taken one at a time within a process: their grids need all their CTAs resident. */
 int wtbg_create(wtbg_ctx** ctx, int device);
 int wtbg_destroy(wtbg_ctx* ctx);
 const char* wtbg_error_string(int status);
@@ -363,10 +366,15 @@ int wtbg_set_precision(wtbg_ctx* ctx, int mode);
 /* ---- exciton band structure, all Q of a path in one call (the Q loop of bsebnds,
  *      bse_kpath-tool.f90:246-435).  kptq holds nq blocks of (nk,3) k+Q meshes, q4 nq rows of
  *      (distance, qx, qy, qz); W (nq, N) receives each Q's eigenvalues ascending, identical to
- *      nq calls of wtbg_bse_q_eigenvalues.  With use_graph != 0 the tridiagonalisation (the
- *      launch-bound part: four launches per column) runs as one captured CUDA graph replayed
- *      for every Q after the first; the mat-vec chunk is autotuned per (device, N) on the
- *      first Q.  ms_q (nq, may be NULL) receives the device time of each Q. */
+ *      nq calls of wtbg_bse_q_eigenvalues.  Where the two-stage reduction is used (34 <= N <= 384
+ *      rows per SM unless wtbg_set_reduction says otherwise) the Q points go in groups of up to 64:
+ *      the first stage of up to four of them side by side (up to three further N x N matrices with
+ *      their buffers, kept in the context until the next wtbg_set_model), one launch of the second stage
+ *      for all; use_graph has no effect there, and ms_q holds the group's device time divided by its
+ *      points.  With the one-stage reduction use_graph != 0 runs the tridiagonalisation (the
+ *      launch-bound part: four launches per column) as one captured CUDA graph replayed for every Q
+ *      after the first, the mat-vec chunk being autotuned per (device, N) on the first Q, and ms_q (nq,
+ *      may be NULL) receives the device time of each Q. */
 int wtbg_bse_q_batch(wtbg_ctx* ctx, int nk, int nq, const double* kptq, const double* q4,
                      const wtbg_coulomb* p, int use_graph, double* W, double* ms_q);
 

@@ -770,8 +770,8 @@ __global__ void __launch_bounds__(256) k_vectors_out(const double2* __restrict__
   }
 }
 
-// The layout change on the device and one copy per piece of at most 128 MB (pieces are ranges of the
-// slowest output index m).  On the host it was a strided walk over the whole array: with the copy it
+// The layout change on the device and one copy per piece (pieces are ranges of the slowest output index m, of
+// at most 128 MB or one index: a w-th of the vectors themselves).  On the host it was a strided walk over the whole array: with the copy it
 // took 23 ms of 32 for 1296 k-points of 40 bands.
 int copy_vectors_out(wtbg_ctx* ctx, const double2* d_U, int nk, int nb, int w, double* vec) {
   const size_t per = (size_t)nk * nb * 16;

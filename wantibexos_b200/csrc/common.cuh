@@ -235,7 +235,7 @@ inline int set_device(wtbg_ctx* ctx) {
 int launch_bands_batch(wtbg_ctx* const* ctxs, int nmod);
 int launch_eigsys_all(wtbg_ctx* ctx, int nk, const double* d_kpt, double* d_eig, double2* d_U, int* d_nocp,
                       int* d_kstat);
-// U [nk][nb][w] into the caller's vec(k, j, m) = k + nk (j + nb m), in bounded pieces through ctx->tmp2
+// U [nk][nb][w] into the caller's vec(k, j, m) = k + nk (j + nb m), in pieces through ctx->tmp2
 int copy_vectors_out(wtbg_ctx* ctx, const double2* d_U, int nk, int nb, int w, double* vec);
 int launch_berry(wtbg_ctx* ctx, int nk, const double* d_kpt, const double* d_eig, const double2* d_U, const int* d_nocp,
                  double gamma, double degtol, double* d_out);

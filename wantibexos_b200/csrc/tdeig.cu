@@ -62,8 +62,8 @@ __global__ void k_td_records(const double* __restrict__ d, const double* __restr
 // Number of eigenvalues of the scaled T below x, one point per thread: the sign changes of the leading
 // minors p_{k+1} = (d_k - x) p_k - e_{k-1}^2 p_{k-1} (the counts of the pivots p_{k+1} / p_k, and as backward
 // stable: each step is exact for d_k - x and e_{k-1}^2 changed by a few roundings).  Without a division the chain
-// is one FMA a step (N = 576 0.41 -> 0.07 ms, 3600 3.6 -> 0.71 ms); scaled every eight steps.  The records stream through a four-stage ring shared by the
-// block of TD_TILE threads, all of which must call this.
+// is one FMA a step (N = 576 0.41 -> 0.07 ms, 3600 3.6 -> 0.71 ms); scaled every eight steps.  The records stream
+// through a four-stage ring shared by the block of TD_TILE threads, all of which must call this.
 constexpr int TD_ST = 4;
 __device__ __forceinline__ int block_sturm(const double2* __restrict__ rec, int n, double x,
                                            double2 (*ring)[TD_TILE]) {

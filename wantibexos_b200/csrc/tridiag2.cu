@@ -1392,7 +1392,7 @@ __global__ void __launch_bounds__(32 * BG_WARPS, 1) k_bulge(BulgeArgs a) {
 //   * the reflector's vector is used unscaled: with u = x - beta e_0 the reflector is
 //     H = I - kappa u u^H, kappa = -u_0 / (beta |u_0|^2), and every product D u, B1 u, u^H B is the
 //     product with x minus beta times the first column (row), so the products of a step run beside
-//     the scalars (one reciprocal square root, one reciprocal) instead of after them;
+//     the scalars (a root, its reciprocal and one more reciprocal) instead of after them;
 //   * the block below (B1) is the next step's bulge block (B): the four warps that update it keep it
 //     in registers, so it is written once, after its second update.  Four groups of four warps take
 //     turns: group n mod 4 does B1 of step n, then B of step n+1, then the diagonal block of step n+2,
@@ -1408,7 +1408,7 @@ __global__ void __launch_bounds__(32 * BG_WARPS, 1) k_bulge(BulgeArgs a) {
 // qb = 4 (bit 2) + (lane >> 3), and an element's place in the band, 63 c + i from its block's corner, is
 // one lane offset plus the constant 504 m + 4 r; the sums over the columns (B1, D) stay within one
 // warp, and the shared-memory accesses are free of bank conflicts.
-// Measured (whole stage, five velocity vectors): N = 576 4.3 ms, 2304 18.9 ms, 8100 80 ms, 14400 161 ms;
+// Measured (whole stage, five velocity vectors): N = 576 4.3 ms, 2304 19.2 ms, 8100 85 ms, 14400 178 ms;
 // with one CTA of four warps per sweep and CTA barriers between the parts of a step it was 10.9, 46.7,
 // 169 and 309 ms.  Tried: bulk copies instead of cp.async (longer latency, 19.5 ms at 2304), blocks
 // loaded from L2 into a second set of registers (spills, 24 ms), two groups that swap B1 and B (21 ms).
@@ -2039,7 +2039,7 @@ static bool two_stage_fits(wtbg_ctx* ctx, long long N) {
 // solve, one-stage against two-stage: N = 36 1.01 / 0.49 ms, 144 4.1 / 2.3, 576 17.4 / 10.4, 1156 36.8 /
 // 22.0, 2304 83.7 / 47.6, 14400 2423 / 979 (the one-stage reduction is four launches per column, the
 // two-stage one five per 32 columns and one for the chase).  Later steps brought the two-stage solve of N = 576 to
-// 6.5 ms, of 2304 to 30, of 14400 to 843.
+// 6.5 ms, of 2304 to 30, of 14400 to 854.
 bool use_two_stage(wtbg_ctx* ctx) { return ctx->tri_mode != 1 && two_stage_fits(ctx, ctx->N); }
 
 // Work buffers of the two-stage reduction for N (nband bands side by side for Q groups).
@@ -2460,7 +2460,8 @@ int two_stage_group_add(wtbg_ctx* ctx, int slot, int nq) {
 // a small matrix is a chain of kernels that leave most of the device idle (the panel QR takes 16 SMs or 64), and at
 // large N the panels of one run beside the products of another.  The kernels that spin on a grid barrier are all
 // resident at once: k_wfuse takes nsm / lanes CTAs, and the grid-wide panel QR (64 CTAs up to N = 9216) runs only
-// where there are two lanes; four where every panel goes to a cluster.  A path of 12 Q points of N = 576 27.8 ->
+// where there are two lanes; four where every panel goes to a cluster.  Other contexts of the device are kept
+// out meanwhile (SpinSection).  A path of 12 Q points of N = 576 27.8 ->
 // 13.3 ms, 6 of 1156 34.8 -> 20.9, 4 of 2304 58.4 -> 38.2 (two lanes 43.8), 3 of 5625 240 -> 214, of 8100 526 -> 486.
 int two_stage_lanes(wtbg_ctx* ctx, long long N, int nq) {
   const int nsm = ctx->nsm > 0 ? ctx->nsm : 148;
