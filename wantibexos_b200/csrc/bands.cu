@@ -715,6 +715,8 @@ __global__ void k_sp_gather(const float* rows, const int* order, long long N, fl
 // Work-area placement of the per-k kernels: the model's matrices go to dynamic shared memory
 // when they fit the budget, else every CTA of a grid capped at 4 CTAs per SM gets a slice of
 // ctx->gwork in global memory (L2-resident at these sizes) and loops over k.
+// The kernels' limit is always set to the budget: it belongs to the function, and a smaller one for one context's
+// model could come between another thread's setting and its launch.
 constexpr size_t kSmemBudget = 200 * 1024;
 static int place_work(wtbg_ctx* ctx, size_t bytes, long long nk, unsigned char** gwork, long long* gstride,
                       size_t* dyn, int* grid) {
@@ -840,7 +842,7 @@ int launch_bands(wtbg_ctx* ctx, bool q_mesh) {
   size_t smem = 0;
   int grid = 0;
   if (int r = place_work(ctx, bands_smem(w, ctx->nvec), ctx->nk, &a.gwork, &a.gstride, &smem, &grid)) return r;
-  CK(cudaFuncSetAttribute(k_bands, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CK(cudaFuncSetAttribute(k_bands, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
   k_bands<<<grid, bands_threads(ctx, w, a.nk), smem, ctx->stream>>>(a, BatchItems{}, a.nk); WTBG_COUNT(ctx, 1);
   CKL("k_bands");
   return 0;
@@ -922,7 +924,7 @@ int launch_bands_batch(wtbg_ctx* const* ctxs, int nmod) {
     smem = 0;
     per = 4;
   }
-  CK(cudaFuncSetAttribute(k_bands, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CK(cudaFuncSetAttribute(k_bands, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
   if (smem > 0) CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_bands, threads, smem));
   const int grid = (int)std::min<long long>(nitems, (long long)nsm * std::max(1, per));
   k_bands<<<grid, threads, smem, s>>>(BandsArgs{}, BatchItems{d_mod, d_im, d_ik, d_cnt}, (int)nitems);
@@ -959,7 +961,7 @@ int launch_eigsys_all(wtbg_ctx* ctx, int nk, const double* d_kpt, double* d_eig,
   size_t smem = 0;
   int grid = 0;
   if (int r = place_work(ctx, bands_smem(w, ctx->nvec), nk, &a.gwork, &a.gstride, &smem, &grid)) return r;
-  CK(cudaFuncSetAttribute(k_bands, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CK(cudaFuncSetAttribute(k_bands, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
   k_bands<<<grid, bands_threads(ctx, w, a.nk), smem, ctx->stream>>>(a, BatchItems{}, a.nk); WTBG_COUNT(ctx, 1);
   CKL("k_bands(all)");
   return 0;
@@ -990,7 +992,7 @@ int launch_velocity(wtbg_ctx* ctx, double eta32) {
   size_t smem = 0;
   int grid = 0;
   if (int r = place_work(ctx, need, ctx->nk, &a.gwork, &a.gstride, &smem, &grid)) return r;
-  CK(cudaFuncSetAttribute(k_velocity, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CK(cudaFuncSetAttribute(k_velocity, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
   k_velocity<<<grid, kBandsThreads, smem, ctx->stream>>>(a); WTBG_COUNT(ctx, 1);
   CKL("k_velocity");
   return 0;
@@ -1057,7 +1059,7 @@ int launch_berry(wtbg_ctx* ctx, int nk, const double* d_kpt, const double* d_eig
   const auto need = [&](int ld) { return sizeof(double2) * ((size_t)nvec + 5 * (size_t)w * ld); };
   a.ld = need(w | 1) <= kSmemBudget ? (w | 1) : w;
   if (int r = place_work(ctx, need(a.ld), nk, &a.gwork, &a.gstride, &smem, &grid)) return r;
-  CK(cudaFuncSetAttribute(k_berry, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CK(cudaFuncSetAttribute(k_berry, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
   k_berry<<<grid, kBandsThreads, smem, ctx->stream>>>(a); WTBG_COUNT(ctx, 1);
   CKL("k_berry");
   return 0;
@@ -1091,7 +1093,7 @@ int launch_optbz(wtbg_ctx* ctx, int nk, int nv, int nc, const double* d_kpt, con
   if (int r = place_work(ctx, sizeof(double2) * ((size_t)nvec + 4 * (size_t)w * w), nk, &a.gwork, &a.gstride, &smem,
                          &grid))
     return r;
-  CK(cudaFuncSetAttribute(k_optbz, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CK(cudaFuncSetAttribute(k_optbz, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
   k_optbz<<<grid, kBandsThreads, smem, ctx->stream>>>(a); WTBG_COUNT(ctx, 1);
   CKL("k_optbz");
   return 0;

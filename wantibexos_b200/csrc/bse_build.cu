@@ -401,7 +401,8 @@ int launch_bse_build(wtbg_ctx* ctx, const wtbg_coulomb* p, const double* q4) {
   if (TK < 1) TK = 1;
   while (TK > 1 && build_smem(TK, nc, nv, w) > 96 * 1024) --TK;
   const size_t smem = build_smem(TK, nc, nv, w);
-  if (smem > 200 * 1024) return set_err(ctx, WTBG_ERR_UNSUPPORTED, "bse_build: tile does not fit in shared memory");
+  constexpr size_t budget = 200 * 1024;   // also the kernel's limit, whatever the tile: it is shared by all threads
+  if (smem > budget) return set_err(ctx, WTBG_ERR_UNSUPPORTED, "bse_build: tile does not fit in shared memory");
   BuildArgs a;
   const bool q = (q4 != nullptr);
   a.Uc = q ? ctx->Uq.as<double2>() : ctx->U.as<double2>();
@@ -461,7 +462,7 @@ int launch_bse_build(wtbg_ctx* ctx, const wtbg_coulomb* p, const double* q4) {
     if (r) return r;
     a.vq = vq;
   }
-  CK(cudaFuncSetAttribute(k_bse_build, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  CK(cudaFuncSetAttribute(k_bse_build, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget));
   const long long ntile = (long long)a.nbk * (a.nbk + 1) / 2;
   if (ntile > 0x7fffffffLL) return set_err(ctx, WTBG_ERR_UNSUPPORTED, "bse_build: too many tiles");
   const bool prof = ctx->profiling != 0;

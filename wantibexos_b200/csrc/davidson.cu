@@ -1066,7 +1066,7 @@ static int cholqr2(wtbg_ctx* ctx, double2* T, int q, double2* tmp, DavWork& w) {
   for (int pass = 0; pass < 2; ++pass) {
     if (int r = gram(ctx, T, (int)N, q, T, (int)N, q, w.small, w.part)) return r;
     const size_t csm = (size_t)((q + 1) * (q | 1)) * 16;
-    CK(cudaFuncSetAttribute(k_chol_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csm));
+    CK(cudaFuncSetAttribute(k_chol_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, 65 * 65 * 16));   // q <= 64
     k_chol_inv<<<1, 512, csm, ctx->stream>>>(w.small, q, w.small + 64 * 64, w.istat); WTBG_COUNT(ctx, 1);
     CKL("chol");
     if (int r = tall(ctx, T, (int)N, q, w.small + 64 * 64, q, tmp, (int)N, false)) return r;
